@@ -24,6 +24,9 @@ OBJDIR = os.path.join(ROOT, "_build")
 LIB_KERNELS = os.path.join(LIBDIR, "libmhh_gb300.so")
 LIB_HOST = os.path.join(LIBDIR, "libmhh_host.so")
 
+# Translation units with many kernels compile once per precision (MHH_PREC).
+PER_PRECISION = ("mhh_pres.cu", "mhh_stencil.cu")
+
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -77,10 +80,13 @@ def build(verbose=False, force=False, extra_nvcc=()):
     if force or not os.path.exists(LIB_KERNELS) or _newest(cu + hdr) > os.path.getmtime(LIB_KERNELS):
         objs, cmds = [], []
         for src in cu:
-            obj = os.path.join(OBJDIR, os.path.basename(src)[:-3] + ".o")
-            objs.append(obj)
-            cmds.append([nvcc, "-std=c++17", *ARCH, "-O3", "-lineinfo", "-Xcompiler", "-fPIC",
-                         "-I" + INCLUDE, "-I" + CSRC, *extra_nvcc, "-c", src, "-o", obj])
+            name = os.path.basename(src)
+            for prec in ((64, 32) if name in PER_PRECISION else (0,)):
+                obj = os.path.join(OBJDIR, name[:-3] + (f".f{prec}.o" if prec else ".o"))
+                objs.append(obj)
+                cmds.append([nvcc, "-std=c++17", *ARCH, "-O3", "-lineinfo", "-Xcompiler", "-fPIC",
+                             *([f"-DMHH_PREC={prec}"] if prec else []),
+                             "-I" + INCLUDE, "-I" + CSRC, *extra_nvcc, "-c", src, "-o", obj])
         _run_parallel(cmds)
         _run_parallel([[nvcc, *ARCH, "-shared", "-o", LIB_KERNELS, *objs, "-lcudart",
                         "-Xlinker", "-rpath," + _cudalib(cuda)]])

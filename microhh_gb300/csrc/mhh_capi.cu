@@ -355,7 +355,7 @@ namespace
         if ((rc = upload(c->pw.bmati, bi)) || (rc = upload(c->pw.bmatj, bj))) return rc;
         if ((rc = upload(c->pw.a, a)) || (rc = upload(c->pw.c, cc))) return rc;
         if ((rc = upload(c->pw.dz2, dz2)) || (rc = upload(c->pw.dz2rho, dz2r))) return rc;
-        if ((rc = tdma_table(c->pw, d.itot, d.jtot, d.ktot, c->setup))) return fail(rc, "tridiagonal table");
+        if ((rc = tdma_table(c->pw, d.itot, d.jtot, d.ktot, c->prec, c->setup))) return fail(rc, "tridiagonal table");
         return MHH_OK;
     }
 
@@ -894,6 +894,7 @@ int mhh_ctx_estimate_bytes(const mhh_grid_desc* g, int precision, size_t* bytes)
     b += 14.*kcells*tf;                         // profiles
     b += n*tf + n*8. + g->ktot*8.;              // packed pressure + work + level means
     b += groups*(8. + 8. + 8. + 8. + 4. + 8.); // elimination tables
+    b += 1.1*groups*(precision == MHH_FP64 ? 24. : 12. + 20.);   // the same in block order
     b += 2.*(g->itot + g->jtot)*(16. + 8.);    // twiddles
     b += 12.*ij*8. + ij*4. + 2.*10000*4.;      // surface layer
     b += 2.*kcells*8.;                          // mixing length
@@ -910,7 +911,7 @@ int mhh_ctx_destroy(mhh_ctx* c)
     // stream reaches it; the caller has finished its own work on the fields.
     for (auto& p : c->dprof) if (p) cudaFreeAsync(p, c->setup);
     fft_plan_free(&c->pw.px, c->setup); fft_plan_free(&c->pw.py, c->setup);
-    void* ptrs[] = {c->pw.pk, c->pw.work, c->pw.dcm, c->pw.rtab, c->pw.wtab, c->pw.gtab, c->pw.htab, c->pw.stab, c->pw.stabd, c->pw.gftab, c->pw.hftab, c->pw.fmode, c->pw.bmati, c->pw.bmatj, c->pw.a, c->pw.c, c->pw.dz2, c->pw.dz2rho,
+    void* ptrs[] = {c->pw.pk, c->pw.work, c->pw.dcm, c->pw.rtab, c->pw.wtab, c->pw.gtab, c->pw.htab, c->pw.stab, c->pw.stabd, c->pw.fmode, c->pw.ctab, c->pw.dtab, c->pw.list, c->pw.ltab, c->pw.lstab, c->pw.bmati, c->pw.bmatj, c->pw.a, c->pw.c, c->pw.dz2, c->pw.dz2rho,
                     c->red, c->statbuf, c->bufprof, c->sw.fm, c->sw.fh, c->sw.phim, c->sw.phih, c->sw.ustar, c->sw.obuk, c->sw.dudz, c->sw.dvdz, c->sw.dbdz, c->sw.dutot,
                     c->sw.nobuk, c->sw.zL, c->sw.f, c->sw.mlen2, c->sw.mlen2f};
     for (void* p : ptrs) if (p) cudaFreeAsync(p, c->setup);

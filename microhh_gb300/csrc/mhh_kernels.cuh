@@ -141,9 +141,18 @@ namespace mhh
         double* htab;         // same shape: backward coefficient of the rescaled recurrence
         float* stab;          // same shape: output scale dz^2/den in float
         double* stabd;        // same shape: output scale dz^2/den
-        float* gftab;         // same shape: gtab in float
-        float* hftab;         // same shape: htab in float
         unsigned char* fmode; // (itot/2+1)*(jtot/2+1): 1 where the group's recurrence may run in float
+        // Column-resident solve: 2^lg groups per block (-1: columns too tall
+        // for shared memory), coefficients in block order (FP32 contexts:
+        // ctab g, h, s in float; FP64 contexts: dtab 1/den, den, c/den), and
+        // in FP32 contexts the nlist groups that sweep in FP64 with theirs.
+        int lg;
+        float* ctab;
+        double* dtab;
+        int nlist;
+        int* list;
+        double* ltab;
+        float* lstab;
         void* dcm;            // ktot values (TF): each level's mean, (X_00/jtot)/itot
         int niu, nju;
     };
@@ -163,7 +172,7 @@ namespace mhh
     int pres_fuse();
     void set_fft_column_pairs(int p);
 
-    int tdma_table(PresWork& pw, int itot, int jtot, int ktot, cudaStream_t s);
+    int tdma_table(PresWork& pw, int itot, int jtot, int ktot, int precision, cudaStream_t s);
 
     template<typename TF> void launch_pres_in(const Dims& d, const Prof<TF>& pr, const TF* u, const TF* v, const TF* w,
                                               const TF* ut, const TF* vt, const TF* wt, TF* pk, double dti, cudaStream_t s);

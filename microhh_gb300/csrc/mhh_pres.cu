@@ -1,9 +1,8 @@
 // mhh_pres.cu -- the Pres_2 Poisson solve on the GPU without cuFFT:
 // divergence of the predicted velocity, hand-written real FFTs along x and y
-// (halfcomplex layout, so the spectral solve is the reference's), a Thomas
-// solve per spectral column (in double; in the float form in float where the
-// column's forward sweep damps), inverse FFTs and the scatter back into the
-// ghost-cell layout.
+// (halfcomplex layout, so the spectral solve is the reference's) and the
+// scatter back into the ghost-cell layout; the Thomas solve per spectral
+// column between the forward and inverse transforms is in mhh_tdma.cu.
 //
 // FFT: two real sequences x, y of length n are transformed together as
 // z = x + i y with a mixed-radix (4, 2, 3, 5, 7) Stockham autosort FFT in
@@ -1206,6 +1205,7 @@ namespace mhh
         (void)jtot;
     }
 
+#if MHH_PREC == 64
     int fft_plan_init(FftPlan* pl, int n, cudaStream_t s)
     {
         std::memset(pl, 0, sizeof(*pl));
@@ -1237,6 +1237,7 @@ namespace mhh
         if (pl->tw_f) cudaFreeAsync(pl->tw_f, s);
         pl->tw_d = nullptr; pl->tw_f = nullptr;
     }
+#endif
 
     // ---------------------------------------------------------------------
     // Right-hand side, src/pres_2.cxx:155-196: divergence of ut + u/dt into
@@ -1266,593 +1267,6 @@ namespace mhh
     }
 
     // ---------------------------------------------------------------------
-    // Tridiagonal solve per spectral column in double, src/pres_2.cxx:200-326:
-    // b = dz^2 rho (bmati + bmatj) - (a + c), b[0] += a[0]; the top row gets
-    // -c for the mean mode (p = 0 at the top) and +c otherwise (dp/dz = 0);
-    // right-hand side dz^2 p; Thomas algorithm.
-    //
-    // The elimination coefficients depend on the column only through
-    // lambda = bmati[i] + bmatj[j], and bmati, bmatj are mirror-symmetric
-    // (i and itot - i share a wave number), so the columns form groups of up
-    // to four with identical coefficients.  den_k and c_k/den_k of every group
-    // are computed once at set-up (k_tdma_table), rounded as the reference
-    // rounds them.  The reference-order solve (k_tdma) then repeats the
-    // reference's per-cell operations (a product, a difference and a division
-    // forward, a product and a difference back) with one thread for the four
-    // columns of a group: the mean mode's solve is ill-conditioned, so its
-    // result follows every rounding of the sweep.  The rescaled solve
-    // (k_tdma_col) needs two FMAs per cell, with one thread per column
-    // (k_tdma_scaled: the same with four columns per thread).
-    // ---------------------------------------------------------------------
-    constexpr double TDMA_FLOAT_GAMMA = 0.999;
-
-    __global__ void k_tdma_table(int niu, int nju, int ktot, const double* __restrict__ bmati,
-                                 const double* __restrict__ bmatj, const double* __restrict__ a,
-                                 const double* __restrict__ c, const double* __restrict__ dz2rho,
-                                 const double* __restrict__ dz2, double* __restrict__ rtab,
-                                 double* __restrict__ wtab, double* __restrict__ gtab, double* __restrict__ htab,
-                                 float* __restrict__ stab, double* __restrict__ stabd,
-                                 float* __restrict__ gftab, float* __restrict__ hftab,
-                                 unsigned char* __restrict__ fmode)
-    {
-        const int iu = blockIdx.x*blockDim.x + threadIdx.x;
-        const int ju = blockIdx.y;
-        if (iu >= niu) return;
-        const long long stride = (long long)niu*nju;
-        const long long base = iu + (long long)ju*niu;
-        const double lam = bmati[iu] + bmatj[ju];
-        const bool mean_mode = (iu == 0 && ju == 0);
-        // src/pres_2.cxx:266-326 and :200-263, products not contracted.
-        double b = mulx(dz2rho[0], lam) - (a[0] + c[0]);
-        b += a[0];
-        if (ktot == 1) b += mean_mode ? -c[0] : c[0];
-        double den = b;
-        rtab[base] = den;
-        for (int k=1; k<ktot; ++k)
-        {
-            double bk = mulx(dz2rho[k], lam) - (a[k] + c[k]);
-            if (k == ktot-1) bk += mean_mode ? -c[k] : c[k];
-            const double w3 = c[k-1]/den;
-            wtab[base + (k-1)*stride] = w3;
-            den = bk - mulx(a[k], w3);
-            rtab[base + k*stride] = den;
-        }
-        wtab[base + (ktot-1)*stride] = 0.;
-        // Rescaled recurrence: with s_k = dz2_k/den_k, y_k = s_k z_k and
-        // x_k = s_k xi_k the sweeps become
-        //   z_k = p_k - g_k z_{k-1},      g_k = a_k s_{k-1}/dz2_k,
-        //   xi_k = z_k - h_k xi_{k+1},    h_k = c_k s_{k+1}/dz2_k,
-        // and x_k = s_k xi_k: one FMA per cell and sweep.
-        for (int k=0; k<ktot; ++k)
-        {
-            const double sk = dz2[k]/rtab[base + k*stride];
-            stabd[base + k*stride] = sk;
-            stab[base + k*stride] = float(sk);
-            gtab[base + k*stride] = k ? a[k]*(dz2[k-1]/rtab[base + (k-1)*stride])/dz2[k] : 0.;
-            htab[base + k*stride] = k < ktot-1 ? c[k]*(dz2[k+1]/rtab[base + (k+1)*stride])/dz2[k] : 0.;
-        }
-        // Float sweeps where the forward sweep damps: a rounding error of z_k
-        // enters the next level multiplied by g_{k+1}, and as |g| -> 1 (small
-        // |lambda| dz^2: the largest horizontal scales) the forward values
-        // become running sums whose round-off grows with the level.  With
-        // max |g| <= TDMA_FLOAT_GAMMA the float solve of a column stays
-        // within about ten float roundings of its largest value (measured on
-        // 256 uniform levels with random right-hand sides: 9 ulp at |g| =
-        // 0.999, 4 ulp at 0.9).  The large backward factor h at the top
-        // level (the Neumann row) multiplies a value that s scales down, and
-        // adds no more.  The groups above the bound and the mean mode keep
-        // FP64.
-        double gam = 0.;
-        for (int k=0; k<ktot; ++k)
-        {
-            const double g = gtab[base + k*stride], h = htab[base + k*stride];
-            gftab[base + k*stride] = float(g);
-            hftab[base + k*stride] = float(h);
-            gam = fmax(gam, fabs(g));
-        }
-        fmode[base] = (!mean_mode && gam <= TDMA_FLOAT_GAMMA) ? 1 : 0;
-    }
-
-    // The k loops run in batches of levels (TDMA_KF forward, TDMA_KBK
-    // backward, where the batch holds doubles): the loads of a batch do not
-    // depend on the recurrence, so they are issued together and the few
-    // threads of this kernel (one per column group) keep enough bytes in
-    // flight to stream from HBM instead of waiting one level at a time.
-    constexpr int TDMA_KF = 8;
-    constexpr int TDMA_KBK = 4;
-
-    // Output of column col at level k.  The mean mode (col 0) is not stored:
-    // its level mean (X_00/jtot)/itot goes to dcm[k] and the column gets
-    // zero, so that the inverse transforms carry only the other modes and the
-    // large hydrostatic part of p stays out of their round-off; the inverse
-    // x transform (or the scatter) adds the mean to every point.
-    template<typename TF>
-    __device__ __forceinline__ TF dc_out(TF val, int col, int k, int itot, int jtot, TF* __restrict__ dcm)
-    {
-        if (col != 0) return val;
-        dcm[k] = TF((double(val) / jtot) / itot);
-        return TF(0);
-    }
-
-    template<typename TF> struct TdmaP
-    {
-        int itot, jtot, ktot, niu, nju;
-        const double *rtab, *wtab, *a, *dz2, *gtab, *htab;
-        const float* stab;
-        const double* stabd;
-        TF* pk; double* work; TF* dcm;
-        const float *gftab, *hftab;
-        const unsigned char* fmode;
-    };
-
-    template<typename TF>
-    __device__ __forceinline__ void tdma_body(const TdmaP<TF>& A, const VBlock& vb)
-    {
-        const int itot = A.itot, jtot = A.jtot, ktot = A.ktot, niu = A.niu, nju = A.nju;
-        const double* __restrict__ rtab = A.rtab; const double* __restrict__ wtab = A.wtab;
-        const double* __restrict__ a = A.a; const double* __restrict__ dz2 = A.dz2;
-        TF* __restrict__ pk = A.pk; double* __restrict__ work = A.work; TF* __restrict__ dcm = A.dcm;
-        const int iu = vb.x*blockDim.x + threadIdx.x;
-        const int ju = vb.y;
-        if (iu >= niu) return;
-        const long long stride = (long long)niu*nju;
-        const long long base = iu + (long long)ju*niu;
-        const long long kk = (long long)itot*jtot;
-        const int i1 = (iu == 0 || 2*iu == itot) ? -1 : itot - iu;
-        const int j1 = (ju == 0 || 2*ju == jtot) ? -1 : jtot - ju;
-        // The group's columns (i, j), (itot-i, j), (i, jtot-j), (itot-i, jtot-j);
-        // a column that coincides with the first is masked out.  Column
-        // offsets within a level are 32-bit (itot*jtot < 2^31 is checked at
-        // set-up); level offsets are 64-bit pointers.
-        const bool use[4] = {true, i1 >= 0, j1 >= 0, i1 >= 0 && j1 >= 0};
-        const int ia = iu, ib = i1 >= 0 ? i1 : iu;
-        const int ja = ju*itot, jb = (j1 >= 0 ? j1 : ju)*itot;
-        const int col[4] = {ia + ja, ib + ja, ia + jb, ib + jb};
-
-        // Forward sweep: y_k = (dz2_k p_k - a_k y_{k-1}) / den_k, rounded
-        // after each operation as in src/pres_2.cxx:200-263.
-        double y[4] = {0., 0., 0., 0.};
-        for (int k0=0; k0<ktot; k0+=TDMA_KF)
-        {
-            const int nk = min(TDMA_KF, ktot - k0);
-            double r[TDMA_KF];
-            TF pv[TDMA_KF][4];
-            #pragma unroll
-            for (int b=0; b<TDMA_KF; ++b)
-            {
-                if (b < nk)
-                {
-                    const long long k = k0 + b;
-                    r[b] = __ldg(&rtab[base + k*stride]);
-                    const TF* row = pk + k*kk;
-                    #pragma unroll
-                    for (int q=0; q<4; ++q)
-                        if (use[q]) pv[b][q] = row[col[q]];
-                }
-            }
-            #pragma unroll
-            for (int b=0; b<TDMA_KF; ++b)
-            {
-                if (b < nk)
-                {
-                    const int k = k0 + b;
-                    const double dzk = dz2[k];
-                    const double ak = a[k];
-                    double* wrow = work + (long long)k*kk;
-                    #pragma unroll
-                    for (int q=0; q<4; ++q)
-                    {
-                        if (use[q])
-                        {
-                            double x = mulx(dzk, double(pv[b][q]));
-                            if (k) x = x - mulx(ak, y[q]);
-                            y[q] = x / r[b];
-                            wrow[col[q]] = y[q];
-                        }
-                    }
-                }
-            }
-        }
-        // Back substitution: x_k = y_k - (c_k/den_k) x_{k+1}.
-        {
-            TF* row = pk + (long long)(ktot-1)*kk;
-            #pragma unroll
-            for (int q=0; q<4; ++q)
-                if (use[q]) row[col[q]] = dc_out<TF>(TF(y[q]), col[q], ktot-1, itot, jtot, dcm);
-        }
-        for (int k0=ktot-2; k0>=0; k0-=TDMA_KBK)
-        {
-            const int nk = min(TDMA_KBK, k0 + 1);
-            double r[TDMA_KBK];
-            double wv[TDMA_KBK][4];
-            #pragma unroll
-            for (int b=0; b<TDMA_KBK; ++b)
-            {
-                if (b < nk)
-                {
-                    const long long k = k0 - b;
-                    r[b] = __ldg(&wtab[base + k*stride]);
-                    const double* wrow = work + k*kk;
-                    #pragma unroll
-                    for (int q=0; q<4; ++q)
-                        if (use[q]) wv[b][q] = wrow[col[q]];
-                }
-            }
-            #pragma unroll
-            for (int b=0; b<TDMA_KBK; ++b)
-            {
-                if (b < nk)
-                {
-                    const int k = k0 - b;
-                    const double w3 = r[b];
-                    TF* row = pk + (long long)k*kk;
-                    #pragma unroll
-                    for (int q=0; q<4; ++q)
-                    {
-                        if (use[q])
-                        {
-                            y[q] = wv[b][q] - mulx(w3, y[q]);
-                            row[col[q]] = dc_out<TF>(TF(y[q]), col[q], k, itot, jtot, dcm);
-                        }
-                    }
-                }
-            }
-        }
-    }
-
-    template<typename TF> __device__ __forceinline__ double to_f64(TF v);
-    template<> __device__ __forceinline__ double to_f64<float>(float v) { return f2d_exact(v); }
-    template<> __device__ __forceinline__ double to_f64<double>(double v) { return v; }
-
-    // Output x_k = s_k xi_k in the field precision: in float the product of
-    // the rounded factors (the result is stored in float anyway).
-    template<typename TF> __device__ __forceinline__ TF scale_out(double xi, float s, double sd);
-    template<> __device__ __forceinline__ float scale_out<float>(double xi, float s, double) { return d2f_rn(xi)*s; }
-    template<> __device__ __forceinline__ double scale_out<double>(double xi, float, double sd) { return xi*sd; }
-
-    // The Thomas solve with the rescaled recurrence (coefficients from
-    // k_tdma_table): in the float form the whole solve costs two FP64 FMAs
-    // per cell, the elimination itself staying in double.
-    template<typename TF>
-    __device__ __forceinline__ void tdma_scaled_body(const TdmaP<TF>& A, const VBlock& vb)
-    {
-        const int itot = A.itot, jtot = A.jtot, ktot = A.ktot, niu = A.niu, nju = A.nju;
-        const double* __restrict__ gtab = A.gtab; const double* __restrict__ htab = A.htab;
-        const float* __restrict__ stab = A.stab; const double* __restrict__ stabd = A.stabd;
-        TF* __restrict__ pk = A.pk; double* __restrict__ work = A.work; TF* __restrict__ dcm = A.dcm;
-        const int iu = vb.x*blockDim.x + threadIdx.x;
-        const int ju = vb.y;
-        if (iu >= niu) return;
-        const long long stride = (long long)niu*nju;
-        const long long base = iu + (long long)ju*niu;
-        const long long kk = (long long)itot*jtot;
-        const int i1 = (iu == 0 || 2*iu == itot) ? -1 : itot - iu;
-        const int j1 = (ju == 0 || 2*ju == jtot) ? -1 : jtot - ju;
-        const bool use[4] = {true, i1 >= 0, j1 >= 0, i1 >= 0 && j1 >= 0};
-        const int ia = iu, ib = i1 >= 0 ? i1 : iu;
-        const int ja = ju*itot, jb = (j1 >= 0 ? j1 : ju)*itot;
-        const int col[4] = {ia + ja, ib + ja, ia + jb, ib + jb};
-
-        // Forward: z_k = p_k - g_k z_{k-1}.
-        double z[4] = {0., 0., 0., 0.};
-        for (int k0=0; k0<ktot; k0+=TDMA_KF)
-        {
-            const int nk = min(TDMA_KF, ktot - k0);
-            double g[TDMA_KF];
-            TF pv[TDMA_KF][4];
-            #pragma unroll
-            for (int b=0; b<TDMA_KF; ++b)
-            {
-                if (b < nk)
-                {
-                    const long long k = k0 + b;
-                    g[b] = __ldg(&gtab[base + k*stride]);
-                    const TF* row = pk + k*kk;
-                    #pragma unroll
-                    for (int q=0; q<4; ++q)
-                        if (use[q]) pv[b][q] = row[col[q]];
-                }
-            }
-            #pragma unroll
-            for (int b=0; b<TDMA_KF; ++b)
-            {
-                if (b < nk)
-                {
-                    double* wrow = work + (long long)(k0 + b)*kk;
-                    #pragma unroll
-                    for (int q=0; q<4; ++q)
-                    {
-                        if (use[q])
-                        {
-                            z[q] = fma(-g[b], z[q], to_f64<TF>(pv[b][q]));
-                            wrow[col[q]] = z[q];
-                        }
-                    }
-                }
-            }
-        }
-        // Backward: xi_k = z_k - h_k xi_{k+1}; x_k = s_k xi_k.
-        {
-            const long long k = ktot - 1;
-            const float s = __ldg(&stab[base + k*stride]);
-            const double sd = sizeof(TF) == 8 ? __ldg(&stabd[base + k*stride]) : 0.;
-            TF* row = pk + k*kk;
-            #pragma unroll
-            for (int q=0; q<4; ++q)
-                if (use[q]) row[col[q]] = dc_out<TF>(scale_out<TF>(z[q], s, sd), col[q], (int)k, itot, jtot, dcm);
-        }
-        for (int k0=ktot-2; k0>=0; k0-=TDMA_KBK)
-        {
-            const int nk = min(TDMA_KBK, k0 + 1);
-            double h[TDMA_KBK], sd[TDMA_KBK];
-            float s[TDMA_KBK];
-            double zv[TDMA_KBK][4];
-            #pragma unroll
-            for (int b=0; b<TDMA_KBK; ++b)
-            {
-                if (b < nk)
-                {
-                    const long long k = k0 - b;
-                    h[b] = __ldg(&htab[base + k*stride]);
-                    s[b] = __ldg(&stab[base + k*stride]);
-                    sd[b] = sizeof(TF) == 8 ? __ldg(&stabd[base + k*stride]) : 0.;
-                    const double* wrow = work + k*kk;
-                    #pragma unroll
-                    for (int q=0; q<4; ++q)
-                        if (use[q]) zv[b][q] = wrow[col[q]];
-                }
-            }
-            #pragma unroll
-            for (int b=0; b<TDMA_KBK; ++b)
-            {
-                if (b < nk)
-                {
-                    TF* row = pk + (long long)(k0 - b)*kk;
-                    #pragma unroll
-                    for (int q=0; q<4; ++q)
-                    {
-                        if (use[q])
-                        {
-                            z[q] = fma(-h[b], z[q], zv[b][q]);
-                            row[col[q]] = dc_out<TF>(scale_out<TF>(z[q], s[b], sd[b]), col[q], k0 - b, itot, jtot, dcm);
-                        }
-                    }
-                }
-            }
-        }
-    }
-
-    // The rescaled solve with one column per thread: the four columns that
-    // share the coefficients of one eigenvalue (i, itot-i) x (j, jtot-j) sit
-    // in four adjacent lanes, which read the same table entries in one
-    // transaction.  Four times the threads of k_tdma_scaled, so that the FP64
-    // recurrences and the loads of the next levels of other warps overlap.
-    constexpr int TDC_KF = 8;
-    constexpr int TDC_KB = 4;
-
-    template<typename TF>
-    __device__ __forceinline__ void tdma_col_fp64(const TdmaP<TF>& A, int col, long long base);
-
-    // At most 64 registers, so that eight blocks (32 warps) fit on an SM:
-    // the loads of one warp's next levels overlap the FP64 recurrences of
-    // the others.
-    template<typename TF>
-    __device__ __forceinline__ void tdma_col_body(const TdmaP<TF>& A, const VBlock& vb)
-    {
-        const int itot = A.itot, jtot = A.jtot, niu = A.niu;
-        const int t = vb.x*blockDim.x + threadIdx.x;
-        const int iu = t >> 2, q = t & 3;
-        const int ju = vb.y;
-        if (iu >= niu) return;
-        const int i1 = (iu == 0 || 2*iu == itot) ? -1 : itot - iu;
-        const int j1 = (ju == 0 || 2*ju == jtot) ? -1 : jtot - ju;
-        // Lane q holds column (q&1 ? itot-i : i, q&2 ? jtot-j : j); a mirror
-        // that coincides with the first column has no lane.
-        if (((q & 1) && i1 < 0) || ((q & 2) && j1 < 0)) return;
-        const int col = ((q & 1) ? i1 : iu) + ((q & 2) ? j1 : ju)*itot;
-        tdma_col_fp64<TF>(A, col, iu + (long long)ju*niu);
-    }
-
-    // One column's rescaled solve with the elimination in FP64 (forward
-    // values in the FP64 work array).
-    template<typename TF>
-    __device__ __forceinline__ void tdma_col_fp64(const TdmaP<TF>& A, int col, long long base)
-    {
-        const int itot = A.itot, jtot = A.jtot, ktot = A.ktot;
-        const double* __restrict__ gtab = A.gtab; const double* __restrict__ htab = A.htab;
-        const float* __restrict__ stab = A.stab; const double* __restrict__ stabd = A.stabd;
-        TF* __restrict__ pk = A.pk; double* __restrict__ work = A.work; TF* __restrict__ dcm = A.dcm;
-        const long long stride = (long long)A.niu*A.nju;
-        const long long kk = (long long)itot*jtot;
-
-        // Forward: z_k = p_k - g_k z_{k-1}.
-        double z = 0.;
-        for (int k0=0; k0<ktot; k0+=TDC_KF)
-        {
-            const int nk = min(TDC_KF, ktot - k0);
-            double g[TDC_KF];
-            TF pv[TDC_KF];
-            #pragma unroll
-            for (int b=0; b<TDC_KF; ++b)
-                if (b < nk)
-                {
-                    g[b] = __ldg(gtab + base + (long long)(k0 + b)*stride);
-                    pv[b] = pk[col + (long long)(k0 + b)*kk];
-                }
-            #pragma unroll
-            for (int b=0; b<TDC_KF; ++b)
-                if (b < nk)
-                {
-                    z = fma(-g[b], z, to_f64<TF>(pv[b]));
-                    work[col + (long long)(k0 + b)*kk] = z;
-                }
-        }
-        // Backward: xi_k = z_k - h_k xi_{k+1}; x_k = s_k xi_k.
-        {
-            const long long k = ktot - 1;
-            const float s = __ldg(stab + base + k*stride);
-            const double sd = sizeof(TF) == 8 ? __ldg(stabd + base + k*stride) : 0.;
-            pk[col + k*kk] = dc_out<TF>(scale_out<TF>(z, s, sd), col, (int)k, itot, jtot, dcm);
-        }
-        for (int k0=ktot-2; k0>=0; k0-=TDC_KB)
-        {
-            const int nk = min(TDC_KB, k0 + 1);
-            double h[TDC_KB], sd[TDC_KB], zv[TDC_KB];
-            float s[TDC_KB];
-            #pragma unroll
-            for (int b=0; b<TDC_KB; ++b)
-                if (b < nk)
-                {
-                    const long long k = k0 - b;
-                    h[b] = __ldg(htab + base + k*stride);
-                    s[b] = __ldg(stab + base + k*stride);
-                    sd[b] = sizeof(TF) == 8 ? __ldg(stabd + base + k*stride) : 0.;
-                    zv[b] = work[col + k*kk];
-                }
-            #pragma unroll
-            for (int b=0; b<TDC_KB; ++b)
-                if (b < nk)
-                {
-                    z = fma(-h[b], z, zv[b]);
-                    pk[col + (long long)(k0 - b)*kk] = dc_out<TF>(scale_out<TF>(z, s[b], sd[b]), col, k0 - b, itot, jtot, dcm);
-                }
-        }
-    }
-
-    // The rescaled solve in float for the column groups whose sweeps damp
-    // (fmode, set with the tables), in FP64 for the others.  A float column
-    // keeps its forward values in pk itself, where the backward sweep
-    // overwrites them with the solution: 16 bytes per cell move instead of
-    // 24 (float right-hand side and solution, FP64 work array), the tables
-    // are read in float, no FP64 instruction runs, and the loads run sixteen
-    // levels ahead of the recurrence.  Lanes as in k_tdma_col; a group's
-    // four lanes take the same branch.
-    constexpr int TDF_KF = 16;
-    constexpr int TDF_KB = 8;
-
-    __device__ __forceinline__ void tdma_mixed_body(const TdmaP<float>& A, const VBlock& vb)
-    {
-        const int itot = A.itot, jtot = A.jtot, ktot = A.ktot, niu = A.niu;
-        const int t = vb.x*blockDim.x + threadIdx.x;
-        const int iu = t >> 2, q = t & 3;
-        const int ju = vb.y;
-        if (iu >= niu) return;
-        const int i1 = (iu == 0 || 2*iu == itot) ? -1 : itot - iu;
-        const int j1 = (ju == 0 || 2*ju == jtot) ? -1 : jtot - ju;
-        if (((q & 1) && i1 < 0) || ((q & 2) && j1 < 0)) return;
-        const int col = ((q & 1) ? i1 : iu) + ((q & 2) ? j1 : ju)*itot;
-        const long long base = iu + (long long)ju*niu;
-        if (!A.fmode[base])
-        {
-            tdma_col_fp64<float>(A, col, base);
-            return;
-        }
-        const float* __restrict__ gf = A.gftab; const float* __restrict__ hf = A.hftab;
-        const float* __restrict__ stab = A.stab;
-        float* __restrict__ pk = A.pk;
-        const long long stride = (long long)niu*A.nju;
-        const long long kk = (long long)itot*jtot;
-
-        // Forward: z_k = p_k - g_k z_{k-1}, stored over p_k.
-        float z = 0.f;
-        for (int k0=0; k0<ktot; k0+=TDF_KF)
-        {
-            const int nk = min(TDF_KF, ktot - k0);
-            float g[TDF_KF], pv[TDF_KF];
-            #pragma unroll
-            for (int b=0; b<TDF_KF; ++b)
-                if (b < nk)
-                {
-                    g[b] = __ldg(gf + base + (long long)(k0 + b)*stride);
-                    pv[b] = pk[col + (long long)(k0 + b)*kk];
-                }
-            #pragma unroll
-            for (int b=0; b<TDF_KF; ++b)
-                if (b < nk)
-                {
-                    z = fmaf(-g[b], z, pv[b]);
-                    pk[col + (long long)(k0 + b)*kk] = z;
-                }
-        }
-        // Backward: xi_k = z_k - h_k xi_{k+1}; x_k = s_k xi_k.
-        pk[col + (long long)(ktot - 1)*kk] = z*__ldg(stab + base + (long long)(ktot - 1)*stride);
-        float xi = z;
-        for (int k0=ktot-2; k0>=0; k0-=TDF_KB)
-        {
-            const int nk = min(TDF_KB, k0 + 1);
-            float h[TDF_KB], sv[TDF_KB], zv[TDF_KB];
-            #pragma unroll
-            for (int b=0; b<TDF_KB; ++b)
-                if (b < nk)
-                {
-                    const long long k = k0 - b;
-                    h[b] = __ldg(hf + base + k*stride);
-                    sv[b] = __ldg(stab + base + k*stride);
-                    zv[b] = pk[col + k*kk];
-                }
-            #pragma unroll
-            for (int b=0; b<TDF_KB; ++b)
-                if (b < nk)
-                {
-                    xi = fmaf(-h[b], xi, zv[b]);
-                    pk[col + (long long)(k0 - b)*kk] = xi*sv[b];
-                }
-        }
-    }
-
-    int tdma_table(PresWork& pw, int itot, int jtot, int ktot, cudaStream_t s)
-    {
-        pw.niu = itot/2 + 1;
-        pw.nju = jtot/2 + 1;
-        const size_t n = (size_t)pw.niu*pw.nju*ktot;
-        if (cudaMallocAsync((void**)&pw.rtab, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.wtab, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.gtab, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.htab, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.stab, sizeof(float)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.stabd, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.gftab, sizeof(float)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.hftab, sizeof(float)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.fmode, (size_t)pw.niu*pw.nju, s) != cudaSuccess) return MHH_ERR_CUDA;
-        dim3 grid((pw.niu + 127)/128, pw.nju);
-        k_tdma_table<<<grid, 128, 0, s>>>(pw.niu, pw.nju, ktot, pw.bmati, pw.bmatj, pw.a, pw.c, pw.dz2rho, pw.dz2,
-                                    pw.rtab, pw.wtab, pw.gtab, pw.htab, pw.stab, pw.stabd, pw.gftab, pw.hftab,
-                                    pw.fmode);
-        count_launch();
-        return cudaStreamSynchronize(s) == cudaSuccess ? MHH_OK : MHH_ERR_CUDA;
-    }
-
-    template<typename TF>
-    void launch_tdma(const Dims& d, const PresWork& pw, TF* pk, const KernelOpts& o, cudaStream_t s)
-    {
-        dim3 grid((pw.niu + 127)/128, pw.nju);
-        TF* dcm = static_cast<TF*>(pw.dcm);
-        int v = o.tdma < 0 ? (sizeof(TF) == 4 ? 3 : 0) : o.tdma;
-        if (v == 3 && sizeof(TF) == 8) v = 1;
-        const TdmaP<TF> A{d.itot, d.jtot, d.ktot, pw.niu, pw.nju, pw.rtab, pw.wtab, pw.a, pw.dz2, pw.gtab, pw.htab,
-                          pw.stab, pw.stabd, pk, pw.work, dcm, pw.gftab, pw.hftab, pw.fmode};
-        if constexpr (sizeof(TF) == 4)
-        {
-            if (v == 3)
-            {
-                dim3 gridc((4*pw.niu + 127)/128, pw.nju);
-                launch_body<TdmaP<float>, tdma_mixed_body, 128, 8>(gridc, dim3(128), 0, s, A);
-                count_launch();
-                return;
-            }
-        }
-        if (v == 1)
-        {
-            dim3 gridc((4*pw.niu + 127)/128, pw.nju);
-            launch_body<TdmaP<TF>, tdma_col_body<TF>, 128, 8>(gridc, dim3(128), 0, s, A);
-        }
-        else if (v == 2)
-            launch_body<TdmaP<TF>, tdma_scaled_body<TF>, 128>(grid, dim3(128), 0, s, A);
-        else
-            launch_body<TdmaP<TF>, tdma_body<TF>, 128>(grid, dim3(128), 0, s, A);
-        count_launch();
-    }
-
     // Packed solution back into the ghost layout with the bottom ghost level
     // p[kstart-1] = p[kstart], src/pres_2.cxx:330-358 (the periodic fill
     // follows separately).
@@ -1882,9 +1296,13 @@ namespace mhh
     template void launch_pres_in<TF>(const Dims&, const Prof<TF>&, const TF*, const TF*, const TF*, const TF*, const TF*, const TF*, TF*, double, cudaStream_t); \
     template void launch_fft_x<TF>(const FftPlan&, TF*, int, bool, double, cudaStream_t, const FftFuse<TF>*); \
     template void launch_fft_y<TF>(const FftPlan&, TF*, int, int, int, bool, double, cudaStream_t); \
-    template void launch_tdma<TF>(const Dims&, const PresWork&, TF*, const KernelOpts&, cudaStream_t); \
     template void launch_pres_scatter<TF>(const Dims&, const TF*, const TF*, TF*, cudaStream_t);
 
+    // Compiled once per precision (MHH_PREC, set by the build) to keep the
+    // build short.
+#if MHH_PREC == 64
     MHH_PRES_INST(double)
+#else
     MHH_PRES_INST(float)
+#endif
 }

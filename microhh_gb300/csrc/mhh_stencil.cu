@@ -804,6 +804,11 @@ namespace mhh
     template void launch_presout_rk3<TF>(const Dims&, const Prof<TF>&, const TF*, TF*, TF*, TF*, TF*, TF*, TF*, TF*, TF*, int, double, cudaStream_t); \
     template void launch_reduce<TF>(int, const Dims&, const Prof<TF>&, const TF*, const TF*, const TF*, const TF*, double, unsigned long long*, cudaStream_t);
 
+    // Compiled once per precision (MHH_PREC, set by the build) to keep the
+    // build short.
+#if MHH_PREC == 64
     MHH_INSTANTIATE(double)
+#else
     MHH_INSTANTIATE(float)
+#endif
 }
