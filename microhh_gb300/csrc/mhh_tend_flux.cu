@@ -184,6 +184,15 @@ namespace mhh
         cp_async_wait_all();
         __syncthreads();
 
+        // Double form: the viscosity sums of the own faces at levels m and m+1.
+        TF ex0 = 0, ey0 = 0, ex1 = 0, ey1 = 0;
+        if (sizeof(TF) == 8 && face)
+        {
+            const TF* E = sm + (SE + m0%4)*FPS + pc;
+            ex0 = E[-1] + E[0];
+            ey0 = E[-FPW] + E[0];
+        }
+
         for (int m = m0; m < k1; ++m)
         {
             const int buf = (m - m0) & 1;
@@ -225,29 +234,19 @@ namespace mhh
             TF txz = 0, tyz = 0;
             if (face)
             {
-                const TF txy = (TF(0.25)*(PL(E0,-1,-1) + PL(E0,0,-1) + PL(E0,-1,0) + PL(E0,0,0)) + visc)
-                             * ((PL(U0,0,0) - PL(U0,0,-1))*dyi + (PL(V0,0,0) - PL(V0,-1,0))*dxi);
                 if constexpr (sizeof(TF) == 4)
                 {
+                    const TF txy = (TF(0.25)*(PL(E0,-1,-1) + PL(E0,0,-1) + PL(E0,-1,0) + PL(E0,0,0)) + visc)
+                                 * ((PL(U0,0,0) - PL(U0,0,-1))*dyi + (PL(V0,0,0) - PL(V0,-1,0))*dxi);
                     // tau_xz and tau_yz in one packed pair.
-                    const float2 e = __ffma2_rn(__fadd2_rn(__fadd2_rn(f2(PL(E0,-1,0), PL(E0,0,-1)), f2(PL(E0,0,0), PL(E0,0,0))),
-                                                           __fadd2_rn(f2(PL(E1,-1,0), PL(E1,0,-1)), f2(PL(E1,0,0), PL(E1,0,0)))),
-                                                f2(0.25f, 0.25f), f2(visc, visc));
-                    const float2 g = __ffma2_rn(sub2(f2(PL(U1,0,0), PL(V1,0,0)), f2(PL(U0,0,0), PL(V0,0,0))), f2(dzhi1, dzhi1),
-                                                __fmul2_rn(sub2(f2(PL(W1,0,0), PL(W1,0,0)), f2(PL(W1,-1,0), PL(W1,0,-1))),
-                                                           f2(dxi, dyi)));
-                    const float2 t = __fmul2_rn(e, g);
-                    txz = t.x; tyz = t.y;
-                }
-                else
-                {
-                    txz = (TF(0.25)*(PL(E0,-1,0) + PL(E0,0,0) + PL(E1,-1,0) + PL(E1,0,0)) + visc)
-                        * ((PL(U1,0,0) - PL(U0,0,0))*dzhi1 + (PL(W1,0,0) - PL(W1,-1,0))*dxi);
-                    tyz = (TF(0.25)*(PL(E0,0,-1) + PL(E0,0,0) + PL(E1,0,-1) + PL(E1,0,0)) + visc)
-                        * ((PL(V1,0,0) - PL(V0,0,0))*dzhi1 + (PL(W1,0,0) - PL(W1,0,-1))*dyi);
-                }
-                if constexpr (sizeof(TF) == 4)
-                {
+                    const float2 ez = __ffma2_rn(__fadd2_rn(__fadd2_rn(f2(PL(E0,-1,0), PL(E0,0,-1)), f2(PL(E0,0,0), PL(E0,0,0))),
+                                                            __fadd2_rn(f2(PL(E1,-1,0), PL(E1,0,-1)), f2(PL(E1,0,0), PL(E1,0,0)))),
+                                                 f2(0.25f, 0.25f), f2(visc, visc));
+                    const float2 gz = __ffma2_rn(sub2(f2(PL(U1,0,0), PL(V1,0,0)), f2(PL(U0,0,0), PL(V0,0,0))), f2(dzhi1, dzhi1),
+                                                 __fmul2_rn(sub2(f2(PL(W1,0,0), PL(W1,0,0)), f2(PL(W1,-1,0), PL(W1,0,-1))),
+                                                            f2(dxi, dyi)));
+                    const float2 tz = __fmul2_rn(ez, gz);
+                    txz = tz.x; tyz = tz.y;
                     // Float form: the x- and y-face advective fluxes of each
                     // field in packed pairs (both computed by every face
                     // thread; the plane holds the stencils of the edge faces).
@@ -297,64 +296,68 @@ namespace mhh
                 }
                 else
                 {
+                    // Double form, bound by the FP64 pipe: sums of the eddy
+                    // viscosity at the face's two cells shared between the
+                    // stresses and carried up a level, constant factors
+                    // folded, each flux one FMA off its advective part.
+                    ex1 = PL(E1,-1,0) + PL(E1,0,0);
+                    ey1 = PL(E1,0,-1) + PL(E1,0,0);
+                    const TF txy = fma(ex0 + (PL(E0,-1,-1) + PL(E0,0,-1)), TF(0.25), visc)
+                                 * fma(PL(V0,0,0) - PL(V0,-1,0), dxi, (PL(U0,0,0) - PL(U0,0,-1))*dyi);
                     if (face_x)
                     {
+                        txz = fma(ex0 + ex1, TF(0.25), visc)
+                            * fma(PL(W1,0,0) - PL(W1,-1,0), dxi, (PL(U1,0,0) - PL(U0,0,0))*dzhi1);
                         // u at the cell centre i-1.
                         {
-                            const TF uw = i2(PL(U0,-1,0), PL(U0,0,0));
-                            const TF A = adv6(uw, PL(U0,-3,0), PL(U0,-2,0), PL(U0,-1,0), PL(U0,0,0), PL(U0,1,0), PL(U0,2,0));
-                            const TF D = TF(2)*(PL(E0,-1,0) + visc)*(PL(U0,0,0) - PL(U0,-1,0))*dxi;
-                            gx[(gxi)*4 + 0] = D - A;
+                            const TF uw = PL(U0,-1,0) + PL(U0,0,0);
+                            const TF A = uw*upwind5<true>(uw, PL(U0,-3,0), PL(U0,-2,0), PL(U0,-1,0), PL(U0,0,0), PL(U0,1,0), PL(U0,2,0));
+                            gx[(gxi)*4 + 0] = fma(fma(PL(E0,-1,0), TF(2)*dxi, TF(2)*dxi*visc), PL(U0,0,0) - PL(U0,-1,0), -A);
                         }
                         // v at (i-1/2, j-1/2).
                         {
-                            const TF uw = i2(PL(U0,0,-1), PL(U0,0,0));
-                            const TF A = adv6(uw, PL(V0,-3,0), PL(V0,-2,0), PL(V0,-1,0), PL(V0,0,0), PL(V0,1,0), PL(V0,2,0));
-                            gx[(gxi)*4 + 1] = txy - A;
+                            const TF uw = PL(U0,0,-1) + PL(U0,0,0);
+                            gx[(gxi)*4 + 1] = fma(-uw, upwind5<true>(uw, PL(V0,-3,0), PL(V0,-2,0), PL(V0,-1,0), PL(V0,0,0), PL(V0,1,0), PL(V0,2,0)), txy);
                         }
                         // w at (i-1/2, m+1/2).
                         {
-                            const TF uw = i2(PL(U0,0,0), PL(U1,0,0));
-                            const TF A = adv6(uw, PL(W1,-3,0), PL(W1,-2,0), PL(W1,-1,0), PL(W1,0,0), PL(W1,1,0), PL(W1,2,0));
-                            gx[(gxi)*4 + 2] = txz - A;
+                            const TF uw = PL(U0,0,0) + PL(U1,0,0);
+                            gx[(gxi)*4 + 2] = fma(-uw, upwind5<true>(uw, PL(W1,-3,0), PL(W1,-2,0), PL(W1,-1,0), PL(W1,0,0), PL(W1,1,0), PL(W1,2,0)), txz);
                         }
                         if (SCAL)
                         {
                             const TF uw = PL(U0,0,0);
                             const TF A = LIM ? lim_flux(uw, PL(S0,-2,0), PL(S0,-1,0), PL(S0,0,0), PL(S0,1,0), 0)
-                                             : adv6(uw, PL(S0,-3,0), PL(S0,-2,0), PL(S0,-1,0), PL(S0,0,0), PL(S0,1,0), PL(S0,2,0));
-                            const TF D = (TF(0.5)*(PL(E0,-1,0) + PL(E0,0,0))*tpri + svisc)*(PL(S0,0,0) - PL(S0,-1,0))*dxi;
-                            gx[(gxi)*4 + 3] = D - A;
+                                             : uw*upwind5<false>(uw, PL(S0,-3,0), PL(S0,-2,0), PL(S0,-1,0), PL(S0,0,0), PL(S0,1,0), PL(S0,2,0));
+                            gx[(gxi)*4 + 3] = fma(fma(ex0, TF(0.5)*tpri*dxi, svisc*dxi), PL(S0,0,0) - PL(S0,-1,0), -A);
                         }
                     }
                     if (face_y)
                     {
+                        tyz = fma(ey0 + ey1, TF(0.25), visc)
+                            * fma(PL(W1,0,0) - PL(W1,0,-1), dyi, (PL(V1,0,0) - PL(V0,0,0))*dzhi1);
                         // u at (i-1/2, j-1/2).
                         {
-                            const TF vs = i2(PL(V0,-1,0), PL(V0,0,0));
-                            const TF A = adv6(vs, PL(U0,0,-3), PL(U0,0,-2), PL(U0,0,-1), PL(U0,0,0), PL(U0,0,1), PL(U0,0,2));
-                            gy[(gyi)*4 + 0] = txy - A;
+                            const TF vs = PL(V0,-1,0) + PL(V0,0,0);
+                            gy[(gyi)*4 + 0] = fma(-vs, upwind5<true>(vs, PL(U0,0,-3), PL(U0,0,-2), PL(U0,0,-1), PL(U0,0,0), PL(U0,0,1), PL(U0,0,2)), txy);
                         }
                         // v at the cell centre j-1.
                         {
-                            const TF vs = i2(PL(V0,0,-1), PL(V0,0,0));
-                            const TF A = adv6(vs, PL(V0,0,-3), PL(V0,0,-2), PL(V0,0,-1), PL(V0,0,0), PL(V0,0,1), PL(V0,0,2));
-                            const TF D = TF(2)*(PL(E0,0,-1) + visc)*(PL(V0,0,0) - PL(V0,0,-1))*dyi;
-                            gy[(gyi)*4 + 1] = D - A;
+                            const TF vs = PL(V0,0,-1) + PL(V0,0,0);
+                            const TF A = vs*upwind5<true>(vs, PL(V0,0,-3), PL(V0,0,-2), PL(V0,0,-1), PL(V0,0,0), PL(V0,0,1), PL(V0,0,2));
+                            gy[(gyi)*4 + 1] = fma(fma(PL(E0,0,-1), TF(2)*dyi, TF(2)*dyi*visc), PL(V0,0,0) - PL(V0,0,-1), -A);
                         }
                         // w at (j-1/2, m+1/2).
                         {
-                            const TF vs = i2(PL(V0,0,0), PL(V1,0,0));
-                            const TF A = adv6(vs, PL(W1,0,-3), PL(W1,0,-2), PL(W1,0,-1), PL(W1,0,0), PL(W1,0,1), PL(W1,0,2));
-                            gy[(gyi)*4 + 2] = tyz - A;
+                            const TF vs = PL(V0,0,0) + PL(V1,0,0);
+                            gy[(gyi)*4 + 2] = fma(-vs, upwind5<true>(vs, PL(W1,0,-3), PL(W1,0,-2), PL(W1,0,-1), PL(W1,0,0), PL(W1,0,1), PL(W1,0,2)), tyz);
                         }
                         if (SCAL)
                         {
                             const TF vs = PL(V0,0,0);
                             const TF A = LIM ? lim_flux(vs, PL(S0,0,-2), PL(S0,0,-1), PL(S0,0,0), PL(S0,0,1), 0)
-                                             : adv6(vs, PL(S0,0,-3), PL(S0,0,-2), PL(S0,0,-1), PL(S0,0,0), PL(S0,0,1), PL(S0,0,2));
-                            const TF D = (TF(0.5)*(PL(E0,0,-1) + PL(E0,0,0))*tpri + svisc)*(PL(S0,0,0) - PL(S0,0,-1))*dyi;
-                            gy[(gyi)*4 + 3] = D - A;
+                                             : vs*upwind5<false>(vs, PL(S0,0,-3), PL(S0,0,-2), PL(S0,0,-1), PL(S0,0,0), PL(S0,0,1), PL(S0,0,2));
+                            gy[(gyi)*4 + 3] = fma(fma(ey0, TF(0.5)*tpri*dyi, svisc*dyi), PL(S0,0,0) - PL(S0,0,-1), -A);
                         }
                     }
                 }
@@ -379,8 +382,17 @@ namespace mhh
                 }
                 else
                 {
-                    gzu_t = rhoh1*(du - zadv(qu, i2(PL(W1,-1,0), PL(W1,0,0)), ot));
-                    gzv_t = rhoh1*(dv - zadv(qv, i2(PL(W1,0,-1), PL(W1,0,0)), ot));
+                    const TF wu = PL(W1,-1,0) + PL(W1,0,0), wv = PL(W1,0,-1) + PL(W1,0,0);
+                    if (ot == 6)
+                    {
+                        gzu_t = rhoh1*fma(-wu, upwind5<true>(wu, qu[0], qu[1], qu[2], qu[3], qu[4], qu[5]), du);
+                        gzv_t = rhoh1*fma(-wv, upwind5<true>(wv, qv[0], qv[1], qv[2], qv[3], qv[4], qv[5]), dv);
+                    }
+                    else
+                    {
+                        gzu_t = rhoh1*(du - zadv(qu, TF(0.5)*wu, ot));
+                        gzv_t = rhoh1*(dv - zadv(qv, TF(0.5)*wv, ot));
+                    }
                 }
                 // Float form, interior levels: the vertical advective fluxes of
                 // w (through full level kf) and of s (through half level kf),
@@ -407,6 +419,8 @@ namespace mhh
                         const int side = kf == d.kstart+1 ? -1 : (kf == d.kend-1 ? 1 : 0);
                         as = ot ? lim_flux(qw[2], qs[1], qs[2], qs[3], qs[4], side) : TF(0);
                     }
+                    else if (sizeof(TF) == 8 && ot == 6)
+                        as = qw[2]*upwind5<false>(qw[2], qs[0], qs[1], qs[2], qs[3], qs[4], qs[5]);
                     else as = zadv(qs, qw[2], ot);
                     gzs_t = rhoh1*(ds - as);
                 }
@@ -417,6 +431,11 @@ namespace mhh
                     const TF dw = TF(2)*(PL(E1,0,0) + visc)*(qw[3] - qw[2])*prof[3*PLEV + lq];
                     TF aw;
                     if (paired) aw = aws.x;
+                    else if (sizeof(TF) == 8 && ow == 6)
+                    {
+                        const TF ww = qw[2] + qw[3];
+                        aw = ww*upwind5<true>(ww, qw[0], qw[1], qw[2], qw[3], qw[4], qw[5]);
+                    }
                     else if (ow == 6) aw = adv6(i2(qw[2], qw[3]), qw[0], qw[1], qw[2], qw[3], qw[4], qw[5]);
                     else if (ow == 4) aw = i2(qw[2], qw[3])*i4ws(qw[1], qw[2], qw[3], qw[4])
                                          - fabs(i2(qw[2], qw[3]))*i3ws(qw[1], qw[2], qw[3], qw[4]);
@@ -496,6 +515,7 @@ namespace mhh
             }
 
             gzu_b = gzu_t; gzv_b = gzv_t; gzw_b = gzw_t; gzs_b = gzs_t;
+            ex0 = ex1; ey0 = ey1;
             #pragma unroll
             for (int q=0; q<5; ++q) { qu[q] = qu[q+1]; qv[q] = qv[q+1]; qw[q] = qw[q+1]; qs[q] = qs[q+1]; }
             qu[5] = nu; qv[5] = nv; qw[5] = nw; qs[5] = ns;
