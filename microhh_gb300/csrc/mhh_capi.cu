@@ -529,16 +529,23 @@ namespace
     }
 
     template<typename TF>
-    int surface_exec(mhh_ctx* c, const mhh_fields* f, const mhh_bcfields* bc, int thermo_bc, cudaStream_t s)
+    int surface_exec(mhh_ctx* c, const mhh_fields* f, const mhh_bcfields* bc, int thermo_bc, cudaStream_t s,
+                     const mhh_substep_config* ghosts = nullptr)
     {
         if (!c->surf_ready) return fail(MHH_ERR_ARG, "surface layer not initialised");
         const int thermo = (c->phys.thermo && f->s) ? 1 : 0;
         Timed t("surface", s);
+        // In the fused substep the surface kernels also fill the scalar's wall
+        // ghost levels.
+        SurfGhost<TF> g{};
+        if (ghosts && f->s)
+            g = SurfGhost<TF>{T<TF>(f->s), ghosts->sbcbot, ghosts->sbctop, CT<TF>(bc->s_bot), CT<TF>(bc->s_gradbot),
+                              CT<TF>(bc->s_top), CT<TF>(bc->s_gradtop), prof<TF>(c).dzh};
         launch_surface<TF>(c->d, prof<TF>(c), c->sw, CT<TF>(f->u), CT<TF>(f->v), CT<TF>(f->s),
                            T<TF>(bc->u_bot), T<TF>(bc->v_bot), T<TF>(bc->u_fluxbot), T<TF>(bc->v_fluxbot),
                            T<TF>(bc->u_gradbot), T<TF>(bc->v_gradbot),
                            T<TF>(bc->s_bot), T<TF>(bc->s_fluxbot), T<TF>(bc->s_gradbot),
-                           thermo, thermo_bc, c->phys.z0m, c->phys.z0h, s);
+                           thermo, thermo_bc, c->phys.z0m, c->phys.z0h, g, s);
         return check_cuda("surface");
     }
 
@@ -589,10 +596,8 @@ namespace
         const bool surf = c->phys.surface != 0;
         if (surf)
         {
-            int rc = surface_exec<TF>(c, f, bc, cfg->sbcbot, s);
+            int rc = surface_exec<TF>(c, f, bc, cfg->sbcbot, s, cfg);
             if (rc) return rc;
-            Timed t("boundaries", s);
-            ghost_all<TF>(c, cfg, f, bc, false, s);
         }
         TendArgs<TF> a = tend_args<TF>(c, f, bc);
         const bool force = cfg->swlspres != 0;
@@ -826,7 +831,6 @@ int mhh_ctx_create(const mhh_grid_desc* desc, const double* z, int precision, co
     if (!rc) rc = dalloc(&c->sw.dudz, d.ijcells);
     if (!rc) rc = dalloc(&c->sw.dvdz, d.ijcells);
     if (!rc) rc = dalloc(&c->sw.dbdz, d.ijcells);
-    if (!rc) rc = dalloc(&c->sw.dutot, d.ijcells);
     if (!rc) rc = dalloc(&c->sw.fm, d.ijcells);
     if (!rc) rc = dalloc(&c->sw.fh, d.ijcells);
     if (!rc) rc = dalloc(&c->sw.phim, d.ijcells);
@@ -896,7 +900,7 @@ int mhh_ctx_estimate_bytes(const mhh_grid_desc* g, int precision, size_t* bytes)
     b += groups*(8. + 8. + 8. + 8. + 4. + 8.); // elimination tables
     b += 1.1*groups*(precision == MHH_FP64 ? 24. : 12. + 20.);   // the same in block order
     b += 2.*(g->itot + g->jtot)*(16. + 8.);    // twiddles
-    b += 12.*ij*8. + ij*4. + 2.*10000*4.;      // surface layer
+    b += 11.*ij*8. + ij*4. + 2.*10000*4.;      // surface layer
     b += 2.*kcells*8.;                          // mixing length
     // cudaMalloc granularity: about 40 allocations of up to 2 MiB each.
     b += 40.*2.*1024*1024;
@@ -912,7 +916,7 @@ int mhh_ctx_destroy(mhh_ctx* c)
     for (auto& p : c->dprof) if (p) cudaFreeAsync(p, c->setup);
     fft_plan_free(&c->pw.px, c->setup); fft_plan_free(&c->pw.py, c->setup);
     void* ptrs[] = {c->pw.pk, c->pw.work, c->pw.dcm, c->pw.rtab, c->pw.wtab, c->pw.gtab, c->pw.htab, c->pw.stab, c->pw.stabd, c->pw.fmode, c->pw.ctab, c->pw.dtab, c->pw.list, c->pw.ltab, c->pw.lstab, c->pw.bmati, c->pw.bmatj, c->pw.a, c->pw.c, c->pw.dz2, c->pw.dz2rho,
-                    c->red, c->statbuf, c->bufprof, c->sw.fm, c->sw.fh, c->sw.phim, c->sw.phih, c->sw.ustar, c->sw.obuk, c->sw.dudz, c->sw.dvdz, c->sw.dbdz, c->sw.dutot,
+                    c->red, c->statbuf, c->bufprof, c->sw.fm, c->sw.fh, c->sw.phim, c->sw.phih, c->sw.ustar, c->sw.obuk, c->sw.dudz, c->sw.dvdz, c->sw.dbdz,
                     c->sw.nobuk, c->sw.zL, c->sw.f, c->sw.mlen2, c->sw.mlen2f};
     for (void* p : ptrs) if (p) cudaFreeAsync(p, c->setup);
     if (c->red_host) cudaFreeHost(c->red_host);

@@ -102,6 +102,20 @@ namespace mhh
         atomicMax(dst, bits);
     }
 
+    // Wall ghost levels of a field at column n, 2nd order
+    // (src/boundary.cxx:700-760): cb and ct are the column's lowest and highest
+    // interior cells.
+    template<typename TF>
+    __device__ __forceinline__ void wall_ghost(TF* a, int n, long long cb, long long ct, int kk, int bot_type,
+                                               const TF* bot, const TF* gradbot, TF dzhb, int top_type,
+                                               const TF* top, const TF* gradtop, TF dzht)
+    {
+        if (bot_type == MHH_BC_DIRICHLET) a[cb - kk] = TF(2)*bot[n] - a[cb];
+        else a[cb - kk] = -gradbot[n]*dzhb + a[cb];
+        if (top_type == MHH_BC_DIRICHLET) a[ct + kk] = TF(2)*top[n] - a[ct];
+        else a[ct + kk] = gradtop[n]*dzht + a[ct];
+    }
+
     // Exact float <-> double conversions on the integer pipe (IEEE 754
     // binary32/binary64 layouts): the FP64 pipe of this GPU is narrow and
     // its conversions would cost as much as the solve.  Zeros, subnormals,

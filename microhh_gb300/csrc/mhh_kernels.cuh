@@ -202,7 +202,7 @@ namespace mhh
     // ---- surface layer (mhh_surface.cu) ----
     struct SurfWork
     {
-        double *ustar, *obuk, *dudz, *dvdz, *dbdz, *dutot;
+        double *ustar, *obuk, *dudz, *dvdz, *dbdz;
         double *fm, *fh, *phim, *phih;   // per-cell Monin-Obukhov functions of the last stability call
         double z0h;
         int* nobuk;
@@ -214,9 +214,20 @@ namespace mhh
         double thb_s, thbh_s;      // the same in the scalar's storage units
     };
 
+    // The wall ghost levels of the scalar that the surface kernels fill after
+    // its surface values (a == NULL: none).
+    template<typename TF>
+    struct SurfGhost
+    {
+        TF* a;
+        int bot_type, top_type;
+        const TF *bot, *gradbot, *top, *gradtop, *dzh;
+    };
+
     template<typename TF> void launch_surface(const Dims& d, const Prof<TF>& pr, const SurfWork& sw,
                                               const TF* u, const TF* v, const TF* s,
                                               TF* u_bot, TF* v_bot, TF* u_flux, TF* v_flux, TF* u_grad, TF* v_grad,
                                               TF* s_bot, TF* s_flux, TF* s_grad,
-                                              int thermo, int thermo_bc, double z0m, double z0h, cudaStream_t st);
+                                              int thermo, int thermo_bc, double z0m, double z0h,
+                                              const SurfGhost<TF>& ghost, cudaStream_t st);
 }

@@ -141,17 +141,10 @@ namespace mhh
         const TF dzhb = dzh[d.kstart], dzht = dzh[d.kend];
         for (int f=0; f<gl.n; ++f)
         {
-            TF* a = gl.a[f];
             const long long cb = n + (long long)d.kstart*d.ijcells;
             const long long ct = n + (long long)(d.kend-1)*d.ijcells;
-            if (gl.bot_type[f] == MHH_BC_DIRICHLET)
-                a[cb - d.ijcells] = TF(2)*gl.abot[f][n] - a[cb];
-            else
-                a[cb - d.ijcells] = -gl.agradbot[f][n]*dzhb + a[cb];
-            if (gl.top_type[f] == MHH_BC_DIRICHLET)
-                a[ct + d.ijcells] = TF(2)*gl.atop[f][n] - a[ct];
-            else
-                a[ct + d.ijcells] = gl.agradtop[f][n]*dzht + a[ct];
+            wall_ghost(gl.a[f], n, cb, ct, d.ijcells, gl.bot_type[f], gl.abot[f], gl.agradbot[f], dzhb,
+                       gl.top_type[f], gl.atop[f], gl.agradtop[f], dzht);
         }
     }
 

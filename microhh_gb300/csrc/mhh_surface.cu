@@ -32,20 +32,61 @@ namespace mhh
     }
 
     // include/boundary_surface_kernels.h:282-298, with the search kept inside
-    // the table.
-    __device__ double find_zL(const float* zL, const float* f, int* np, float Ri)
+    // the table.  The walk from the cell's last position reads eight entries
+    // at a time, so that it waits once per eight steps (the first call walks
+    // from the bottom of the table).
+    __device__ double find_zL(const float* __restrict__ zL, const float* __restrict__ f, int* np, float Ri)
     {
+        constexpr int W = 8;
         int n = *np;
         if (__fsub_rn(f[n], Ri) > 0.f)
-            while (n > 0 && __fsub_rn(f[n-1], Ri) > 0.f) --n;
+        {
+            for (bool more = true; more && n > 0; )
+            {
+                float v[W];
+                #pragma unroll
+                for (int q=0; q<W; ++q) v[q] = f[max(n - 1 - q, 0)];
+                #pragma unroll
+                for (int q=0; q<W; ++q)
+                {
+                    more = more && n > 0 && __fsub_rn(v[q], Ri) > 0.f;
+                    if (more) --n;
+                }
+            }
+        }
         else
-            while (__fsub_rn(f[n], Ri) < 0.f && n < NZL_LUT-1) ++n;
+        {
+            for (bool more = true; more && n < NZL_LUT-1; )
+            {
+                float v[W];
+                #pragma unroll
+                for (int q=0; q<W; ++q) v[q] = f[min(n + q, NZL_LUT - 1)];
+                #pragma unroll
+                for (int q=0; q<W; ++q)
+                {
+                    more = more && __fsub_rn(v[q], Ri) < 0.f && n < NZL_LUT-1;
+                    if (more) ++n;
+                }
+            }
+        }
         *np = n;
         if (n == 0 || n == NZL_LUT-1) return (double)zL[n];
         const float num = __fsub_rn(Ri, f[n-1]);
         const float den = __fsub_rn(f[n], f[n-1]);
         const float dz = __fsub_rn(zL[n], zL[n-1]);
         return (double)__fadd_rn(zL[n-1], __fmul_rn(__fdiv_rn(num, den), dz));
+    }
+
+    // Cell n of a 2-D array with ghost cells: its interior image, and whether
+    // it is interior itself.  A ghost cell computes its image's values from the
+    // same operands, which equals the periodic copy of the reference.
+    __device__ __forceinline__ int surf_image(const Dims& d, int n, bool& inside)
+    {
+        const int j = n / d.icells, i = n - j*d.icells;
+        const int wi = i < d.istart ? i + d.itot : (i >= d.iend ? i - d.itot : i);
+        const int wj = j < d.jstart ? j + d.jtot : (j >= d.jend ? j - d.jtot : j);
+        inside = wi == i && wj == j;
+        return wi + wj*d.icells;
     }
 
     // Everything the surface-layer kernels of one context read and write.
@@ -56,22 +97,18 @@ namespace mhh
         TF *u_bot, *v_bot, *u_flux, *v_flux, *u_grad, *v_grad, *s_bot, *s_flux, *s_grad;
         double zsl, z0m, z0h, thref_s, threfh_s, thb_s, thbh_s;
         int thermo, thermo_bc;
+        SurfGhost<TF> g;
     };
 
-    // Filtered wind speed, include/boundary_surface_kernels.h:132-178
-    // (interior), in the field precision.
+    // Filtered wind speed of the interior cell ij,
+    // include/boundary_surface_kernels.h:132-178, in the field precision.
     template<typename TF>
-    __device__ __forceinline__ void dutot_body(const SurfP<TF>& P, const VBlock& vb)
+    __device__ __forceinline__ TF wind_speed(const SurfP<TF>& P, int ij)
     {
         const Dims& d = P.d;
         const TF* __restrict__ u = P.u; const TF* __restrict__ v = P.v;
         const TF* __restrict__ ubot = P.u_bot; const TF* __restrict__ vbot = P.v_bot;
-        double* __restrict__ dutot = P.sw.dutot;
-        const int i = d.istart + vb.x*blockDim.x + threadIdx.x;
-        const int j = d.jstart + vb.y*blockDim.y + threadIdx.y;
-        if (i >= d.iend || j >= d.jend) return;
         const long long ii = 1, jj = d.icells;
-        const long long ij = i + j*jj;
         const long long c = ij + (long long)d.kstart*d.ijcells;
         using CT = TF;
         auto U = [&](long long q) { return CT(u[q]); };
@@ -87,7 +124,7 @@ namespace mhh
             + h*V(c+ii-jj) + V(c+ii) + V(c+ii+jj) + h*V(c+ii+2*jj));
         const CT du2 = sq(uf - h*(CT(ubot[ij]) + CT(ubot[ij+ii])))
                      + sq(vf - h*(CT(vbot[ij]) + CT(vbot[ij+jj])));
-        dutot[ij] = to_d<CT>(fmax(pow(du2, CT(0.5)), CT(1.e-1)));
+        return fmax(pow(du2, CT(0.5)), CT(1.e-1));
     }
 
     // The Monin-Obukhov functions of one cell, each evaluated once: the
@@ -122,10 +159,21 @@ namespace mhh
         return r;
     }
 
-    // Obukhov length and friction velocity, src/boundary_surface.cxx:55-160
-    // (all cells; the neutral branch when there is no thermodynamics).
+    // The surface layer runs as two kernels over all cells of the 2-D arrays,
+    // ghost cells included: the Obukhov state of every cell, then everything
+    // that needs its neighbours'.  One kernel per module of the reference and
+    // per periodic copy made nine launches, bound by launch and latency: per RK3
+    // step with the scalar's ghost levels 0.125 ms at 32^3 and 0.19 at 512 x
+    // 512, now 0.049 and 0.11; in double 0.36 at 64^3, now 0.15.
+    constexpr int SURF_NT = 64;
+
+    // Wind speed, Obukhov length and friction velocity,
+    // src/boundary_surface.cxx:55-160 (the neutral branch when there is no
+    // thermodynamics).  Blocks of two warps: a double evaluation of the
+    // similarity functions is some 300 operations on the narrow FP64 pipe, so
+    // small grids spread over all SMs.
     template<typename TF>
-    __device__ __forceinline__ void stability_body(const SurfP<TF>& P, const VBlock& vb)
+    __device__ __forceinline__ void surf_state_body(const SurfP<TF>& P, const VBlock& vb)
     {
         const Dims& d = P.d;
         const SurfWork& sw = P.sw;
@@ -136,7 +184,8 @@ namespace mhh
         const int n = vb.x*blockDim.x + threadIdx.x;
         if (n >= d.ijcells) return;
         using CT = TF;
-        const CT du = from_d<CT>(sw.dutot[n]);
+        bool inside;
+        const CT du = wind_speed(P, surf_image(d, n, inside));
         const CT zs = CT(zsl);
         CT L;
         if (!thermo)
@@ -164,99 +213,80 @@ namespace mhh
         sw.phim[n] = to_d<CT>(mc.phim); sw.phih[n] = to_d<CT>(mc.phih);
     }
 
-    // Momentum fluxes, src/boundary_surface.cxx:163-190 (interior).
+    // Momentum fluxes (src/boundary_surface.cxx:163-190), surface gradients of
+    // u and v and the scalar's surface value, gradient or flux (:255-338), the
+    // Monin-Obukhov gradients for the next viscosity (interior cells,
+    // include/boundary_surface_kernels.h:180-238) and, where the caller asks,
+    // the scalar's wall ghost levels.
     template<typename TF>
-    __device__ __forceinline__ void surfm_body(const SurfP<TF>& P, const VBlock& vb)
+    __device__ __forceinline__ void surf_flux_body(const SurfP<TF>& P, const VBlock& vb)
     {
         const Dims& d = P.d;
         const SurfWork& sw = P.sw;
-        const TF* __restrict__ u = P.u; const TF* __restrict__ v = P.v;
+        const TF* __restrict__ u = P.u; const TF* __restrict__ v = P.v; const TF* s = P.s;
         const TF* __restrict__ ubot = P.u_bot; const TF* __restrict__ vbot = P.v_bot;
-        TF* __restrict__ uflux = P.u_flux; TF* __restrict__ vflux = P.v_flux;
-        const int i = d.istart + vb.x*blockDim.x + threadIdx.x;
-        const int j = d.jstart + vb.y*blockDim.y + threadIdx.y;
-        if (i >= d.iend || j >= d.jend) return;
-        const long long ii = 1, jj = d.icells;
-        const long long ij = i + j*jj;
-        const long long c = ij + (long long)d.kstart*d.ijcells;
-        using CT = TF;
-        auto D = [&](const double* a, long long q) { return from_d<CT>(a[q]); };
-        const CT fc = D(sw.ustar, ij)*D(sw.fm, ij);
-        uflux[ij] = -(CT(u[c]) - CT(ubot[ij]))*CT(0.5)*(D(sw.ustar, ij-ii)*D(sw.fm, ij-ii) + fc);
-        vflux[ij] = -(CT(v[c]) - CT(vbot[ij]))*CT(0.5)*(D(sw.ustar, ij-jj)*D(sw.fm, ij-jj) + fc);
-    }
-
-    // Surface gradients of u and v and the scalar surface value, gradient or
-    // flux, src/boundary_surface.cxx:255-338 (all cells).
-    template<typename TF>
-    __device__ __forceinline__ void surf_grads_body(const SurfP<TF>& P, const VBlock& vb)
-    {
-        const Dims& d = P.d;
-        const SurfWork& sw = P.sw;
-        const TF* __restrict__ u = P.u; const TF* __restrict__ v = P.v;
-        const TF* __restrict__ ubot = P.u_bot; const TF* __restrict__ vbot = P.v_bot;
-        TF* __restrict__ ugrad = P.u_grad; TF* __restrict__ vgrad = P.v_grad;
-        const TF* __restrict__ s = P.s; TF* __restrict__ sbot = P.s_bot; TF* __restrict__ sgrad = P.s_grad;
-        TF* __restrict__ sflux = P.s_flux;
-        const double zsl = P.zsl;
+        const double zsl = P.zsl, threfh_s = P.threfh_s;
         const int thermo = P.thermo, thermo_bc = P.thermo_bc;
         const int n = vb.x*blockDim.x + threadIdx.x;
         if (n >= d.ijcells) return;
-        const long long c = n + (long long)d.kstart*d.ijcells;
+        bool inside;
+        const int ij = surf_image(d, n, inside);
+        const int ii = 1, jj = d.icells;
+        const long long k0 = (long long)d.kstart*d.ijcells;
         using CT = TF;
+        auto D = [&](const double* a, int q) { return from_d<CT>(a[q]); };
+        {
+            const CT fc = D(sw.ustar, ij)*D(sw.fm, ij);
+            P.u_flux[n] = -(CT(u[k0 + ij]) - CT(ubot[ij]))*CT(0.5)*(D(sw.ustar, ij-ii)*D(sw.fm, ij-ii) + fc);
+            P.v_flux[n] = -(CT(v[k0 + ij]) - CT(vbot[ij]))*CT(0.5)*(D(sw.ustar, ij-jj)*D(sw.fm, ij-jj) + fc);
+        }
         const CT z = CT(zsl);
-        ugrad[n] = (CT(u[c]) - CT(ubot[n]))/z;
-        vgrad[n] = (CT(v[c]) - CT(vbot[n]))/z;
+        P.u_grad[n] = (CT(u[k0 + n]) - CT(ubot[n]))/z;
+        P.v_grad[n] = (CT(v[k0 + n]) - CT(vbot[n]))/z;
+        CT flux = CT(0);
         if (thermo)
         {
-            const CT th = CT(s[c]);
+            const CT th = CT(s[k0 + n]);
             const CT us = from_d<CT>(sw.ustar[n]), fh = from_d<CT>(sw.fh[n]);
+            flux = CT(P.s_flux[n]);
             if (thermo_bc == MHH_BC_DIRICHLET)
             {
-                sflux[n] = -(th - CT(sbot[n]))*us*fh;
-                sgrad[n] = (th - CT(sbot[n]))/z;
+                flux = -(th - CT(P.s_bot[n]))*us*fh;
+                P.s_flux[n] = flux;
+                P.s_grad[n] = (th - CT(P.s_bot[n]))/z;
             }
             else
             {
-                const CT bot = CT(sflux[n])/(us*fh) + th;
-                sbot[n] = bot;
-                sgrad[n] = (th - bot)/z;
+                const CT bot = flux/(us*fh) + th;
+                P.s_bot[n] = bot;
+                P.s_grad[n] = (th - bot)/z;
             }
         }
-    }
-
-    // Monin-Obukhov gradients for the next viscosity, include/boundary_surface_kernels.h:180-238.
-    template<typename TF>
-    __device__ __forceinline__ void duvdz_body(const SurfP<TF>& P, const VBlock& vb)
-    {
-        const Dims& d = P.d;
-        const SurfWork& sw = P.sw;
-        const TF* __restrict__ u = P.u; const TF* __restrict__ v = P.v;
-        const TF* __restrict__ ubot = P.u_bot; const TF* __restrict__ vbot = P.v_bot;
-        const TF* __restrict__ sflux = P.s_flux;
-        const double zsl = P.zsl, threfh_s = P.threfh_s;
-        const int thermo = P.thermo;
-        const int i = d.istart + vb.x*blockDim.x + threadIdx.x;
-        const int j = d.jstart + vb.y*blockDim.y + threadIdx.y;
-        if (i >= d.iend || j >= d.jend) return;
-        const long long ii = 1, jj = d.icells;
-        const long long ij = i + j*jj;
-        const long long c = ij + (long long)d.kstart*d.ijcells;
-        using CT = TF;
-        const CT du_c = CT(0.5)*((CT(u[c]) - CT(ubot[ij])) + (CT(u[c+ii]) - CT(ubot[ij+ii])));
-        const CT dv_c = CT(0.5)*((CT(v[c]) - CT(vbot[ij])) + (CT(v[c+jj]) - CT(vbot[ij+jj])));
-        const CT us = from_d<CT>(sw.ustar[ij]);
-        const CT fmv = from_d<CT>(sw.fm[ij]);
-        const CT ufb = -du_c*us*fmv;
-        const CT vfb = -dv_c*us*fmv;
-        const CT ph = from_d<CT>(sw.phim[ij]);
-        const CT kz = CT(KAPPA)*CT(zsl);
-        sw.dudz[ij] = to_d<CT>(-ufb/(kz*us)*ph);
-        sw.dvdz[ij] = to_d<CT>(-vfb/(kz*us)*ph);
-        if (thermo)
+        if (inside)
         {
-            const CT bfb = CT(GRAV)/CT(threfh_s)*CT(sflux[ij]);
-            sw.dbdz[ij] = to_d<CT>(-bfb/(kz*us)*from_d<CT>(sw.phih[ij]));
+            const long long c = k0 + n;
+            const CT du_c = CT(0.5)*((CT(u[c]) - CT(ubot[n])) + (CT(u[c+ii]) - CT(ubot[n+ii])));
+            const CT dv_c = CT(0.5)*((CT(v[c]) - CT(vbot[n])) + (CT(v[c+jj]) - CT(vbot[n+jj])));
+            const CT us = from_d<CT>(sw.ustar[n]);
+            const CT fmv = from_d<CT>(sw.fm[n]);
+            const CT ufb = -du_c*us*fmv;
+            const CT vfb = -dv_c*us*fmv;
+            const CT ph = from_d<CT>(sw.phim[n]);
+            const CT kz = CT(KAPPA)*CT(zsl);
+            sw.dudz[n] = to_d<CT>(-ufb/(kz*us)*ph);
+            sw.dvdz[n] = to_d<CT>(-vfb/(kz*us)*ph);
+            if (thermo)
+            {
+                const CT bfb = CT(GRAV)/CT(threfh_s)*flux;
+                sw.dbdz[n] = to_d<CT>(-bfb/(kz*us)*from_d<CT>(sw.phih[n]));
+            }
+        }
+        if (P.g.a)
+        {
+            const SurfGhost<TF>& g = P.g;
+            const long long cb = k0 + n, ct = n + (long long)(d.kend-1)*d.ijcells;
+            wall_ghost(g.a, n, cb, ct, d.ijcells, g.bot_type, g.bot, g.gradbot, g.dzh[d.kstart],
+                       g.top_type, g.top, g.gradtop, g.dzh[d.kend]);
         }
     }
 
@@ -265,28 +295,21 @@ namespace mhh
                         const TF* u, const TF* v, const TF* s,
                         TF* u_bot, TF* v_bot, TF* u_flux, TF* v_flux, TF* u_grad, TF* v_grad,
                         TF* s_bot, TF* s_flux, TF* s_grad,
-                        int thermo, int thermo_bc, double z0m, double z0h, cudaStream_t st)
+                        int thermo, int thermo_bc, double z0m, double z0h, const SurfGhost<TF>& ghost, cudaStream_t st)
     {
         const double zsl = sw.zsl, thref_s = sw.thref_s, threfh_s = sw.threfh_s;
-        dim3 b2(32, 8), g2((d.itot + 31)/32, (d.jtot + 7)/8);
-        const int nb = (d.ijcells + 255)/256;
+        const dim3 nb((d.ijcells + SURF_NT - 1)/SURF_NT);
         const SurfP<TF> P{d, sw, u, v, s, u_bot, v_bot, u_flux, v_flux, u_grad, v_grad, s_bot, s_flux, s_grad,
-                          zsl, z0m, z0h, thref_s, threfh_s, sw.thb_s, sw.thbh_s, thermo, thermo_bc};
-        launch_body<SurfP<TF>, dutot_body<TF>, 256>(g2, b2, 0, st, P);
-        launch_cyclic2d<double>(sw.dutot, d, st);
-        launch_body<SurfP<TF>, stability_body<TF>, 256>(dim3(nb), dim3(256), 0, st, P);
-        launch_body<SurfP<TF>, surfm_body<TF>, 256>(g2, b2, 0, st, P);
-        launch_cyclic2d<TF>(u_flux, d, st);
-        launch_cyclic2d<TF>(v_flux, d, st);
-        launch_body<SurfP<TF>, surf_grads_body<TF>, 256>(dim3(nb), dim3(256), 0, st, P);
-        launch_body<SurfP<TF>, duvdz_body<TF>, 256>(g2, b2, 0, st, P);
-        count_launch(5);
+                          zsl, z0m, z0h, thref_s, threfh_s, sw.thb_s, sw.thbh_s, thermo, thermo_bc, ghost};
+        launch_body<SurfP<TF>, surf_state_body<TF>, SURF_NT>(nb, dim3(SURF_NT), 0, st, P);
+        launch_body<SurfP<TF>, surf_flux_body<TF>, SURF_NT>(nb, dim3(SURF_NT), 0, st, P);
+        count_launch(2);
     }
 
     template void launch_surface<double>(const Dims&, const Prof<double>&, const SurfWork&, const double*, const double*,
         const double*, double*, double*, double*, double*, double*, double*, double*, double*, double*,
-        int, int, double, double, cudaStream_t);
+        int, int, double, double, const SurfGhost<double>&, cudaStream_t);
     template void launch_surface<float>(const Dims&, const Prof<float>&, const SurfWork&, const float*, const float*,
         const float*, float*, float*, float*, float*, float*, float*, float*, float*, float*,
-        int, int, double, double, cudaStream_t);
+        int, int, double, double, const SurfGhost<float>&, cudaStream_t);
 }
