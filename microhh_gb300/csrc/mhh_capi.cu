@@ -460,11 +460,7 @@ namespace
             // The right-hand side is computed inside the forward x transform
             // and the inverse x transform stores into the ghost layout of p:
             // two field passes fewer each way.
-            {
-                Timed t("pres_in", s);
-                fl.n = 1; fl.p[0] = T<TF>(f->ut); launch_cyclic(fl, d, MHH_EDGE_EW, s);
-                fl.p[0] = T<TF>(f->vt); launch_cyclic(fl, d, MHH_EDGE_NS, s);
-            }
+            { Timed t("pres_in", s); launch_cyclic_tend(T<TF>(f->ut), T<TF>(f->vt), d, s); }
             FftFuse<TF> fz;
             std::memset(&fz, 0, sizeof(fz));
             fz.d = d; fz.pr = pr;
@@ -480,17 +476,12 @@ namespace
             { Timed t("fft_y", s); launch_fft_y<TF>(c->pw.py, pk, d.itot, d.jtot, d.ktot, true, 1./d.jtot, s); }
             fz.mode = 2;
             { Timed t("fft_x", s); launch_fft_x<TF>(c->pw.px, pk, d.jtot*d.ktot, true, 1./d.itot, s, &fz); }
-            {
-                Timed t("pres_scatter", s);
-                fl.p[0] = T<TF>(f->p); launch_cyclic(fl, d, MHH_EDGE_BOTH, s);
-            }
         }
         else
         {
         {
             Timed t("pres_in", s);
-            fl.n = 1; fl.p[0] = T<TF>(f->ut); launch_cyclic(fl, d, MHH_EDGE_EW, s);
-            fl.p[0] = T<TF>(f->vt); launch_cyclic(fl, d, MHH_EDGE_NS, s);
+            launch_cyclic_tend(T<TF>(f->ut), T<TF>(f->vt), d, s);
             launch_pres_in<TF>(d, pr, CT<TF>(f->u), CT<TF>(f->v), CT<TF>(f->w), CT<TF>(f->ut), CT<TF>(f->vt), CT<TF>(f->wt),
                                pk, 1./sub_dt, s);
         }
@@ -502,8 +493,11 @@ namespace
         {
             Timed t("pres_scatter", s);
             launch_pres_scatter<TF>(d, pk, static_cast<const TF*>(c->pw.dcm), T<TF>(f->p), s);
-            fl.p[0] = T<TF>(f->p); launch_cyclic(fl, d, MHH_EDGE_BOTH, s);
         }
+        }
+        {
+            Timed t("pres_scatter", s);
+            fl.n = 1; fl.p[0] = T<TF>(f->p); launch_cyclic(fl, d, MHH_EDGE_BOTH, s);
         }
         if (with_out)
         {
@@ -550,37 +544,25 @@ namespace
     }
 
     template<typename TF>
-    void ghost_all(mhh_ctx* c, const mhh_substep_config* cfg, const mhh_fields* f, const mhh_bcfields* bc,
-                   bool momentum, cudaStream_t s)
-    {
-        GhostList<TF> gl{};
-        auto add = [&](void* a, int bt, void* abot, void* agb, int tt, void* atop, void* agt)
-        {
-            const int q = gl.n++;
-            gl.a[q] = T<TF>(a); gl.bot_type[q] = bt; gl.top_type[q] = tt;
-            gl.abot[q] = CT<TF>(abot); gl.agradbot[q] = CT<TF>(agb);
-            gl.atop[q] = CT<TF>(atop); gl.agradtop[q] = CT<TF>(agt);
-        };
-        if (momentum)
-        {
-            add(f->u, cfg->mbcbot, bc->u_bot, bc->u_gradbot, cfg->mbctop, bc->u_top, bc->u_gradtop);
-            add(f->v, cfg->mbcbot, bc->v_bot, bc->v_gradbot, cfg->mbctop, bc->v_top, bc->v_gradtop);
-        }
-        if (f->s)
-            add(f->s, cfg->sbcbot, bc->s_bot, bc->s_gradbot, cfg->sbctop, bc->s_top, bc->s_gradtop);
-        if (gl.n) launch_ghost<TF>(gl, c->d, prof<TF>(c).dzh, s);
-    }
-
-    template<typename TF>
     int substep_begin(mhh_ctx* c, const mhh_substep_config* cfg, const mhh_fields* f, const mhh_bcfields* bc, cudaStream_t s)
     {
         {
             Timed t("boundaries", s);
             FieldList<TF> fl{};
-            fl.p[fl.n++] = T<TF>(f->u); fl.p[fl.n++] = T<TF>(f->v); fl.p[fl.n++] = T<TF>(f->w);
-            if (f->s) fl.p[fl.n++] = T<TF>(f->s);
-            launch_cyclic(fl, c->d, MHH_EDGE_BOTH, s);
-            ghost_all<TF>(c, cfg, f, bc, true, s);
+            GhostList<TF> gl{};
+            auto add = [&](void* a, int bt, void* abot, void* agb, int tt, void* atop, void* agt)
+            {
+                const int q = gl.n++;
+                fl.p[fl.n++] = T<TF>(a);
+                gl.a[q] = T<TF>(a); gl.bot_type[q] = bt; gl.top_type[q] = tt;
+                gl.abot[q] = CT<TF>(abot); gl.agradbot[q] = CT<TF>(agb);
+                gl.atop[q] = CT<TF>(atop); gl.agradtop[q] = CT<TF>(agt);
+            };
+            add(f->u, cfg->mbcbot, bc->u_bot, bc->u_gradbot, cfg->mbctop, bc->u_top, bc->u_gradtop);
+            add(f->v, cfg->mbcbot, bc->v_bot, bc->v_gradbot, cfg->mbctop, bc->v_top, bc->v_gradtop);
+            if (f->s) add(f->s, cfg->sbcbot, bc->s_bot, bc->s_gradbot, cfg->sbctop, bc->s_top, bc->s_gradtop);
+            fl.p[fl.n++] = T<TF>(f->w);
+            launch_ghosts<TF>(fl, gl, c->d, prof<TF>(c).dzh, s);
         }
         if (cfg->diff == MHH_DIFF_SMAG2)
             return viscosity<TF>(c, f, s);

@@ -108,12 +108,25 @@ namespace mhh
     template<typename TF>
     __device__ __forceinline__ void wall_ghost(TF* a, int n, long long cb, long long ct, int kk, int bot_type,
                                                const TF* bot, const TF* gradbot, TF dzhb, int top_type,
-                                               const TF* top, const TF* gradtop, TF dzht)
+                                               const TF* top, const TF* gradtop, TF dzht, int image = 0)
     {
-        if (bot_type == MHH_BC_DIRICHLET) a[cb - kk] = TF(2)*bot[n] - a[cb];
-        else a[cb - kk] = -gradbot[n]*dzhb + a[cb];
-        if (top_type == MHH_BC_DIRICHLET) a[ct + kk] = TF(2)*top[n] - a[ct];
-        else a[ct + kk] = gradtop[n]*dzht + a[ct];
+        // image: offset of the interior cell that a ghost column mirrors.
+        const TF ab = a[cb + image], at = a[ct + image];
+        if (bot_type == MHH_BC_DIRICHLET) a[cb - kk] = TF(2)*bot[n] - ab;
+        else a[cb - kk] = -gradbot[n]*dzhb + ab;
+        if (top_type == MHH_BC_DIRICHLET) a[ct + kk] = TF(2)*top[n] - at;
+        else a[ct + kk] = gradtop[n]*dzht + at;
+    }
+
+    // Interior image of cell n of a 2-D plane with ghost cells, and whether the
+    // cell is interior itself.
+    __device__ __forceinline__ int plane_image(const Dims& d, int n, bool& inside)
+    {
+        const int j = n / d.icells, i = n - j*d.icells;
+        const int wi = i < d.istart ? i + d.itot : (i >= d.iend ? i - d.itot : i);
+        const int wj = j < d.jstart ? j + d.jtot : (j >= d.jend ? j - d.jtot : j);
+        inside = wi == i && wj == j;
+        return wi + wj*d.icells;
     }
 
     // Exact float <-> double conversions on the integer pipe (IEEE 754

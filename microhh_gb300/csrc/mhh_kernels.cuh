@@ -73,6 +73,13 @@ namespace mhh
     template<typename TF> void launch_set_bc(TF* val, TF* grad, TF* flux, int type, double aval, double visc,
                                              int sfg, const Dims& d, cudaStream_t s);
     template<typename TF> void launch_ghost(const GhostList<TF>& gl, const Dims& d, const TF* dzh, cudaStream_t s);
+    // The ghost columns of ut and the ghost rows of vt, the periodic fill the
+    // pressure right-hand side needs, in one launch.
+    template<typename TF> void launch_cyclic_tend(TF* ut, TF* vt, const Dims& d, cudaStream_t s);
+    // Periodic ghost cells of the fields fl and wall ghost levels gl (the first
+    // gl.n fields of fl) in one launch.
+    template<typename TF> void launch_ghosts(const FieldList<TF>& fl, const GhostList<TF>& gl, const Dims& d, const TF* dzh,
+                                             cudaStream_t s);
     template<typename TF> void launch_viscosity(const Dims& d, const Prof<TF>& pr, const TF* u, const TF* v, const TF* w,
                                                 const TF* th, TF* evisc, const TF* mlen2, const double* dudz,
                                                 const double* dvdz, const double* dbdz, double cs, double tpr,
@@ -177,8 +184,8 @@ namespace mhh
     template<typename TF> void launch_pres_in(const Dims& d, const Prof<TF>& pr, const TF* u, const TF* v, const TF* w,
                                               const TF* ut, const TF* vt, const TF* wt, TF* pk, double dti, cudaStream_t s);
     // Work fused into the row (x) FFT: mode 1 computes the pressure
-    // right-hand side in place of loading the forward transform's input;
-    // mode 2 stores the inverse transform's output into the ghost layout of p.
+    // right-hand side in place of loading the forward transform's input; mode 2 stores the
+    // inverse transform's output into the ghost layout of p.
     // With mode 2, dcm (if set) holds each level's mean, which the tridiagonal
     // solve took out of the mean mode; it is added to every stored point.
     template<typename TF>

@@ -16,14 +16,16 @@ namespace mhh
     // equals the reference's east-west-then-north-south copy, corners
     // included, and reads interior cells only.
     // ---------------------------------------------------------------------
-    template<typename TF> struct CyclicP { FieldList<TF> fl; Dims d; int edges; };
+    // edges2: two fields, the second in the grid's second z slice with its own
+    // edges.
+    template<typename TF> struct CyclicP { FieldList<TF> fl; Dims d; int edges, edges2; };
 
     template<typename TF>
     __device__ __forceinline__ void cyclic_body(const CyclicP<TF>& P, const VBlock& vb)
     {
-        const FieldList<TF>& fl = P.fl;
         const Dims& d = P.d;
-        const int edges = P.edges;
+        const int edges = vb.z ? P.edges2 : P.edges;
+        const int f0 = vb.z, f1 = P.edges2 ? f0 + 1 : P.fl.n;
         const int nghost_i = 2*d.igc, nghost_j = 2*d.jgc;
         // Work items: the ghost columns (all j) and the ghost rows: interior i
         // when the columns are filled too, every i for a north-south-only fill
@@ -63,8 +65,8 @@ namespace mhh
                 else if (j >= d.jend) sj = j - d.jtot;
             }
             const long long dst = ijk(d, i, j, k), src = ijk(d, si, sj, k);
-            for (int f=0; f<fl.n; ++f)
-                fl.p[f][dst] = fl.p[f][src];
+            for (int f=f0; f<f1; ++f)
+                P.fl.p[f][dst] = P.fl.p[f][src];
         }
     }
 
@@ -76,7 +78,18 @@ namespace mhh
         int bx = (int)((nitem + threads - 1) / threads);
         if (bx > 64) bx = 64;
         dim3 grid(bx, d.kcells);
-        launch_body<CyclicP<TF>, cyclic_body<TF>, 128>(grid, dim3(threads), 0, s, CyclicP<TF>{fl, d, edges});
+        launch_body<CyclicP<TF>, cyclic_body<TF>, 128>(grid, dim3(threads), 0, s, CyclicP<TF>{fl, d, edges, 0});
+        count_launch();
+    }
+
+    template<typename TF>
+    void launch_cyclic_tend(TF* ut, TF* vt, const Dims& d, cudaStream_t s)
+    {
+        FieldList<TF> fl{};
+        fl.n = 2; fl.p[0] = ut; fl.p[1] = vt;
+        const int nitem = max(2*d.igc*d.jcells, 2*d.jgc*d.icells);
+        launch_body<CyclicP<TF>, cyclic_body<TF>, 128>(dim3(min((nitem + 127)/128, 64), d.kcells, 2), dim3(128), 0, s,
+                                                       CyclicP<TF>{fl, d, MHH_EDGE_EW, MHH_EDGE_NS});
         count_launch();
     }
 
@@ -152,6 +165,74 @@ namespace mhh
     void launch_ghost(const GhostList<TF>& gl, const Dims& d, const TF* dzh, cudaStream_t s)
     {
         launch_body<GhostP<TF>, ghost_body<TF>, 256>(dim3((d.ijcells + 255)/256), dim3(256), 0, s, GhostP<TF>{gl, d, dzh});
+        count_launch();
+    }
+
+    // The ghost cells of the prognostic fields at the start of a substep in one
+    // launch: the periodic fill of all levels but the wall ghost levels of the
+    // fields with walls, and those levels from the interior images of their
+    // columns (block rows from kcells on).  Periodic and wall fill as two
+    // launches took 0.039 ms per step at 32^3, this 0.024.  (Filling evisc and p
+    // inside the kernels that write them saved their launches too but slowed
+    // those kernels by more on all but the smallest grids: viscosity at 512 x
+    // 512 x 256 1.82 -> 1.93-2.13 ms per step, inverse x transform +0.1, gradient
+    // and RK3 update 2.34 -> 2.7.)
+    template<typename TF> struct GhostsP { FieldList<TF> fl; GhostList<TF> gl; Dims d; const TF* dzh; };
+
+    template<typename TF>
+    __device__ __forceinline__ void ghosts_body(const GhostsP<TF>& P, const VBlock& vb)
+    {
+        const Dims& d = P.d;
+        if (vb.y >= d.kcells)
+        {
+            const GhostList<TF>& gl = P.gl;
+            const int n = ((vb.y - d.kcells)*vb.gx + vb.x)*blockDim.x + threadIdx.x;
+            if (n >= d.ijcells) return;
+            bool inside;
+            const int image = plane_image(d, n, inside) - n;
+            const TF dzhb = P.dzh[d.kstart], dzht = P.dzh[d.kend];
+            const long long cb = n + (long long)d.kstart*d.ijcells;
+            const long long ct = n + (long long)(d.kend-1)*d.ijcells;
+            for (int f=0; f<gl.n; ++f)
+                wall_ghost(gl.a[f], n, cb, ct, d.ijcells, gl.bot_type[f], gl.abot[f], gl.agradbot[f], dzhb,
+                           gl.top_type[f], gl.atop[f], gl.agradtop[f], dzht, image);
+            return;
+        }
+        // Fields with walls come first in fl (gl.n of them).
+        const int k = vb.y;
+        const int f0 = k == d.kstart-1 || k == d.kend ? P.gl.n : 0;
+        const int nghost_i = 2*d.igc;
+        const int ncol = nghost_i*d.jcells, nitem = ncol + 2*d.jgc*d.itot;
+        for (int m = vb.x*blockDim.x + threadIdx.x; m < nitem; m += vb.gx*blockDim.x)
+        {
+            int i, j;
+            if (m < ncol)
+            {
+                j = m / nghost_i;
+                const int g = m - j*nghost_i;
+                i = g < d.igc ? g : d.iend + (g - d.igc);
+            }
+            else
+            {
+                const int g = (m - ncol) / d.itot;
+                i = d.istart + (m - ncol) - g*d.itot;
+                j = g < d.jgc ? g : d.jend + (g - d.jgc);
+            }
+            bool inside;
+            const int n = i + j*d.icells, src = plane_image(d, n, inside);
+            const long long l = (long long)k*d.ijcells;
+            for (int f=f0; f<P.fl.n; ++f) P.fl.p[f][l + n] = P.fl.p[f][l + src];
+        }
+    }
+
+    template<typename TF>
+    void launch_ghosts(const FieldList<TF>& fl, const GhostList<TF>& gl, const Dims& d, const TF* dzh, cudaStream_t s)
+    {
+        constexpr int NT = 128;
+        const int nitem = 2*d.igc*d.jcells + 2*d.jgc*d.itot;
+        const int bx = min((nitem + NT - 1)/NT, 64);
+        const int wall = gl.n ? ((d.ijcells + NT - 1)/NT + bx - 1)/bx : 0;
+        launch_body<GhostsP<TF>, ghosts_body<TF>, NT>(dim3(bx, d.kcells + wall), dim3(NT), 0, s, GhostsP<TF>{fl, gl, d, dzh});
         count_launch();
     }
 
@@ -789,6 +870,8 @@ namespace mhh
     template void launch_cyclic2d<TF>(TF*, const Dims&, cudaStream_t); \
     template void launch_set_bc<TF>(TF*, TF*, TF*, int, double, double, int, const Dims&, cudaStream_t); \
     template void launch_ghost<TF>(const GhostList<TF>&, const Dims&, const TF*, cudaStream_t); \
+    template void launch_cyclic_tend<TF>(TF*, TF*, const Dims&, cudaStream_t); \
+    template void launch_ghosts<TF>(const FieldList<TF>&, const GhostList<TF>&, const Dims&, const TF*, cudaStream_t); \
     template void launch_viscosity<TF>(const Dims&, const Prof<TF>&, const TF*, const TF*, const TF*, const TF*, TF*, \
         const TF*, const double*, const double*, const double*, double, double, double, int, bool, bool, const KernelOpts&, cudaStream_t); \
     template void launch_tendency<TF>(const Dims&, const Prof<TF>&, const TendArgs<TF>&, int, int, bool, bool, bool, bool, const KernelOpts&, cudaStream_t); \

@@ -77,18 +77,6 @@ namespace mhh
         return (double)__fadd_rn(zL[n-1], __fmul_rn(__fdiv_rn(num, den), dz));
     }
 
-    // Cell n of a 2-D array with ghost cells: its interior image, and whether
-    // it is interior itself.  A ghost cell computes its image's values from the
-    // same operands, which equals the periodic copy of the reference.
-    __device__ __forceinline__ int surf_image(const Dims& d, int n, bool& inside)
-    {
-        const int j = n / d.icells, i = n - j*d.icells;
-        const int wi = i < d.istart ? i + d.itot : (i >= d.iend ? i - d.itot : i);
-        const int wj = j < d.jstart ? j + d.jtot : (j >= d.jend ? j - d.jtot : j);
-        inside = wi == i && wj == j;
-        return wi + wj*d.icells;
-    }
-
     // Everything the surface-layer kernels of one context read and write.
     template<typename TF> struct SurfP
     {
@@ -161,7 +149,8 @@ namespace mhh
 
     // The surface layer runs as two kernels over all cells of the 2-D arrays,
     // ghost cells included: the Obukhov state of every cell, then everything
-    // that needs its neighbours'.  One kernel per module of the reference and
+    // that needs its neighbours'; a ghost cell computes its image's values from
+    // the same operands, which equals the periodic copy of the reference.  One kernel per module of the reference and
     // per periodic copy made nine launches, bound by launch and latency: per RK3
     // step with the scalar's ghost levels 0.125 ms at 32^3 and 0.19 at 512 x
     // 512, now 0.049 and 0.11; in double 0.36 at 64^3, now 0.15.
@@ -185,7 +174,7 @@ namespace mhh
         if (n >= d.ijcells) return;
         using CT = TF;
         bool inside;
-        const CT du = wind_speed(P, surf_image(d, n, inside));
+        const CT du = wind_speed(P, plane_image(d, n, inside));
         const CT zs = CT(zsl);
         CT L;
         if (!thermo)
@@ -230,7 +219,7 @@ namespace mhh
         const int n = vb.x*blockDim.x + threadIdx.x;
         if (n >= d.ijcells) return;
         bool inside;
-        const int ij = surf_image(d, n, inside);
+        const int ij = plane_image(d, n, inside);
         const int ii = 1, jj = d.icells;
         const long long k0 = (long long)d.kstart*d.ijcells;
         using CT = TF;
