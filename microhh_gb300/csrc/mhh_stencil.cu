@@ -794,6 +794,10 @@ namespace mhh
     // reference, and their maximum is taken in that precision before the one
     // conversion per block: a maximum commutes with the exact float-to-double
     // conversion, so the result is the same as a maximum over doubles.
+    // A block covers a 32 x 8 tile of columns and RED_K levels, so that one
+    // atomic stands for 2048 cells.
+    constexpr int RED_K = 8;
+
     template<typename TF, int WHAT>
     __global__ void __launch_bounds__(256)
     k_reduce(Dims d, Prof<TF> pr, const TF* __restrict__ u, const TF* __restrict__ v, const TF* __restrict__ w,
@@ -802,39 +806,46 @@ namespace mhh
         using RT = typename std::conditional<(WHAT <= 1), TF, double>::type;
         const int i = d.istart + blockIdx.x*blockDim.x + threadIdx.x;
         const int j = d.jstart + blockIdx.y*blockDim.y + threadIdx.y;
-        const int k = d.kstart + blockIdx.z;
-        RT val = 0;
+        const int k0 = d.kstart + blockIdx.z*RED_K, k1 = min(k0 + RED_K, d.kend);
+        RT best = 0;
         if (i < d.iend && j < d.jend)
         {
             const long long ii = 1, jj = d.icells, kk = d.ijcells;
-            const long long c = ijk(d, i, j, k);
-            if constexpr (WHAT == 0)
+            #pragma unroll 2
+            for (int k=k0; k<k1; ++k)
             {
-                // CFL 2i5: w interpolated with 2nd/4th/6th order by level.
-                const int ord = face_order_w(d, k);
-                TF wc;
-                if (ord == 2) wc = f2(w, c+kk, kk);
-                else if (ord == 4) wc = f4(w, c+kk, kk);
-                else wc = f6(w, c+kk, kk);
-                val = fabs(f6(u, c+ii, ii))*dxi_of<TF>(d) + fabs(f6(v, c+jj, jj))*dyi_of<TF>(d) + fabs(wc)*ld(pr.dzi, k);
-            }
-            else if constexpr (WHAT == 1)
-            {
-                val = fabs(i2(ld(u, c), ld(u, c+ii)))*dxi_of<TF>(d) + fabs(i2(ld(v, c), ld(v, c+jj)))*dyi_of<TF>(d)
-                    + fabs(i2(ld(w, c), ld(w, c+kk)))*ld(pr.dzi, k);
-            }
-            else if constexpr (WHAT == 2)
-            {
-                const double dzi = double(ld(pr.dzi, k));
-                val = fabs(double(ld(ev, c))*tprfi*(d.dxi*d.dxi + d.dyi*d.dyi + dzi*dzi));
-            }
-            else
-            {
-                const double div = double(ld(pr.rhoref, k))*(double(ld(u, c+ii)-ld(u, c))*d.dxi + double(ld(v, c+jj)-ld(v, c))*d.dyi)
-                                 + (double(ld(pr.rhorefh, k+1))*double(ld(w, c+kk)) - double(ld(pr.rhorefh, k))*double(ld(w, c)))*double(ld(pr.dzi, k));
-                val = fabs(div);
+                RT val = 0;
+                const long long c = ijk(d, i, j, k);
+                if constexpr (WHAT == 0)
+                {
+                    // CFL 2i5: w interpolated with 2nd/4th/6th order by level.
+                    const int ord = face_order_w(d, k);
+                    TF wc;
+                    if (ord == 2) wc = f2(w, c+kk, kk);
+                    else if (ord == 4) wc = f4(w, c+kk, kk);
+                    else wc = f6(w, c+kk, kk);
+                    val = fabs(f6(u, c+ii, ii))*dxi_of<TF>(d) + fabs(f6(v, c+jj, jj))*dyi_of<TF>(d) + fabs(wc)*ld(pr.dzi, k);
+                }
+                else if constexpr (WHAT == 1)
+                {
+                    val = fabs(i2(ld(u, c), ld(u, c+ii)))*dxi_of<TF>(d) + fabs(i2(ld(v, c), ld(v, c+jj)))*dyi_of<TF>(d)
+                        + fabs(i2(ld(w, c), ld(w, c+kk)))*ld(pr.dzi, k);
+                }
+                else if constexpr (WHAT == 2)
+                {
+                    const double dzi = double(ld(pr.dzi, k));
+                    val = fabs(double(ld(ev, c))*tprfi*(d.dxi*d.dxi + d.dyi*d.dyi + dzi*dzi));
+                }
+                else
+                {
+                    const double div = double(ld(pr.rhoref, k))*(double(ld(u, c+ii)-ld(u, c))*d.dxi + double(ld(v, c+jj)-ld(v, c))*d.dyi)
+                                     + (double(ld(pr.rhorefh, k+1))*double(ld(w, c+kk)) - double(ld(pr.rhorefh, k))*double(ld(w, c)))*double(ld(pr.dzi, k));
+                    val = fabs(div);
+                }
+                best = max_nan(best, val);
             }
         }
+        RT val = best;
         // Block max (NaN kept), then one atomic per block.
         for (int o=16; o>0; o>>=1)
             val = max_nan(val, __shfl_xor_sync(0xffffffffu, val, o));
@@ -857,7 +868,7 @@ namespace mhh
                        const TF* ev, double tprfi, unsigned long long* out, cudaStream_t s)
     {
         dim3 block(32, 8);
-        dim3 grid((d.itot + 31)/32, (d.jtot + 7)/8, d.ktot);
+        dim3 grid((d.itot + 31)/32, (d.jtot + 7)/8, (d.ktot + RED_K - 1)/RED_K);
         if (what == 0) k_reduce<TF, 0><<<grid, block, 0, s>>>(d, pr, u, v, w, ev, tprfi, out);
         else if (what == 1) k_reduce<TF, 1><<<grid, block, 0, s>>>(d, pr, u, v, w, ev, tprfi, out);
         else if (what == 2) k_reduce<TF, 2><<<grid, block, 0, s>>>(d, pr, u, v, w, ev, tprfi, out);
