@@ -102,6 +102,9 @@ namespace mhh
     template<typename TF> void launch_tendency_flux(const Dims& d, const Prof<TF>& pr, const TendArgs<TF>& a,
                                                     bool surf, bool scal, bool buoy, bool lim, int kchunk,
                                                     cudaStream_t s);
+    // Advec_2 + Diff_2 in flux form; force: a.fbody is added to u.
+    template<typename TF> void launch_tendency_2(const Dims& d, const Prof<TF>& pr, const TendArgs<TF>& a, bool scal,
+                                                 bool buoy, bool force, int kchunk, cudaStream_t s);
     // Buffer-layer relaxation, src/buffer.cxx:37-59: prof holds, kcells each,
     // sigma(z) at full levels, sigma(zh) at half levels (zero below the
     // layer) and the u, v, s buffer profiles.

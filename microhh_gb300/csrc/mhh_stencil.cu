@@ -521,6 +521,13 @@ namespace mhh
             else launch_tendency_les<TF>(d, pr, a, surf, scal, buoy, s);
             return;
         }
+        // The DNS combination in flux form (mhh_tend_2.cu); its terms alone (the
+        // module calls) and every other combination run per cell.
+        if (var == 2 && adv == MHH_ADVEC_2 && dif == MHH_DIFF_2)
+        {
+            launch_tendency_2<TF>(d, pr, a, scal, buoy, force, o.tend_kchunk, s);
+            return;
+        }
         if (lim)
         {
             if (dif == MHH_DIFF_SMAG2) launch_tend_lim<TF, MHH_DIFF_SMAG2>(d, pr, a, surf, buoy, force, s);

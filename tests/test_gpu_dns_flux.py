@@ -1,0 +1,54 @@
+"""The DNS tendencies in flux form (mhh_tend_2.cu: Advec_2 + Diff_2, every face
+flux once) against the per-cell kernel, at the edges of its 32 x 8 tiles and of
+its level chunks, with and without the scalar, buoyancy and the pressure force."""
+import numpy as np
+import pytest
+
+from microhh_gb300 import cases
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def mhh():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import microhh_gb300
+    microhh_gb300.load()
+    return microhh_gb300
+
+
+def make(itot, jtot, ktot, thermo):
+    c = cases.channel(itot, jtot, ktot, seed=71, dt=2.e-4, adaptivestep=False)
+    if thermo:
+        c.thermo, c.svisc, c.swlspres = True, 1. / 130., False
+        c.sbcbot, c.sbctop, c.sbot, c.stop = cases.BC_DIRICHLET, cases.BC_NEUMANN, 301., 0.2
+        rng = np.random.default_rng(72)
+        c.fields["th"] = 300. + 0.1 * rng.standard_normal((ktot, jtot, itot))
+    return c
+
+
+@pytest.mark.parametrize("thermo", [False, True], ids=["channel", "thermo"])
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("itot,jtot,ktot", [(4, 3, 2), (31, 7, 9), (32, 8, 8), (33, 9, 65), (64, 16, 129), (98, 25, 66)])
+def test_flux_form_against_per_cell(mhh, itot, jtot, ktot, precision, thermo):
+    """One substep in both forms.  They round the same sums in another order:
+    the bounds of the channel against the oracle, 1e-12 in FP64 and 5e-6 in
+    float (theta, stored as its difference from 300 K, by the same rule)."""
+    case = make(itot, jtot, ktot, thermo)
+    out = {}
+    for variant in (0, 2):
+        mhh.set_option("tendency_kernel", variant)
+        try:
+            m = mhh.Model(case, precision=precision)
+            m.run_substeps(1, fused=True)
+            out[variant] = {n: case.interior(m.get(n)) - (300. if n == "th" else 0.) for n in case.prognostic_names()}
+            m.close()
+        finally:
+            mhh.set_option("tendency_kernel", -1)
+    tol = 1e-12 if precision == 64 else 5e-6
+    for n, a in out[2].items():
+        b = out[0][n]
+        assert np.isfinite(a).all()
+        assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b), (n, np.linalg.norm(a - b) / np.linalg.norm(b))
