@@ -123,8 +123,8 @@ namespace mhh
     struct FftPlan
     {
         int n;
-        int nfac;
-        int fac[16];
+        int ngfac;        // radices (2 to 10) of the run-time plan
+        int gfac[16];
         double* tw_d;     // exp(-2 pi i k/n), k < n, as (re, im) pairs (double)
         float* tw_f;      // the same in float
     };

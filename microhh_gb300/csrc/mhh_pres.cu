@@ -5,11 +5,13 @@
 // column between the forward and inverse transforms is in mhh_tdma.cu.
 //
 // FFT: two real sequences x, y of length n are transformed together as
-// z = x + i y with a mixed-radix (4, 2, 3, 5, 7) Stockham autosort FFT in
-// shared memory (ping-pong buffers, one barrier per stage), or for n = 128,
+// z = x + i y with a mixed-radix Stockham autosort FFT in shared memory
+// (ping-pong buffers, one barrier per stage; compile-time stages for the common
+// lengths, run-time plans of radices 2 to 10 for the others), or for n = 128,
 // 256 and 512 with a warp-synchronous schedule (one warp per sequence), then
 // separated by Hermitian symmetry into FFTW's halfcomplex order r_0 ..
 // r_{n/2}, i_{(n+1)/2-1} .. i_1 (the convention of src/fft.cxx:145-206).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -44,32 +46,6 @@ namespace mhh
         typename C2<TF>::T r; r.x = __ldg(t + 2*e); r.y = __ldg(t + 2*e + 1); return r;
     }
 
-    // Radix-R butterfly (R = 5 or 7, a compile-time constant) of one item of
-    // a run-time-plan stage: the inputs x[i + q*T] times the stage twiddles
-    // w^(q*k*step) (an index below n), then a direct DFT whose twiddles
-    // w^(q*r*T) are w^(((q*r) mod R)*T).
-    template<typename TF, int R>
-    __device__ __forceinline__ void radix_gen(const typename C2<TF>::T* __restrict__ x, typename C2<TF>::T* __restrict__ y,
-                                              const TF* __restrict__ tt, int i, int T, int k, int step, int j, int p)
-    {
-        using T2 = typename C2<TF>::T;
-        T2 u[R];
-        u[0] = x[i];
-        #pragma unroll
-        for (int q=1; q<R; ++q) u[q] = cmul(x[i + q*T], tw<TF>(tt, q*k*step));
-        T2 wr[R];
-        #pragma unroll
-        for (int m=0; m<R; ++m) wr[m] = tw<TF>(tt, m*T);
-        #pragma unroll
-        for (int r=0; r<R; ++r)
-        {
-            T2 acc = u[0];
-            #pragma unroll
-            for (int q=1; q<R; ++q) acc = cadd(acc, cmul(u[q], wr[(q*r) % R]));
-            y[j + r*p] = acc;
-        }
-    }
-
     // Quotient and remainder of a / b for 0 <= a < 2^20 and b >= 1 from a
     // float reciprocal rb ~ 1/b: the float quotient is within one of the
     // exact one, and one correction step in either direction makes it exact
@@ -83,85 +59,6 @@ namespace mhh
         rem = r;
         return q;
     }
-
-    // All Stockham stages for P sequences of length n held in buf[0] (complex,
-    // [P][n]); returns the buffer index that holds the natural-order result.
-    template<typename TF>
-    __device__ int stockham(const FftPlan& pl, typename C2<TF>::T* buf0, typename C2<TF>::T* buf1, int P)
-    {
-        using T2 = typename C2<TF>::T;
-        const TF* tt = twtab<TF>(pl);
-        const int n = pl.n;
-        T2* src = buf0;
-        T2* dst = buf1;
-        int which = 0;
-        int p = 1;
-        for (int s=0; s<pl.nfac; ++s)
-        {
-            const int R = pl.fac[s];
-            const int T = n / R;
-            const int step = n / (p*R);
-            const int nitem = P*T;
-            const float rT = 1.f/(float)T, rp = 1.f/(float)p;
-            for (int it = threadIdx.x; it < nitem; it += blockDim.x)
-            {
-                int i, k;
-                const int seq = div_rcp(it, T, rT, i);
-                div_rcp(i, p, rp, k);
-                const T2* x = src + seq*n;
-                T2* y = dst + seq*n;
-                const int j = (i - k)*R + k;
-                if (R == 2)
-                {
-                    T2 u0 = x[i], u1 = cmul(x[i + T], tw<TF>(tt, k*step));
-                    y[j] = cadd(u0, u1);
-                    y[j + p] = csub(u0, u1);
-                }
-                else if (R == 4)
-                {
-                    // q*k*step < R*p*step = n: no reduction modulo n.
-                    T2 u0 = x[i];
-                    T2 u1 = cmul(x[i +   T], tw<TF>(tt, 1*k*step));
-                    T2 u2 = cmul(x[i + 2*T], tw<TF>(tt, 2*k*step));
-                    T2 u3 = cmul(x[i + 3*T], tw<TF>(tt, 3*k*step));
-                    const T2 a = cadd(u0, u2), b = csub(u0, u2);
-                    const T2 c = cadd(u1, u3), e = csub(u1, u3);
-                    // v_r = sum_q u_q (-i)^(q r)
-                    T2 v1, v3;
-                    v1.x = b.x + e.y; v1.y = b.y - e.x;   // b - i e
-                    v3.x = b.x - e.y; v3.y = b.y + e.x;   // b + i e
-                    y[j] = cadd(a, c);
-                    y[j + p] = v1;
-                    y[j + 2*p] = csub(a, c);
-                    y[j + 3*p] = v3;
-                }
-                else if (R == 3)
-                {
-                    T2 u0 = x[i];
-                    T2 u1 = cmul(x[i +   T], tw<TF>(tt, 1*k*step));
-                    T2 u2 = cmul(x[i + 2*T], tw<TF>(tt, 2*k*step));
-                    const TF s3 = TF(0.86602540378443864676);
-                    const T2 t1 = cadd(u1, u2), t4 = csub(u1, u2);
-                    T2 t2; t2.x = u0.x - TF(0.5)*t1.x; t2.y = u0.y - TF(0.5)*t1.y;
-                    // v1 = t2 - i s3 t4, v2 = t2 + i s3 t4
-                    T2 v1, v2;
-                    v1.x = t2.x + s3*t4.y; v1.y = t2.y - s3*t4.x;
-                    v2.x = t2.x - s3*t4.y; v2.y = t2.y + s3*t4.x;
-                    y[j] = cadd(u0, t1);
-                    y[j + p] = v1;
-                    y[j + 2*p] = v2;
-                }
-                else if (R == 5) radix_gen<TF, 5>(x, y, tt, i, T, k, step, j, p);
-                else radix_gen<TF, 7>(x, y, tt, i, T, k, step, j, p);
-            }
-            __syncthreads();
-            T2* t = src; src = dst; dst = t;
-            which ^= 1;
-            p *= R;
-        }
-        return which;
-    }
-
 
     // ---- fixed-length transforms -----------------------------------------
     // For the common lengths the radices are compile-time constants (8 first,
@@ -542,7 +439,7 @@ namespace mhh
     // Lengths that run the warp-synchronous schedule.
     __host__ __device__ constexpr bool warp_len(int n) { return n == 128 || n == 256 || n == 512; }
 
-    template<typename TF> struct FftP { FftPlan pl; TF* data; SeqLayout L; int Prt; TF scale; FftFuse<TF> fz; };
+    template<typename TF> struct FftP { FftPlan pl; TF* data; SeqLayout L; TF scale; FftFuse<TF> fz; };
     template<typename TF, int FUSE> struct FftOcc { static constexpr int v = (FUSE == 1 && sizeof(TF) == 4) ? 5 : 1; };
 
     template<typename TF, bool INV, int NFIX, int PFIX, int FUSE>
@@ -551,13 +448,11 @@ namespace mhh
         const FftPlan& pl = A.pl;
         TF* __restrict__ data = A.data;
         const SeqLayout& L = A.L;
-        const int Prt = A.Prt;
         const TF scale = A.scale;
         const FftFuse<TF>& fz = A.fz;
         using T2 = typename C2<TF>::T;
         extern __shared__ __align__(16) unsigned char smem_raw[];
-        const int n = NFIX ? NFIX : pl.n;
-        const int P = NFIX ? PFIX : Prt;
+        constexpr int n = NFIX, P = PFIX;
         // Each buffer holds P complex sequences plus P elements of padding:
         // viewed as 2P real sequences, the column (y) layout strides them by
         // n + 1 so that a warp reading one element of 16+ sequences hits
@@ -571,7 +466,7 @@ namespace mhh
 
         constexpr bool WARP = warp_len(NFIX);
         if constexpr (WARP) warp_twiddles<TF, NFIX/64>(tws, twtab<TF>(pl));
-        else if (NFIX)
+        else
         {
             const TF* tt = twtab<TF>(pl);
             for (int e = threadIdx.x; e < n; e += blockDim.x)
@@ -651,7 +546,7 @@ namespace mhh
                 fft_cp_async(r1 + ls*ns + j, ok ? data + ti.sb[ls] + j : data, ok);
             }
         }
-        else if (NFIX && (256 % (2*(PFIX ? PFIX : 1))) == 0)
+        else if ((256 % (2*PFIX)) == 0)
         {
             // Columns: with 2P dividing the block size every thread keeps
             // one sequence (ls) and walks its elements.
@@ -716,19 +611,10 @@ namespace mhh
         __syncthreads();
 
         // 3. FFT.
-        if (NFIX)
-        {
-            T2* src = buf0;
-            T2* dst = buf1;
-            FixedStages<TF, (NFIX ? NFIX : 1), (PFIX ? PFIX : 1), 0, 1>::run(src, dst, tws);
-            res = src; other = dst;
-        }
-        else
-        {
-            const int which = stockham<TF>(pl, buf0, buf1, P);
-            res = which ? buf1 : buf0;
-            other = which ? buf0 : buf1;
-        }
+        T2* src = buf0;
+        T2* dst = buf1;
+        FixedStages<TF, NFIX, PFIX, 0, 1>::run(src, dst, tws);
+        res = src; other = dst;
         }
         TF* rout = reinterpret_cast<TF*>(other);
 
@@ -783,7 +669,7 @@ namespace mhh
                 if (ls < nloc) data[ti.sb[ls] + j] = rout[ls*ns + j];
             }
         }
-        else if (NFIX && (256 % (2*(PFIX ? PFIX : 1))) == 0)
+        else if ((256 % (2*PFIX)) == 0)
         {
             const int ls = threadIdx.x % (2*P);
             if (ls < nloc)
@@ -1079,30 +965,13 @@ namespace mhh
         launch_body<B, body, NT, 1>(dim3((unsigned)nblk), dim3(NT), smem, s, B{data, L, scale, fz, twt, ntiles});
     }
 
-    // Dynamic shared-memory limit of the run-time-plan FFT (two buffers of at
-    // most 96 KB of sequences, plus padding).
-    constexpr int FFT_GENERIC_SMEM = 100*1024;
-
-    template<typename TF>
-    static int pairs_per_block(int n, bool rows)
-    {
-        // Two complex buffers of P*n each within 96 KB; columns want at least
-        // 16 (float) or 8 (double) adjacent sequences for coalescing.
-        const size_t per = 2*sizeof(typename C2<TF>::T)*(size_t)n;
-        int P = (int)((96*1024) / per);
-        const int want = rows ? 4 : (sizeof(TF) == 4 ? 8 : 4);
-        if (P > want) P = want;
-        if (P < 1) P = 1;
-        return P;
-    }
-
     template<typename TF, bool INV, int NF, int PF, int FUSE>
     static void launch_fixed(const FftPlan& pl, TF* data, SeqLayout L, TF scale, const FftFuse<TF>& fz, cudaStream_t s)
     {
         const size_t smem = sizeof(typename C2<TF>::T)*((size_t)2*(PF*NF + PF) + NF);
         const long long nblk = (L.nseq + 2*PF - 1) / (2*PF);
         launch_body<FftP<TF>, fft_body<TF, INV, NF, PF, FUSE>, 256, FftOcc<TF, FUSE>::v>(
-            dim3((unsigned)nblk), dim3(256), smem, s, FftP<TF>{pl, data, L, PF, scale, fz});
+            dim3((unsigned)nblk), dim3(256), smem, s, FftP<TF>{pl, data, L, scale, fz});
     }
 
     template<typename TF, bool INV, int NF>
@@ -1150,17 +1019,405 @@ namespace mhh
             || try_fixed_n<TF, INV, 768>(pl, data, L, scale, fz, s) || try_fixed_n<TF, INV, 16>(pl, data, L, scale, fz, s);
     }
 
-    template<typename TF, bool INV, int FUSE>
+    // ---- run-time plans -----------------------------------------------------
+    // Any length 2^a 3^b 5^c 7^d.  A block transforms a tile of 2P real
+    // sequences (P = 2^lp) held element-major in shared memory, element j of
+    // pair q at j*S + q: consecutive threads take the pairs of one element, so
+    // the index of a butterfly is a shift, its twiddles are broadcasts, and for
+    // columns (y) the pair of adjacent real columns is the complex element as it
+    // lies in memory.  Stages of radix 2 to 10 (as few as the length allows) run
+    // in registers between two buffers, one barrier each; the first forms the
+    // complex input and the store separates the result.  The schedule it
+    // replaces ran radices 2 to 7 with separate packing and separation passes,
+    // global twiddle loads and two integer divisions per element: x and y
+    // transforms per step at 150^3 0.80 -> 0.30 ms in float, 189 x 105 x 90
+    // 0.45 -> 0.20 (what bounds it now is shared-memory latency with a barrier
+    // per stage).
+    constexpr int FG_NT = 128;
+    constexpr int FG_SMEM = 200*1024;
+
+    template<typename T2> __device__ __forceinline__ void gdft2(T2* u)
+    { const T2 a = u[0]; u[0] = cadd(a, u[1]); u[1] = csub(a, u[1]); }
+
+    template<typename TF, typename T2> __device__ __forceinline__ void gdft3(T2& a, T2& b, T2& c)
+    {
+        const TF s3 = TF(0.86602540378443864676);
+        const T2 t1 = cadd(b, c), t4 = csub(b, c);
+        T2 t2; t2.x = a.x - TF(0.5)*t1.x; t2.y = a.y - TF(0.5)*t1.y;
+        a = cadd(a, t1);
+        b.x = t2.x + s3*t4.y; b.y = t2.y - s3*t4.x;
+        c.x = t2.x - s3*t4.y; c.y = t2.y + s3*t4.x;
+    }
+
+    template<typename T2> __device__ __forceinline__ void gdft4(T2& u0, T2& u1, T2& u2, T2& u3)
+    {
+        const T2 a = cadd(u0, u2), b = csub(u0, u2), c = cadd(u1, u3), e = mul_mi<T2>(csub(u1, u3));
+        u0 = cadd(a, c); u2 = csub(a, c); u1 = cadd(b, e); u3 = csub(b, e);
+    }
+
+    // Odd prime R: the pairs u_q, u_{R-q} as sums and differences.
+    template<typename TF, typename T2> __device__ __forceinline__ void gdft5(T2& u0, T2& u1, T2& u2, T2& u3, T2& u4)
+    {
+        const TF c1 = TF(0.30901699437494742410), c2 = TF(-0.80901699437494742410);
+        const TF s1 = TF(0.95105651629515357212), s2 = TF(0.58778525229247312917);
+        const T2 p1 = cadd(u1, u4), p2 = cadd(u2, u3), m1 = csub(u1, u4), m2 = csub(u2, u3);
+        T2 a1, a2, b1, b2;
+        a1.x = u0.x + c1*p1.x + c2*p2.x; a1.y = u0.y + c1*p1.y + c2*p2.y;
+        a2.x = u0.x + c2*p1.x + c1*p2.x; a2.y = u0.y + c2*p1.y + c1*p2.y;
+        b1.x = s1*m1.x + s2*m2.x; b1.y = s1*m1.y + s2*m2.y;
+        b2.x = s2*m1.x - s1*m2.x; b2.y = s2*m1.y - s1*m2.y;
+        u0 = cadd(u0, cadd(p1, p2));
+        u1.x = a1.x + b1.y; u1.y = a1.y - b1.x; u4.x = a1.x - b1.y; u4.y = a1.y + b1.x;
+        u2.x = a2.x + b2.y; u2.y = a2.y - b2.x; u3.x = a2.x - b2.y; u3.y = a2.y + b2.x;
+    }
+
+    template<typename TF, typename T2> __device__ __forceinline__ void gdft7(T2* u)
+    {
+        const TF c[3] = {TF(0.62348980185873353053), TF(-0.22252093395631440429), TF(-0.90096886790241912624)};
+        const TF s[3] = {TF(0.78183148246802980871), TF(0.97492791218182360702), TF(0.43388373911755812048)};
+        T2 p[3], m[3];
+        #pragma unroll
+        for (int q=0; q<3; ++q) { p[q] = cadd(u[q+1], u[6-q]); m[q] = csub(u[q+1], u[6-q]); }
+        const T2 u0 = u[0];
+        u[0] = cadd(u0, cadd(p[0], cadd(p[1], p[2])));
+        #pragma unroll
+        for (int r=1; r<4; ++r)
+        {
+            T2 a = u0, b; b.x = TF(0); b.y = TF(0);
+            #pragma unroll
+            for (int q=1; q<4; ++q)
+            {
+                // cos and sin of 2 pi q r/7 from the first three multiples.
+                const int e = (q*r) % 7;
+                const TF cc = c[(e < 4 ? e : 7 - e) - 1], ss = e < 4 ? s[e - 1] : -s[6 - e];
+                a.x += cc*p[q-1].x; a.y += cc*p[q-1].y;
+                b.x += ss*m[q-1].x; b.y += ss*m[q-1].y;
+            }
+            u[r].x = a.x + b.y; u[r].y = a.y - b.x;
+            u[7-r].x = a.x - b.y; u[7-r].y = a.y + b.x;
+        }
+    }
+
+    // Forward DFT of u[0..R-1] in place.  6 and 10 as 2 x 3 and 2 x 5 by the
+    // coprime-factor map (no twiddles), 9 as 3 x 3.
+    template<typename TF, int R, typename T2>
+    __device__ __forceinline__ void gdft(T2* u)
+    {
+        if constexpr (R == 2) gdft2(u);
+        else if constexpr (R == 3) gdft3<TF>(u[0], u[1], u[2]);
+        else if constexpr (R == 4) gdft4(u[0], u[1], u[2], u[3]);
+        else if constexpr (R == 5) gdft5<TF>(u[0], u[1], u[2], u[3], u[4]);
+        else if constexpr (R == 7) gdft7<TF>(u);
+        else if constexpr (R == 8) dft8<TF, T2>(u);
+        else if constexpr (R == 6)
+        {
+            // n = 3 a + 2 b mod 6, k = 3 a' + 4 b' mod 6.
+            T2 x[2][3] = {{u[0], u[2], u[4]}, {u[3], u[5], u[1]}};
+            gdft3<TF>(x[0][0], x[0][1], x[0][2]);
+            gdft3<TF>(x[1][0], x[1][1], x[1][2]);
+            #pragma unroll
+            for (int b=0; b<3; ++b)
+            {
+                u[(4*b) % 6] = cadd(x[0][b], x[1][b]);
+                u[(4*b + 3) % 6] = csub(x[0][b], x[1][b]);
+            }
+        }
+        else if constexpr (R == 10)
+        {
+            // n = 5 a + 2 b mod 10, k = 5 a' + 6 b' mod 10.
+            T2 x[2][5];
+            #pragma unroll
+            for (int b=0; b<5; ++b) { x[0][b] = u[2*b]; x[1][b] = u[(2*b + 5) % 10]; }
+            gdft5<TF>(x[0][0], x[0][1], x[0][2], x[0][3], x[0][4]);
+            gdft5<TF>(x[1][0], x[1][1], x[1][2], x[1][3], x[1][4]);
+            #pragma unroll
+            for (int b=0; b<5; ++b)
+            {
+                u[(6*b) % 10] = cadd(x[0][b], x[1][b]);
+                u[(6*b + 5) % 10] = csub(x[0][b], x[1][b]);
+            }
+        }
+        else if constexpr (R == 9)
+        {
+            // X[3 s + r] = sum_a w9^(a r) [DFT3_b u[a + 3 b]](r) w3^(a s).
+            const TF c1 = TF(0.76604444311897803520), s1 = TF(-0.64278760968653932632);
+            const TF c2 = TF(0.17364817766693034885), s2 = TF(-0.98480775301220805937);
+            const TF c4 = TF(-0.93969262078590838405), s4 = TF(-0.34202014332566873304);
+            #pragma unroll
+            for (int a=0; a<3; ++a) gdft3<TF>(u[a], u[a+3], u[a+6]);
+            T2 w1, w2, w4;
+            w1.x = c1; w1.y = s1; w2.x = c2; w2.y = s2; w4.x = c4; w4.y = s4;
+            u[4] = cmul(u[4], w1); u[5] = cmul(u[5], w2);
+            u[7] = cmul(u[7], w2); u[8] = cmul(u[8], w4);
+            #pragma unroll
+            for (int r=0; r<3; ++r) gdft3<TF>(u[3*r], u[3*r + 1], u[3*r + 2]);
+            // u[3 r + s] holds X[3 s + r].
+            T2 t;
+            t = u[1]; u[1] = u[3]; u[3] = t;
+            t = u[2]; u[2] = u[6]; u[6] = t;
+            t = u[5]; u[5] = u[7]; u[7] = t;
+        }
+    }
+
+    template<typename TF> struct FftgP
+    {
+        TF* data; SeqLayout L; TF scale; FftFuse<TF> fz; const TF* twt;
+        int n, lp, nst;
+        int pairs;              // columns: the pairs of a tile are adjacent in memory
+        unsigned long long fac; // radices, four bits each, first stage lowest
+    };
+
+    // One Stockham stage of radix R (p = the product of the radices before):
+    // item (i, q), k = i mod p, reads src[i + r T] times w^(r k step) and writes
+    // dst[(i - k) R + k + r p].  FIRST: p = 1, no twiddles; with INV the input
+    // is the conjugated halfcomplex pair.
+    template<typename TF, int R, bool FIRST, bool INV>
+    __device__ __forceinline__ void fg_stage(const typename C2<TF>::T* __restrict__ src, typename C2<TF>::T* __restrict__ dst,
+                                             const typename C2<TF>::T* __restrict__ tw, int n, int p, int S, int lp)
+    {
+        using T2 = typename C2<TF>::T;
+        const int T = n/R, step = T/p;
+        const float rp = 1.f/(float)p;
+        const int q = threadIdx.x & ((1 << lp) - 1);
+        for (int i = threadIdx.x >> lp; i < T; i += FG_NT >> lp)
+        {
+            int k = 0;
+            if (!FIRST) div_rcp(i, p, rp, k);
+            T2 u[R];
+            #pragma unroll
+            for (int r=0; r<R; ++r)
+            {
+                const int e = i + r*T;
+                if (FIRST && INV)
+                {
+                    const int kk = 2*e <= n ? e : n - e;
+                    const bool real_only = kk == 0 || 2*kk == n;
+                    const T2 a = src[kk*S + q], b = src[(real_only ? kk : n - kk)*S + q];
+                    const TF sg = real_only ? TF(0) : (2*e <= n ? TF(1) : TF(-1));
+                    u[r].x = a.x - sg*b.y;
+                    u[r].y = -(sg*b.x + a.y);
+                }
+                else
+                    u[r] = (FIRST || r == 0) ? src[e*S + q] : cmul(src[e*S + q], tw[r*k*step]);
+            }
+            gdft<TF, R>(u);
+            T2* y = dst + ((i - k)*R + k)*S + q;
+            #pragma unroll
+            for (int r=0; r<R; ++r) y[r*p*S] = u[r];
+        }
+    }
+
+    template<typename TF, bool FIRST, bool INV>
+    __device__ __forceinline__ void fg_any(int R, const typename C2<TF>::T* src, typename C2<TF>::T* dst,
+                                           const typename C2<TF>::T* tw, int n, int p, int S, int lp)
+    {
+        switch (R)
+        {
+            case 2: fg_stage<TF, 2, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            case 3: fg_stage<TF, 3, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            case 4: fg_stage<TF, 4, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            case 5: fg_stage<TF, 5, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            case 6: fg_stage<TF, 6, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            case 7: fg_stage<TF, 7, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            case 8: fg_stage<TF, 8, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            case 9: fg_stage<TF, 9, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            default: fg_stage<TF, 10, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+        }
+    }
+
+    template<typename T2>
+    __device__ __forceinline__ void fg_copy2(T2* dst, const T2* src)
+    {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n"
+                     :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"(sizeof(T2)) : "memory");
+    }
+
+    template<typename TF, bool INV, int FUSE, bool ROWS>
+    __device__ __forceinline__ void fftg_body(const FftgP<TF>& A, const VBlock& vb)
+    {
+        using T2 = typename C2<TF>::T;
+        const int n = A.n, lp = A.lp, P = 1 << lp, S = P + (lp ? 1 : 0);
+        const SeqLayout& L = A.L;
+        const FftFuse<TF>& fz = A.fz;
+        extern __shared__ __align__(16) unsigned char smem_raw[];
+        T2* b0 = reinterpret_cast<T2*>(smem_raw);
+        T2* b1 = b0 + (size_t)n*S;
+        T2* tw = b1 + (size_t)n*S;
+        __shared__ TileIdx ti;
+        const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+        const long long s0 = (long long)vb.x*2*P;
+        const int nloc = (int)min((long long)2*P, L.nseq - s0);
+        tile_index<TF>(ti, L, fz, s0, nloc, n, FUSE != 0);
+        __syncthreads();
+        for (int e = tid; e < n; e += FG_NT) fg_copy2(tw + e, reinterpret_cast<const T2*>(A.twt) + e);
+
+        // 1. Load; a missing sequence reads as zero.
+        TF* r0 = reinterpret_cast<TF*>(b0);
+        if (FUSE == 1)
+        {
+            // Rows of the pressure right-hand side in place of a load
+            // (src/pres_2.cxx:155-196), a warp per row.
+            const Dims& d = fz.d;
+            for (int ls = warp; ls < 2*P; ls += FG_NT/32)
+            {
+                TF* dst = r0 + ls;                  // component ls & 1 of pair ls >> 1
+                if (ls < nloc)
+                {
+                    const long long c = ti.sc[ls];
+                    const int kg = ti.sk[ls] + d.kgc;
+                    const TF rho = ld(fz.pr.rhoref, kg), rb = ld(fz.pr.rhorefh, kg), rt = ld(fz.pr.rhorefh, kg+1);
+                    const TF dzi = ld(fz.pr.dzi, kg), dti = fz.dti;
+                    const TF *u = fz.u + c, *v = fz.v + c, *w = fz.w + c, *ut = fz.ut + c, *vt = fz.vt + c, *wt = fz.wt + c;
+                    const int jj = d.icells, kk = d.ijcells;
+                    #pragma unroll 2
+                    for (int i = lane; i < n; i += 32)
+                    {
+                        const TF du = (ld(ut, i+1) + mulx(ld(u, i+1), dti)) - (ld(ut, i) + mulx(ld(u, i), dti));
+                        const TF dv = (ld(vt, i+jj) + mulx(ld(v, i+jj), dti)) - (ld(vt, i) + mulx(ld(v, i), dti));
+                        const TF dw = mulx(rt, ld(wt, i+kk) + mulx(ld(w, i+kk), dti)) - mulx(rb, ld(wt, i) + mulx(ld(w, i), dti));
+                        dst[2*i*S] = mulx(mulx(rho, du), dxi_of<TF>(d)) + mulx(mulx(rho, dv), dyi_of<TF>(d)) + mulx(dw, dzi);
+                    }
+                }
+                else
+                    for (int i = lane; i < n; i += 32) dst[2*i*S] = TF(0);
+            }
+        }
+        else if (ROWS)
+        {
+            for (int ls = warp; ls < 2*P; ls += FG_NT/32)
+            {
+                const bool ok = ls < nloc;
+                const TF* src = ok ? A.data + ti.sb[ls] : A.data;
+                #pragma unroll 4
+                for (int i = lane; i < n; i += 32) fft_cp_async(r0 + ls + 2*i*S, ok ? src + i : src, ok);
+            }
+        }
+        else
+        {
+            const int q = tid & (P - 1);
+            const bool ok0 = 2*q < nloc, ok1 = 2*q + 1 < nloc;
+            const TF* x = A.data + (ok0 ? ti.sb[2*q] : 0);
+            const TF* y = A.data + (ok1 ? ti.sb[2*q + 1] : 0);
+            if (A.pairs && ok1)
+            {
+                #pragma unroll 4
+                for (int j = tid >> lp; j < n; j += FG_NT >> lp)
+                    fg_copy2(b0 + j*S + q, reinterpret_cast<const T2*>(x + (long long)j*L.itot));
+            }
+            else
+                for (int j = tid >> lp; j < n; j += FG_NT >> lp)
+                {
+                    fft_cp_async(r0 + 2*(j*S + q), ok0 ? x + (long long)j*L.itot : x, ok0);
+                    fft_cp_async(r0 + 2*(j*S + q) + 1, ok1 ? y + (long long)j*L.itot : y, ok1);
+                }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+
+        // 2. Stages.
+        T2* src = b0;
+        T2* dst = b1;
+        int p = 1;
+        for (int st=0; st<A.nst; ++st)
+        {
+            const int R = (int)(A.fac >> 4*st) & 15;
+            if (st == 0) fg_any<TF, true, INV>(R, src, dst, tw, n, 1, S, lp);
+            else fg_any<TF, false, INV>(R, src, dst, tw, n, p, S, lp);
+            p *= R;
+            __syncthreads();
+            T2* t = src; src = dst; dst = t;
+        }
+
+        // 3. Store: real and imaginary parts (inverse) or the halfcomplex
+        //    separation (forward).
+        auto pair_out = [&](int k, int q) -> T2
+        {
+            T2 o;
+            if (INV)
+            {
+                const T2 a = src[k*S + q];
+                o.x = a.x*A.scale; o.y = -a.y*A.scale;
+            }
+            else
+            {
+                const int kk = 2*k <= n ? k : n - k;
+                const T2 a = src[kk*S + q], b = src[(kk == 0 ? 0 : n - kk)*S + q];
+                if (2*k <= n) { o.x = TF(0.5)*(a.x + b.x); o.y = TF(0.5)*(a.y + b.y); }
+                else { o.x = TF(0.5)*(a.y - b.y); o.y = TF(-0.5)*(a.x - b.x); }
+            }
+            return o;
+        };
+        if (ROWS)
+        {
+            for (int ls = warp; ls < nloc; ls += FG_NT/32)
+            {
+                if (FUSE == 2)
+                {
+                    // Straight into the ghost layout of p, with the bottom
+                    // ghost level p[kstart-1] = p[kstart]
+                    // (src/pres_2.cxx:330-358).
+                    const TF mean = fz.dcm ? fz.dcm[ti.sk[ls]] : TF(0);
+                    for (int i = lane; i < n; i += 32)
+                    {
+                        const T2 o = pair_out(i, ls >> 1);
+                        TF val = ls & 1 ? o.y : o.x;
+                        if (fz.dcm) val = add_rn(val, mean);
+                        const long long c = ti.sc[ls] + i;
+                        fz.p[c] = val;
+                        if (ti.sk[ls] == 0) fz.p[c - fz.d.ijcells] = val;
+                    }
+                }
+                else
+                {
+                    TF* out = A.data + ti.sb[ls];
+                    for (int i = lane; i < n; i += 32) { const T2 o = pair_out(i, ls >> 1); out[i] = ls & 1 ? o.y : o.x; }
+                }
+            }
+        }
+        else
+        {
+            const int q = tid & (P - 1);
+            const bool ok0 = 2*q < nloc, ok1 = 2*q + 1 < nloc;
+            TF* x = A.data + (ok0 ? ti.sb[2*q] : 0);
+            TF* y = A.data + (ok1 ? ti.sb[2*q + 1] : 0);
+            for (int j = tid >> lp; j < n; j += FG_NT >> lp)
+            {
+                const T2 o = pair_out(j, q);
+                const long long e = (long long)j*L.itot;
+                if (A.pairs && ok1) *reinterpret_cast<T2*>(x + e) = o;
+                else
+                {
+                    if (ok0) x[e] = o.x;
+                    if (ok1) y[e] = o.y;
+                }
+            }
+        }
+    }
+
+    template<typename TF, bool INV, int FUSE, bool ROWS>
     static void launch_generic(const FftPlan& pl, TF* data, SeqLayout L, TF scale, const FftFuse<TF>& fz, cudaStream_t s)
     {
-        const int n = pl.n;
-        const int P = pairs_per_block<TF>(n, L.rows != 0);
-        const size_t smem = 2*sizeof(typename C2<TF>::T)*((size_t)P*n + P);
-        const long long nblk = (L.nseq + 2*P - 1) / (2*P);
-        // The shared memory depends on n: the limit is set to the largest.
-        set_smem_limit<FftP<TF>, fft_body<TF, INV, 0, 0, FUSE>, 256, FftOcc<TF, FUSE>::v>(FFT_GENERIC_SMEM);
-        launch_body<FftP<TF>, fft_body<TF, INV, 0, 0, FUSE>, 256, FftOcc<TF, FUSE>::v>(
-            dim3((unsigned)nblk), dim3(256), smem, s, FftP<TF>{pl, data, L, P, scale, fz});
+        using T2 = typename C2<TF>::T;
+        using B = FftgP<TF>;
+        constexpr auto body = fftg_body<TF, INV, FUSE, ROWS>;
+        B A{};
+        A.data = data; A.L = L; A.scale = scale; A.fz = fz;
+        A.twt = sizeof(TF) == 8 ? reinterpret_cast<const TF*>(pl.tw_d) : reinterpret_cast<const TF*>(pl.tw_f);
+        A.n = pl.n;
+        A.nst = pl.ngfac;
+        for (int q=0; q<pl.ngfac; ++q) A.fac |= (unsigned long long)pl.gfac[q] << 4*q;
+        // Eight pairs (64- or 128-byte runs of columns), fewer where two
+        // buffers of them do not fit.
+        auto bytes = [&](int lp) { return sizeof(T2)*(size_t)pl.n*(2*((1 << lp) + (lp ? 1 : 0)) + 1); };
+        A.lp = 3;
+        while (A.lp > 0 && bytes(A.lp) > (size_t)FG_SMEM) --A.lp;
+        // Pairs of columns move as one element where they are adjacent and the
+        // data is aligned for it.
+        A.pairs = !ROWS && L.itot % 2 == 0 && reinterpret_cast<size_t>(data) % sizeof(T2) == 0;
+        const int per = 2 << A.lp;
+        const long long nblk = (L.nseq + per - 1)/per;
+        set_smem_limit<B, body, FG_NT, 4>(FG_SMEM);
+        launch_body<B, body, FG_NT, 4>(dim3((unsigned)nblk), dim3(FG_NT), bytes(A.lp), s, A);
     }
 
     template<typename TF>
@@ -1172,15 +1429,20 @@ namespace mhh
         count_launch();
         if (inverse ? launch_fixed_any<TF, true>(pl, data, L, scale, fz, s) : launch_fixed_any<TF, false>(pl, data, L, scale, fz, s))
             return;
-        if (inverse)
+        if (!L.rows)
         {
-            if (L.rows && fz.mode == 2) launch_generic<TF, true, 2>(pl, data, L, scale, fz, s);
-            else launch_generic<TF, true, 0>(pl, data, L, scale, fz, s);
+            if (inverse) launch_generic<TF, true, 0, false>(pl, data, L, scale, fz, s);
+            else launch_generic<TF, false, 0, false>(pl, data, L, scale, fz, s);
+        }
+        else if (inverse)
+        {
+            if (fz.mode == 2) launch_generic<TF, true, 2, true>(pl, data, L, scale, fz, s);
+            else launch_generic<TF, true, 0, true>(pl, data, L, scale, fz, s);
         }
         else
         {
-            if (L.rows && fz.mode == 1) launch_generic<TF, false, 1>(pl, data, L, scale, fz, s);
-            else launch_generic<TF, false, 0>(pl, data, L, scale, fz, s);
+            if (fz.mode == 1) launch_generic<TF, false, 1, true>(pl, data, L, scale, fz, s);
+            else launch_generic<TF, false, 0, true>(pl, data, L, scale, fz, s);
         }
     }
 
@@ -1206,15 +1468,42 @@ namespace mhh
     }
 
 #if MHH_PREC == 64
+    // The radices (2 to 10) of the run-time plan: the fewest factors, and of
+    // those the smallest sum (the least arithmetic), larger ones first.
+    static void plan_radices(FftPlan* pl)
+    {
+        const int n = pl->n;
+        std::vector<int> divs, best, pick;      // divisors of n, best radix of each
+        for (int d=1; d<=n; ++d) if (n % d == 0) divs.push_back(d);
+        best.assign(divs.size(), 1 << 20);
+        pick.assign(divs.size(), 0);
+        best[0] = 0;
+        for (size_t a=1; a<divs.size(); ++a)
+            for (int r=2; r<=10; ++r)
+                if (divs[a] % r == 0)
+                {
+                    const size_t b = std::lower_bound(divs.begin(), divs.end(), divs[a]/r) - divs.begin();
+                    const int cost = best[b] + 64 + r;
+                    if (cost < best[a]) { best[a] = cost; pick[a] = r; }
+                }
+        pl->ngfac = 0;
+        for (int d = n; d > 1; )
+        {
+            const size_t a = std::lower_bound(divs.begin(), divs.end(), d) - divs.begin();
+            pl->gfac[pl->ngfac++] = pick[a];
+            d /= pick[a];
+        }
+        std::sort(pl->gfac, pl->gfac + pl->ngfac, [](int x, int y) { return x > y; });
+    }
+
     int fft_plan_init(FftPlan* pl, int n, cudaStream_t s)
     {
         std::memset(pl, 0, sizeof(*pl));
         pl->n = n;
         int r = n;
-        const int radices[] = {4, 2, 3, 5, 7};
-        for (int q=0; q<5 && r>1; ++q)
-            while (r % radices[q] == 0 && pl->nfac < 16) { pl->fac[pl->nfac++] = radices[q]; r /= radices[q]; }
+        for (int f : {2, 3, 5, 7}) while (r % f == 0) r /= f;
         if (r != 1) return MHH_ERR_UNSUPPORTED;
+        plan_radices(pl);
         std::vector<double> td(2*(size_t)n);
         std::vector<float> tf(2*(size_t)n);
         const long double twopi = 6.283185307179586476925286766559005768L;

@@ -31,7 +31,7 @@ def make(itot, jtot, ktot, thermo):
 
 @pytest.mark.parametrize("thermo", [False, True], ids=["channel", "thermo"])
 @pytest.mark.parametrize("precision", [64, 32])
-@pytest.mark.parametrize("itot,jtot,ktot", [(4, 3, 2), (31, 7, 9), (32, 8, 8), (33, 9, 65), (64, 16, 129), (98, 25, 66)])
+@pytest.mark.parametrize("itot,jtot,ktot", [(4, 3, 2), (30, 7, 9), (32, 8, 8), (35, 9, 65), (64, 16, 129), (98, 25, 66)])
 def test_flux_form_against_per_cell(mhh, itot, jtot, ktot, precision, thermo):
     """One substep in both forms.  They round the same sums in another order:
     the bounds of the channel against the oracle, 1e-12 in FP64 and 5e-6 in
