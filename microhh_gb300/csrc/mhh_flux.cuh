@@ -22,6 +22,12 @@ namespace mhh
         else
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(s), "l"(src), "r"(n) : "memory");
     }
+    template<typename TF>
+    __device__ __forceinline__ void cp_async_one(TF* dst, const TF* src)
+    {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n"
+                     :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"(sizeof(TF)) : "memory");
+    }
     __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
     __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 

@@ -70,34 +70,43 @@ namespace mhh
         const int pc = (min(fy, DTY) + 1)*DPW + fx + 1;
         const int gxi = fy*DNX + fx, gyi = fy*DTX + fx;
 
-        // The (at most) two plane elements this thread copies per plane.
-        int go[2];
-        #pragma unroll
-        for (int q=0; q<2; ++q)
+        // 32-bit unsigned indexes, and what the fields of a level share computed
+        // once (see tend_flux_body).  The (at most) two plane elements this
+        // thread copies per plane; beyond the last ghost cell the last one is
+        // copied, which no stored cell uses.
+        const unsigned ij = (unsigned)d.ijcells;
+        const int top = d.kcells - 1, e1 = tid + DNT;
+        const bool two = e1 < DPS;
+        unsigned go0, go1;
         {
-            const int e = tid + q*DNT, pj = e / DPW, pi = e - pj*DPW;
-            const int gi = i0 - 1 + pi, gj = j0 - 1 + pj;
-            go[q] = e >= DPS ? -1 : (gi < d.icells && gj < d.jcells ? gi + gj*d.icells : -2);
+            const int pj = tid / DPW, pi = tid - pj*DPW;
+            go0 = min(i0 - 1 + pi, d.icells - 1) + (unsigned)min(j0 - 1 + pj, d.jcells - 1)*d.icells;
         }
-        auto plane = [&](int slot, const TF* f, int l)
         {
-            if (l > d.kcells - 1) return;
-            TF* dst = sm + (slot + l%4)*DPS + tid;
-            const TF* src = f + (long long)l*d.ijcells;
-            #pragma unroll
-            for (int q=0; q<2; ++q)
-                if (go[q] != -1) cp_async_el(dst + q*DNT, go[q] >= 0 ? src + go[q] : f, go[q] >= 0);
-        };
+            const int pj = e1 / DPW, pi = e1 - pj*DPW;
+            go1 = two ? min(i0 - 1 + pi, d.icells - 1) + (unsigned)min(j0 - 1 + pj, d.jcells - 1)*d.icells : 0u;
+        }
         auto planes = [&](int l)
         {
-            plane(DSU, a.u, l); plane(DSV, a.v, l); plane(DSW, a.w, l);
-            if (SCAL) plane(DSS, a.s, l);
+            const unsigned lo = (unsigned)min(l, top)*ij;
+            TF* dst = sm + (l & 3)*DPS + tid;
+            cp_async_one(dst + DSU*DPS, a.u + (go0 + lo));
+            cp_async_one(dst + DSV*DPS, a.v + (go0 + lo));
+            cp_async_one(dst + DSW*DPS, a.w + (go0 + lo));
+            if (SCAL) cp_async_one(dst + DSS*DPS, a.s + (go0 + lo));
+            if (two)
+            {
+                cp_async_one(dst + DSU*DPS + DNT, a.u + (go1 + lo));
+                cp_async_one(dst + DSV*DPS + DNT, a.v + (go1 + lo));
+                cp_async_one(dst + DSW*DPS + DNT, a.w + (go1 + lo));
+                if (SCAL) cp_async_one(dst + DSS*DPS + DNT, a.s + (go1 + lo));
+            }
         };
 
         const int m0 = k0 - 1;
         for (int q = tid; q < P.kchunk + 2; q += DNT)
         {
-            const int l = min(m0 + q, d.kcells - 1);
+            const int l = min(m0 + q, top);
             lev[0*DPLEV + q] = pr.dzhi[l];
             lev[1*DPLEV + q] = pr.dzi[l];
             if (BUOY) { lev[2*DPLEV + q] = TF(GRAV)/pr.threfh[l]; lev[3*DPLEV + q] = pr.thbh[l]; }
@@ -105,7 +114,7 @@ namespace mhh
         for (int l = m0; l <= m0 + 2; ++l) planes(l);
         cp_async_commit();
 
-        const long long col = cell ? (long long)i + (long long)j*d.icells : 0;
+        const unsigned col = cell ? (unsigned)(i + j*d.icells) : 0u;
         const TF visc = a.visc, svisc = a.svisc;
         const TF dxi = dxi_of<TF>(d), dyi = dyi_of<TF>(d);
         // Factors of the differences and of the products of sums.
@@ -121,13 +130,12 @@ namespace mhh
             const int buf = (m - m0) & 1, lq = m - m0;
             TF* gx = gxb + buf*NF*DNGX;
             TF* gy = gyb + buf*NF*DNGY;
-            const TF* U0 = sm + (DSU + m%4)*DPS + pc;
-            const TF* U1 = sm + (DSU + (m+1)%4)*DPS + pc;
-            const TF* V0 = sm + (DSV + m%4)*DPS + pc;
-            const TF* V1 = sm + (DSV + (m+1)%4)*DPS + pc;
-            const TF* W1 = sm + (DSW + (m+1)%4)*DPS + pc;
-            const TF* S0 = sm + (DSS + m%4)*DPS + pc;
-            const TF* S1 = sm + (DSS + (m+1)%4)*DPS + pc;
+            const TF* L0 = sm + (m & 3)*DPS + pc;
+            const TF* L1 = sm + ((m + 1) & 3)*DPS + pc;
+            const TF* U0 = L0 + DSU*DPS; const TF* U1 = L1 + DSU*DPS;
+            const TF* V0 = L0 + DSV*DPS; const TF* V1 = L1 + DSV*DPS;
+            const TF* W1 = L1 + DSW*DPS;
+            const TF* S0 = L0 + DSS*DPS; const TF* S1 = L1 + DSS*DPS;
             // The planes of level m+3, first used two iterations on, into the
             // slots that iteration m-1 freed.
             if (m + 2 < k1) planes(m + 3);
@@ -135,15 +143,15 @@ namespace mhh
 
             const bool wlev = m+1 > d.kstart && m+1 < d.kend;
             const bool write = cell && m >= k0;
-            const long long c = col + (long long)m*d.ijcells;
+            const unsigned c = col + (unsigned)m*ij;
             TF tu = 0, tv = 0, tw = 0, ts = 0, w2 = 0;
             if (write)
             {
                 tu = a.ut[c]; tv = a.vt[c];
-                if (wlev) tw = a.wt[c + d.ijcells];
+                if (wlev) tw = a.wt[c + ij];
                 if (SCAL) ts = a.st[c];
             }
-            if (cell && m + 2 < d.kcells) w2 = __ldg(a.w + c + 2LL*d.ijcells);
+            if (cell && m + 2 < d.kcells) w2 = __ldg(a.w + (c + 2u*ij));
 
             if (face)
             {
@@ -189,7 +197,7 @@ namespace mhh
                 if (SCAL) zs_t = fma(w1*(S0[0] + S1[0]), q2, (S1[0] - S0[0])*(svisc*dzh));
                 if (BUOY && wlev)
                 {
-                    const TF sb = SCAL ? S0[0] : __ldg(a.s + c), st = SCAL ? S1[0] : __ldg(a.s + c + d.ijcells);
+                    const TF sb = SCAL ? S0[0] : __ldg(a.s + c), st = SCAL ? S1[0] : __ldg(a.s + (c + ij));
                     buoy = lev[2*DPLEV + lq + 1]*(i2(sb, st) - lev[3*DPLEV + lq + 1]);
                 }
             }
@@ -209,7 +217,7 @@ namespace mhh
                 };
                 a.ut[c] = total(0, tu + a.fbody, zu_b, zu_t, dz);
                 a.vt[c] = total(1, tv, zv_b, zv_t, dz);
-                if (wlev) a.wt[c + d.ijcells] = total(2, tw + buoy, zw_b, zw_t, dzh);
+                if (wlev) a.wt[c + ij] = total(2, tw + buoy, zw_b, zw_t, dzh);
                 if (SCAL) a.st[c] = total(3, ts, zs_b, zs_t, dz);
             }
             zu_b = zu_t; zv_b = zv_t; zw_b = zw_t; zs_b = zs_t;
@@ -223,7 +231,7 @@ namespace mhh
         constexpr size_t smem = tend2_smem<TF, SCAL>();
         const int nx = (d.itot + DTX - 1)/DTX, ny = (d.jtot + DTY - 1)/DTY;
         kchunk = min(auto_kchunk(kchunk, (long long)nx*ny, d.ktot), DKCHUNK_MAX);
-        launch_body<Tend2P<TF>, tend2_body<TF, SCAL, BUOY>, DNT, 2>(
+        launch_body<Tend2P<TF>, tend2_body<TF, SCAL, BUOY>, DNT, (sizeof(TF) == 4 ? 3 : 2)>(
             dim3(nx, ny, (d.ktot + kchunk - 1)/kchunk), dim3(DNT), smem, s, Tend2P<TF>{d, pr, a, kchunk});
         count_launch();
     }

@@ -45,9 +45,10 @@ namespace mhh
         constexpr int NFX = FTX + 1, NFY = FTY + 1;
         constexpr int NTHR = 320;
         constexpr int FKCHUNK_MAX = 64;
-        // Plane slots: u 4, v 4, w 3, s 3, evisc 4; level l of a field lives
-        // in slot base + l % n.  Planes are prefetched two levels ahead.
-        constexpr int SU = 0, SV = 4, SW = 8, SS = 11, SE = 14, NSLOT = 18;
+        // Plane slots: four per field; level l of a field lives in slot
+        // base + l % 4, so that the planes of one level sit at one offset from
+        // their fields' bases.  Planes are prefetched two levels ahead.
+        constexpr int SU = 0, SV = 4, SW = 8, SS = 12, SE = 16, NSLOT = 20;
         constexpr int NGX = FTY*NFX;            // x-faces per level and field
         constexpr int NGY = NFY*FTX;            // y-faces per level and field
         constexpr int NEL1 = FPS - NTHR;        // threads that copy a second element
@@ -94,29 +95,34 @@ namespace mhh
         const int pc = (min(fy, FTY) + FH)*FPW + (fx + FH);   // own (i, j) in a plane
         const int gxi = fy*NFX + fx, gyi = fy*FTX + fx;
 
-        // The (at most) two plane elements this thread copies per plane.
-        const int e0 = tid, e1 = tid + NTHR;
-        int go0, go1;
-        bool v0, v1;
+        // Indexes into the fields are 32-bit and unsigned (fewer than 2^32 cells),
+        // and whatever the fields of a level share is computed once: with 64-bit
+        // offsets per field, slots modulo 3 and bounds tests per copy, integer
+        // and uniform instructions were nearly half of the 761 a cell took in
+        // float.
+        //
+        // The (at most) two plane elements this thread copies per plane.  Beyond
+        // the last ghost cell the last one is copied; no stored cell uses it.
+        const unsigned ij = (unsigned)d.ijcells;
+        const int top = d.kcells - 1;
+        const int e1 = tid + NTHR;
+        const bool two = tid < NEL1;
+        unsigned go0, go1;
         {
-            const int pj = e0 / FPW, pi = e0 - pj*FPW;
-            const int gi = i0 - FH + pi, gj = j0 - FH + pj;
-            v0 = gi < d.icells && gj < d.jcells;
-            go0 = v0 ? gi + gj*d.icells : 0;
+            const int pj = tid / FPW, pi = tid - pj*FPW;
+            go0 = min(i0 - FH + pi, d.icells - 1) + (unsigned)min(j0 - FH + pj, d.jcells - 1)*d.icells;
         }
         {
             const int pj = e1 / FPW, pi = e1 - pj*FPW;
-            const int gi = i0 - FH + pi, gj = j0 - FH + pj;
-            v1 = tid < NEL1 && gi < d.icells && gj < d.jcells;
-            go1 = v1 ? gi + gj*d.icells : 0;
+            go1 = two ? min(i0 - FH + pi, d.icells - 1) + (unsigned)min(j0 - FH + pj, d.jcells - 1)*d.icells : 0u;
         }
-        auto plane = [&](int slot, const TF* f, int l)
+        // Plane of field f (level offset lo, slot offset so) into the slots from
+        // base on.
+        auto plane = [&](int base, const TF* f, unsigned lo, int so)
         {
-            if (l > d.kcells - 1) return;
-            TF* dst = sm + slot*FPS;
-            const TF* src = f + (long long)l*d.ijcells;
-            cp_async_el(dst + e0, v0 ? src + go0 : f, v0);
-            if (tid < NEL1) cp_async_el(dst + e1, v1 ? src + go1 : f, v1);
+            TF* dst = sm + base*FPS + so + tid;
+            cp_async_one(dst, f + (go0 + lo));
+            if (two) cp_async_one(dst + NTHR, f + (go1 + lo));
         };
 
         const TF* __restrict__ u = a.u;
@@ -124,18 +130,15 @@ namespace mhh
         const TF* __restrict__ w = a.w;
         const TF* __restrict__ s = a.s;
         const TF* __restrict__ ev = a.evisc;
-        const long long col = cell ? (long long)i + (long long)j*d.icells : 0;
-        auto colval = [&](const TF* f, int l) -> TF
-        {
-            l = l < 0 ? 0 : (l > d.kcells-1 ? d.kcells-1 : l);
-            return __ldg(f + col + (long long)l*d.ijcells);
-        };
+        const unsigned col = cell ? (unsigned)(i + j*d.icells) : 0u;
+        // Offset of level l, clamped to the levels there are.
+        auto level = [&](int l) { return (unsigned)min(max(l, 0), top)*ij; };
 
         // Per-level constants of the chunk: index l - m0 for level l.
         const int m0 = k0 - 1;
         for (int q = tid; q < kchunk + 2; q += NTHR)
         {
-            const int l = min(m0 + q, d.kcells - 1);
+            const int l = min(m0 + q, top);
             prof[0*PLEV + q] = pr.dzhi[l];
             prof[1*PLEV + q] = pr.rhorefh[l];
             prof[2*PLEV + q] = pr.rhoref[l];
@@ -149,9 +152,10 @@ namespace mhh
         // Planes of the first three iterations (m0 .. m0+2).
         for (int l = m0; l <= m0+3; ++l)
         {
-            plane(SU + l%4, u, l); plane(SV + l%4, v, l); plane(SE + l%4, ev, l);
-            if (l > m0) plane(SW + l%3, w, l);
-            if (SCAL && l < m0+3) plane(SS + l%3, s, l);
+            const unsigned lo = level(l);
+            const int so = (l & 3)*FPS;
+            plane(SU, u, lo, so); plane(SV, v, lo, so); plane(SE, ev, lo, so); plane(SW, w, lo, so);
+            if (SCAL && l < m0+3) plane(SS, s, lo, so);
         }
         cp_async_commit();
 
@@ -163,10 +167,11 @@ namespace mhh
             #pragma unroll
             for (int q=0; q<6; ++q)
             {
-                qu[q] = colval(u, m0-2+q);
-                qv[q] = colval(v, m0-2+q);
-                qw[q] = colval(w, m0-1+q);
-                qs[q] = (SCAL || BUOY) ? colval(s, m0-2+q) : TF(0);
+                const unsigned l = col + level(m0 - 2 + q);
+                qu[q] = __ldg(u + l);
+                qv[q] = __ldg(v + l);
+                qw[q] = __ldg(w + (col + level(m0 - 1 + q)));
+                qs[q] = (SCAL || BUOY) ? __ldg(s + l) : TF(0);
             }
         }
         TF ufb = 0, uft = 0, vfb = 0, vft = 0, sfb = 0, sft = 0;
@@ -188,7 +193,7 @@ namespace mhh
         TF ex0 = 0, ey0 = 0, ex1 = 0, ey1 = 0;
         if (sizeof(TF) == 8 && face)
         {
-            const TF* E = sm + (SE + m0%4)*FPS + pc;
+            const TF* E = sm + SE*FPS + (m0 & 3)*FPS + pc;
             ex0 = E[-1] + E[0];
             ey0 = E[-FPW] + E[0];
         }
@@ -198,37 +203,39 @@ namespace mhh
             const int buf = (m - m0) & 1;
             TF* gx = gbase + buf*4*NGX;
             TF* gy = gbase + 2*4*NGX + buf*4*NGY;
-            const TF* U0 = sm + (SU + m%4)*FPS + pc;
-            const TF* U1 = sm + (SU + (m+1)%4)*FPS + pc;
-            const TF* V0 = sm + (SV + m%4)*FPS + pc;
-            const TF* V1 = sm + (SV + (m+1)%4)*FPS + pc;
-            const TF* W1 = sm + (SW + (m+1)%3)*FPS + pc;
-            const TF* S0 = sm + (SS + m%3)*FPS + pc;
-            const TF* E0 = sm + (SE + m%4)*FPS + pc;
-            const TF* E1 = sm + (SE + (m+1)%4)*FPS + pc;
+            // Own point in the planes of levels m and m+1.
+            const TF* L0 = sm + (m & 3)*FPS + pc;
+            const TF* L1 = sm + ((m + 1) & 3)*FPS + pc;
+            const TF* U0 = L0 + SU*FPS; const TF* U1 = L1 + SU*FPS;
+            const TF* V0 = L0 + SV*FPS; const TF* V1 = L1 + SV*FPS;
+            const TF* W1 = L1 + SW*FPS;
+            const TF* S0 = L0 + SS*FPS;
+            const TF* E0 = L0 + SE*FPS; const TF* E1 = L1 + SE*FPS;
             #define PL(P, dx, dy) (P)[(dy)*FPW + (dx)]
 
             const bool write = cell && m >= k0;
             const bool wlev = m+1 > d.kstart && m+1 < d.kend;
-            const long long c = col + (long long)m*d.ijcells;
+            const unsigned c = col + (unsigned)m*ij;
             // Early loads: the tendencies this iteration updates and the queue
             // entries of the next iteration.
             TF tu = 0, tv = 0, tw = 0, ts = 0;
             if (write)
             {
                 tu = a.ut[c]; tv = a.vt[c];
-                if (wlev) tw = a.wt[c + d.ijcells];
+                if (wlev) tw = a.wt[c + ij];
                 if (SCAL) ts = a.st[c];
             }
+            const unsigned lo4 = (unsigned)min(m + 4, top)*ij;
             TF nu = 0, nv = 0, nw = 0, ns = 0;
             if (cell)
             {
-                nu = colval(u, m+4); nv = colval(v, m+4); nw = colval(w, m+5);
-                if (SCAL || BUOY) ns = colval(s, m+4);
+                nu = __ldg(u + (col + lo4)); nv = __ldg(v + (col + lo4));
+                nw = __ldg(w + (col + (unsigned)min(m + 5, top)*ij));
+                if (SCAL || BUOY) ns = __ldg(s + (col + lo4));
             }
 
-            const int lq = m + 1 - m0;      // index of level m+1 in prof
-            const TF dzhi1 = prof[0*PLEV + lq];
+            const TF* pl = prof + (m + 1 - m0);      // constants of level m+1
+            const TF dzhi1 = pl[0*PLEV];
 
             // ---- faces: shear stresses and total fluxes ----
             TF txz = 0, tyz = 0;
@@ -369,7 +376,7 @@ namespace mhh
             {
                 const int kf = m + 1;
                 const int ot = face_order_full(d, kf);
-                const TF rhoh1 = prof[1*PLEV + lq];
+                const TF rhoh1 = pl[1*PLEV];
                 // u and v: diffusive flux from the shear stress of the same
                 // face, or the surface model's flux at the walls.
                 const TF du = (SURF && kf == d.kstart) ? -ufb : ((SURF && kf == d.kend) ? -uft : txz);
@@ -428,7 +435,7 @@ namespace mhh
                 if (kf < d.kend)
                 {
                     const int ow = face_order_w(d, kf);
-                    const TF dw = TF(2)*(PL(E1,0,0) + visc)*(qw[3] - qw[2])*prof[3*PLEV + lq];
+                    const TF dw = TF(2)*(PL(E1,0,0) + visc)*(qw[3] - qw[2])*pl[3*PLEV];
                     TF aw;
                     if (paired) aw = aws.x;
                     else if (sizeof(TF) == 8 && ow == 6)
@@ -440,10 +447,10 @@ namespace mhh
                     else if (ow == 4) aw = i2(qw[2], qw[3])*i4ws(qw[1], qw[2], qw[3], qw[4])
                                          - fabs(i2(qw[2], qw[3]))*i3ws(qw[1], qw[2], qw[3], qw[4]);
                     else aw = i2(qw[2], qw[3])*i2(qw[2], qw[3]);
-                    gzw_t = prof[2*PLEV + lq]*(dw - aw);
+                    gzw_t = pl[2*PLEV]*(dw - aw);
                 }
                 if (BUOY && wlev)
-                    buoy = prof[4*PLEV + lq]*(i2(qs[2], qs[3]) - prof[7*PLEV + lq]);
+                    buoy = pl[4*PLEV]*(i2(qs[2], qs[3]) - pl[7*PLEV]);
             }
             #undef PL
 
@@ -456,18 +463,16 @@ namespace mhh
             // iteration m freed.
             if (m + 3 < k1)
             {
-                plane(SU + (m+4)%4, u, m+4);
-                plane(SV + (m+4)%4, v, m+4);
-                plane(SW + (m+4)%3, w, m+4);
-                plane(SE + (m+4)%4, ev, m+4);
-                if (SCAL) plane(SS + (m+3)%3, s, m+3);
+                const int so = (m & 3)*FPS;
+                plane(SU, u, lo4, so); plane(SV, v, lo4, so); plane(SW, w, lo4, so); plane(SE, ev, lo4, so);
+                if (SCAL) plane(SS, s, (unsigned)(m + 3)*ij, ((m + 3) & 3)*FPS);
             }
             cp_async_commit();
 
             if (write)
             {
                 const int gx0 = gxi, gy0 = gyi;
-                const TF zf = prof[5*PLEV + lq - 1];
+                const TF zf = pl[5*PLEV - 1];
                 if constexpr (sizeof(TF) == 4)
                 {
                     // The four fields' face fluxes in one 16-byte load per face;
@@ -489,14 +494,14 @@ namespace mhh
                         const float2 dgx = sub2(f2(xb.z, xb.w), f2(xa.z, xa.w));
                         const float2 dgy = sub2(f2(yb.z, yb.w), f2(ya.z, ya.w));
                         const float2 dgz = sub2(f2(gzw_t, gzs_t), f2(gzw_b, gzs_b));
-                        const float2 t = __ffma2_rn(dgz, f2(prof[6*PLEV + lq], zf), __ffma2_rn(dgy, f2(dyi, dyi),
+                        const float2 t = __ffma2_rn(dgz, f2(pl[6*PLEV], zf), __ffma2_rn(dgy, f2(dyi, dyi),
                                                     __ffma2_rn(dgx, f2(dxi, dxi), f2(tw + buoy, ts))));
-                        if (wlev) a.wt[c + d.ijcells] = t.x;
+                        if (wlev) a.wt[c + ij] = t.x;
                         a.st[c] = t.y;
                     }
                     else if (wlev)
-                        a.wt[c + d.ijcells] = tw + (xb.z - xa.z)*dxi + (yb.z - ya.z)*dyi
-                                                 + (gzw_t - gzw_b)*prof[6*PLEV + lq] + buoy;
+                        a.wt[c + ij] = tw + (xb.z - xa.z)*dxi + (yb.z - ya.z)*dyi
+                                                 + (gzw_t - gzw_b)*pl[6*PLEV] + buoy;
                 }
                 else
                 {
@@ -505,9 +510,9 @@ namespace mhh
                     a.vt[c] = tv + (gx[(gx0 + 1)*4 + 1] - gx[(gx0)*4 + 1])*dxi
                                  + (gy[(gy0 + FTX)*4 + 1] - gy[(gy0)*4 + 1])*dyi + (gzv_t - gzv_b)*zf;
                     if (wlev)
-                        a.wt[c + d.ijcells] = tw + (gx[(gx0 + 1)*4 + 2] - gx[(gx0)*4 + 2])*dxi
+                        a.wt[c + ij] = tw + (gx[(gx0 + 1)*4 + 2] - gx[(gx0)*4 + 2])*dxi
                                                  + (gy[(gy0 + FTX)*4 + 2] - gy[(gy0)*4 + 2])*dyi
-                                                 + (gzw_t - gzw_b)*prof[6*PLEV + lq] + buoy;
+                                                 + (gzw_t - gzw_b)*pl[6*PLEV] + buoy;
                     if (SCAL)
                         a.st[c] = ts + (gx[(gx0 + 1)*4 + 3] - gx[(gx0)*4 + 3])*dxi
                                      + (gy[(gy0 + FTX)*4 + 3] - gy[(gy0)*4 + 3])*dyi + (gzs_t - gzs_b)*zf;

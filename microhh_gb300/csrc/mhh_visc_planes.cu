@@ -19,6 +19,7 @@
 // and the edge terms keep only the w gradients (include/diff_kernels.h:57-103);
 // that level is computed from the planes directly.
 #include "mhh_kernels.cuh"
+#include "mhh_flux.cuh"
 #include "mhh_batchable.cuh"
 
 namespace mhh
@@ -36,15 +37,16 @@ namespace mhh
         constexpr int VSU = 0, VSV = 4, VSW = 8, VNSLOT = 12;
         constexpr int VNEL1 = VPS - VNT;        // threads that copy a second element
         // Edge buffers: xy [VNY][VNX] for two levels (written and read in the
-        // same iteration); xz [VTY][VNX] and yz [VNY][VTX] for three half
-        // levels (an iteration reads the half levels below and above its
-        // level while the next one writes the following half level).
+        // same iteration); xz [VTY][VNX] and yz [VNY][VTX] for four half levels
+        // (an iteration reads the half levels below and above its level while
+        // the next one writes the following half level; four, so that the slot
+        // is a mask).
         constexpr int NXY = VNY*VNX, NXZ = VTY*VNX, NYZ = VNY*VTX;
 
         constexpr int VPLEV = VKCHUNK_MAX + 2;  // per-level constants of levels m0 .. m0+kchunk+1
 
         template<typename TF>
-        size_t visc_smem() { return sizeof(TF)*(size_t(VNSLOT)*VPS + 2*NXY + 3*(NXZ + NYZ) + 5*VPLEV); }
+        size_t visc_smem() { return sizeof(TF)*(size_t(VNSLOT)*VPS + 2*NXY + 4*(NXZ + NYZ) + 5*VPLEV); }
 
         // The eddy viscosity from S^2 and N^2, src/diff_smag2.cxx:171-174:
         // mlen^2 sqrt(S^2) sqrt(1 - min(N^2/(S^2 Pr), 1 - 1e-9)), as mlen^2
@@ -66,17 +68,6 @@ namespace mhh
                 return t < s2 ? ml2*sqrt(s2 - t) : TF(0);
             }
         }
-    }
-
-    template<typename TF>
-    __device__ __forceinline__ void cp_async_v(TF* dst, const TF* src, bool valid)
-    {
-        const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-        const int n = valid ? (int)sizeof(TF) : 0;
-        if constexpr (sizeof(TF) == 4)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" :: "r"(s), "l"(src), "r"(n) : "memory");
-        else
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(s), "l"(src), "r"(n) : "memory");
     }
 
     template<typename TF> struct ViscPlanesP
@@ -105,9 +96,9 @@ namespace mhh
         extern __shared__ __align__(16) unsigned char smem_raw[];
         TF* sm = reinterpret_cast<TF*>(smem_raw);
         TF* exy = sm + VNSLOT*VPS;          // [2][NXY], by iteration parity
-        TF* exz = exy + 2*NXY;              // [3][NXZ], by half level % 3
-        TF* eyz = exz + 3*NXZ;              // [3][NYZ], by half level % 3
-        TF* lev = eyz + 3*NYZ;              // [5][VPLEV]: dzhi, dzi, g/thref, mlen2, spare
+        TF* exz = exy + 2*NXY;              // [4][NXZ], by half level % 4
+        TF* eyz = exz + 4*NXZ;              // [4][NYZ], by half level % 4
+        TF* lev = eyz + 4*NYZ;              // [5][VPLEV]: dzhi, dzi, g/thref, mlen2, spare
 
         // Warps 0-8 own the edge rows ey = 0..8 (ex = lane); warp 9 owns the
         // last edge column ex = 32 of the rows ey = 0..8.
@@ -123,28 +114,34 @@ namespace mhh
         const int k1 = min(k0 + kchunk, d.kend);
         const int pc = (min(ey, VTY) + VH)*VPW + (ex + VH);
 
-        const int e0 = tid, e1 = tid + VNT;
-        int go0, go1;
-        bool v0, v1;
+        // 32-bit unsigned indexes, and what the fields of a level share computed
+        // once (see tend_flux_body).  Beyond the last ghost cell the last one is
+        // copied; no stored cell uses it.
+        const unsigned ij = (unsigned)d.ijcells;
+        const int top = d.kcells - 1, e1 = tid + VNT;
+        const bool two = tid < VNEL1;
+        unsigned go0, go1;
         {
-            const int pj = e0 / VPW, pi = e0 - pj*VPW;
-            const int gi = i0 - VH + pi, gj = j0 - VH + pj;
-            v0 = gi < d.icells && gj < d.jcells;
-            go0 = v0 ? gi + gj*d.icells : 0;
+            const int pj = tid / VPW, pi = tid - pj*VPW;
+            go0 = min(i0 - VH + pi, d.icells - 1) + (unsigned)min(j0 - VH + pj, d.jcells - 1)*d.icells;
         }
         {
             const int pj = e1 / VPW, pi = e1 - pj*VPW;
-            const int gi = i0 - VH + pi, gj = j0 - VH + pj;
-            v1 = tid < VNEL1 && gi < d.icells && gj < d.jcells;
-            go1 = v1 ? gi + gj*d.icells : 0;
+            go1 = two ? min(i0 - VH + pi, d.icells - 1) + (unsigned)min(j0 - VH + pj, d.jcells - 1)*d.icells : 0u;
         }
-        auto plane = [&](int slot, const TF* f, int l)
+        auto planes = [&](int l)
         {
-            if (l > d.kcells - 1) return;
-            TF* dst = sm + slot*VPS;
-            const TF* src = f + (long long)l*d.ijcells;
-            cp_async_v(dst + e0, v0 ? src + go0 : f, v0);
-            if (tid < VNEL1) cp_async_v(dst + e1, v1 ? src + go1 : f, v1);
+            const unsigned lo = (unsigned)min(l, top)*ij;
+            TF* dst = sm + (l & 3)*VPS + tid;
+            cp_async_one(dst + VSU*VPS, u + (go0 + lo));
+            cp_async_one(dst + VSV*VPS, v + (go0 + lo));
+            cp_async_one(dst + VSW*VPS, w + (go0 + lo));
+            if (two)
+            {
+                cp_async_one(dst + VSU*VPS + VNT, u + (go1 + lo));
+                cp_async_one(dst + VSV*VPS + VNT, v + (go1 + lo));
+                cp_async_one(dst + VSW*VPS + VNT, w + (go1 + lo));
+            }
         };
 
         // Iteration m uses the planes of m and m+1; the loop starts one level
@@ -158,17 +155,17 @@ namespace mhh
             lev[2*VPLEV + q] = TF(GRAV)/pr.thref[l];
             lev[3*VPLEV + q] = mlen2[l];
         }
-        for (int l = m0; l <= m0 + 3; ++l) { plane(VSU + l%4, u, l); plane(VSV + l%4, v, l); plane(VSW + l%4, w, l); }
+        for (int l = m0; l <= m0 + 3; ++l) planes(l);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
 
-        const long long col = cell ? (long long)i + (long long)j*d.icells : 0;
+        const unsigned col = cell ? (unsigned)(i + j*d.icells) : 0u;
         // Theta queue of the own column: levels m-1, m, m+1.
         TF tq0 = 0, tq1 = 0, tq2 = 0;
         if (THERMO && cell)
         {
-            tq0 = __ldg(th + col + (long long)(m0-1 < 0 ? 0 : m0-1)*d.ijcells);
-            tq1 = __ldg(th + col + (long long)m0*d.ijcells);
-            tq2 = __ldg(th + col + (long long)(m0+1)*d.ijcells);
+            tq0 = __ldg(th + (col + (unsigned)max(m0 - 1, 0)*ij));
+            tq1 = __ldg(th + (col + (unsigned)m0*ij));
+            tq2 = __ldg(th + (col + (unsigned)(m0 + 1)*ij));
         }
         const TF dxi = dxi_of<TF>(d), dyi = dyi_of<TF>(d);
         const TF tpri = TF(1)/tpr;
@@ -180,18 +177,15 @@ namespace mhh
         {
             const int lq = m - m0;           // index of level m in lev
             const int b = (m - m0) & 1;      // xy buffer of this iteration
-            const int bt = (m + 1) % 3;      // xz, yz buffer of half level m+1
-            const int bb = m % 3;            // xz, yz buffer of half level m
-            const TF* U0 = sm + (VSU + m%4)*VPS + pc;
-            const TF* U1 = sm + (VSU + (m+1)%4)*VPS + pc;
-            const TF* V0 = sm + (VSV + m%4)*VPS + pc;
-            const TF* V1 = sm + (VSV + (m+1)%4)*VPS + pc;
-            const TF* W0 = sm + (VSW + m%4)*VPS + pc;
-            const TF* W1 = sm + (VSW + (m+1)%4)*VPS + pc;
+            const int bt = (m + 1) & 3;      // xz, yz buffer and plane slot of level m+1
+            const int bb = m & 3;            // the same of level m
+            const TF* U0 = sm + bb*VPS + pc + VSU*VPS; const TF* U1 = sm + bt*VPS + pc + VSU*VPS;
+            const TF* V0 = sm + bb*VPS + pc + VSV*VPS; const TF* V1 = sm + bt*VPS + pc + VSV*VPS;
+            const TF* W0 = sm + bb*VPS + pc + VSW*VPS; const TF* W1 = sm + bt*VPS + pc + VSW*VPS;
             #define Q(P, dx, dy) (P)[(dy)*VPW + (dx)]
 
             TF thn = 0;
-            if (THERMO && cell && m + 2 < d.kcells) thn = __ldg(th + col + (long long)(m+2)*d.ijcells);
+            if (THERMO && cell && m + 2 < d.kcells) thn = __ldg(th + (col + (unsigned)(m + 2)*ij));
 
             // ---- edges: xy at level m, xz and yz at half level m+1 ----
             if (edge)
@@ -252,12 +246,7 @@ namespace mhh
             __syncthreads();
             // Planes first used by iteration m+3 into the slot that iteration
             // m freed.
-            if (m + 3 < k1)
-            {
-                plane(VSU + (m+4)%4, u, m+4);
-                plane(VSV + (m+4)%4, v, m+4);
-                plane(VSW + (m+4)%4, w, m+4);
-            }
+            if (m + 3 < k1) planes(m + 4);
             asm volatile("cp.async.commit_group;\n" ::: "memory");
 
             if (write)
@@ -299,7 +288,7 @@ namespace mhh
                 }
                 else
                     ev = ml2*sqrt(s2);
-                evisc[col + (long long)m*d.ijcells] = ev;
+                evisc[col + (unsigned)m*ij] = ev;
             }
             if (THERMO) { tq0 = tq1; tq1 = tq2; tq2 = thn; }
         }
@@ -315,7 +304,8 @@ namespace mhh
         kchunk = min(auto_kchunk(kchunk, (long long)((d.itot + VTX - 1)/VTX)*((d.jtot + VTY - 1)/VTY), d.ktot),
                      VKCHUNK_MAX);
         dim3 grid((d.itot + VTX - 1)/VTX, (d.jtot + VTY - 1)/VTY, (d.ktot + kchunk - 1)/kchunk);
-        launch_body<ViscPlanesP<TF>, visc_planes_body<TF, SURF, THERMO>, VNT>(grid, dim3(VNT), smem, s,
+        // Three blocks per SM in float (64 registers).
+        launch_body<ViscPlanesP<TF>, visc_planes_body<TF, SURF, THERMO>, VNT, (sizeof(TF) == 4 ? 3 : 1)>(grid, dim3(VNT), smem, s,
             ViscPlanesP<TF>{d, pr, u, v, w, th, evisc, mlen2, dudz, dvdz, dbdz, TF(tpr), kchunk});
         count_launch();
     }

@@ -33,22 +33,32 @@ def make(itot, jtot, ktot, thermo):
 @pytest.mark.parametrize("precision", [64, 32])
 @pytest.mark.parametrize("itot,jtot,ktot", [(4, 3, 2), (30, 7, 9), (32, 8, 8), (35, 9, 65), (64, 16, 129), (98, 25, 66)])
 def test_flux_form_against_per_cell(mhh, itot, jtot, ktot, precision, thermo):
-    """One substep in both forms.  They round the same sums in another order:
-    the bounds of the channel against the oracle, 1e-12 in FP64 and 5e-6 in
-    float (theta, stored as its difference from 300 K, by the same rule)."""
+    """One substep in both forms, which round the same sums in another order.
+    FP64: 1e-12, the bound of the channel against the oracle.  Float: the flux
+    form is no further from FP64 than the per-cell form (half as much again for
+    two samples of the same round-off, which the pressure solve amplifies: on
+    the tallest grid here either form is 4e-6 from FP64 in w)."""
     case = make(itot, jtot, ktot, thermo)
-    out = {}
-    for variant in (0, 2):
+
+    def step(variant, prec):
         mhh.set_option("tendency_kernel", variant)
         try:
-            m = mhh.Model(case, precision=precision)
+            m = mhh.Model(case, precision=prec)
             m.run_substeps(1, fused=True)
-            out[variant] = {n: case.interior(m.get(n)) - (300. if n == "th" else 0.) for n in case.prognostic_names()}
+            out = {n: case.interior(m.get(n)) - (300. if n == "th" else 0.) for n in case.prognostic_names()}
             m.close()
         finally:
             mhh.set_option("tendency_kernel", -1)
-    tol = 1e-12 if precision == 64 else 5e-6
-    for n, a in out[2].items():
-        b = out[0][n]
+        return out
+
+    flux, cell = step(2, precision), step(0, precision)
+    exact = step(0, 64)
+    for n, a in flux.items():
+        norm = np.linalg.norm(exact[n])
         assert np.isfinite(a).all()
-        assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b), (n, np.linalg.norm(a - b) / np.linalg.norm(b))
+        if precision == 64:
+            assert np.linalg.norm(a - cell[n]) <= 1e-12 * norm, n
+        else:
+            ef, ec = np.linalg.norm(a - exact[n]) / norm, np.linalg.norm(cell[n] - exact[n]) / norm
+            print(n, ef, ec)
+            assert ef <= 1.5 * ec + 1e-7, (n, ef, ec)
