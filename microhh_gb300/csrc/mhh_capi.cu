@@ -85,9 +85,9 @@ namespace mhh
     void set_tdma_variant(int v) { g_tdma_variant = v; }
     long long launch_count() { return g_launches.load(); }
 
-    int auto_kchunk(int requested, long long tiles, int ktot)
+    int auto_kchunk(int requested, long long tiles, int ktot, bool dbl, int most)
     {
-        if (requested > 0) return requested;
+        if (requested > 0) return std::min(requested, most);
         static const int nsm = []
         {
             int dev = 0, n = 0;
@@ -95,12 +95,23 @@ namespace mhh
             cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
             return n > 0 ? n : 152;
         }();
-        // 64 levels (fewer halo levels per chunk) while the grid still gives
-        // eight blocks per SM; else 32, halved while it gives fewer than two.
-        if (tiles*((ktot + 63)/64) >= 8LL*nsm) return 64;
-        int kc = 32;
-        while (kc > 8 && tiles*((ktot + kc - 1)/kc) < 2LL*nsm) kc /= 2;
-        return kc;
+        // In levels per SM, a chunk costing its own and three more (the level
+        // below it and the first planes' latency).  Float: two or three blocks
+        // share an SM and its issue slots, so the work spreads evenly up to the
+        // last blocks to finish, which take their whole march.  Double: the FP64
+        // pipe serves one block as fast as two, so whole waves of one block per
+        // SM count.
+        int best = 0;
+        double cost = 0.;
+        for (int n = (ktot + most - 1)/most; n <= ktot; ++n)
+        {
+            const int kc = (ktot + n - 1)/n;
+            const double blocks = double(tiles)*((ktot + kc - 1)/kc);
+            const double t = dbl ? std::ceil(blocks/nsm)*(kc + 3)
+                                 : (double(tiles)*ktot + 3.*blocks)/nsm + 1.25*(kc + 3);
+            if (!best || t < cost) { best = kc; cost = t; }
+        }
+        return best;
     }
 
     // a += delta over a whole 3-D field (mhh_field_shift).

@@ -13,18 +13,22 @@ namespace mhh
     constexpr int ADVEC_2I5_LIM = 26;
 
     // Kernel choices of one call: variant switches (-1 = automatic) and the
-    // level-chunk height of the marching kernels (0 = default 32).
+    // level-chunk height of the marching kernels (0 = chosen by auto_kchunk).
     struct KernelOpts
     {
         int tend, visc, tdma;
         int tend_kchunk, visc_kchunk;
     };
 
-    // Level-chunk height of a marching kernel with `tiles` blocks per chunk
-    // row: the requested height, or for 0 64 where that gives eight blocks
-    // per SM, else the largest of 32, 16, 8 that still gives two (small grids
-    // get more, shorter chunks).
-    int auto_kchunk(int requested, long long tiles, int ktot);
+    // Level-chunk height (at most `most`) of a marching kernel with `tiles`
+    // blocks per chunk of levels: the requested height, or for 0 the one that
+    // keeps the busiest SM least busy.  Halving 32 until the grid gave two
+    // blocks per SM left long marches on small grids and a nearly empty last
+    // wave on middle ones.  Tendencies in ms per step, old rule, this one, and the
+    // best of heights from 2 to 64: 32^3 0.050, 0.030, 0.030; 128 x 128 x 96 0.172,
+    // 0.171, 0.164; 150^3 0.379, 0.359, 0.339; 189 x 105 x 90 0.239, 0.234, 0.234;
+    // FP64 channel 256 x 192 x 128 3.38, 3.01, 3.00.
+    int auto_kchunk(int requested, long long tiles, int ktot, bool dbl, int most);
 
     // Read-only view of a context for kernels in other translation units.
     const Dims& ctx_dims(const mhh_ctx* c);

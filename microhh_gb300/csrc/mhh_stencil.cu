@@ -369,7 +369,7 @@ namespace mhh
         dim3 grid((d.itot + 31)/32, (d.jtot + 7)/8, d.ktot);
         // Automatic choice (-1): the plane-staged kernel in both precisions
         // (in double it keeps the reference's evisc expression).
-        const int var = o.visc < 0 ? 1 : o.visc;
+        const int var = d.ncells >= (1LL << 32) ? 0 : (o.visc < 0 ? 1 : o.visc);
         const bool planes = var == 1 && launch_viscosity_planes<TF>(d, pr, u, v, w, th, evisc, mlen2, dudz, dvdz, dbdz,
                                                                     tpr, surf, thermo, o.visc_kchunk, s);
         if (!planes)
@@ -512,7 +512,8 @@ namespace mhh
         // reference).
         // The limited scalar (adv == ADVEC_2I5_LIM) runs in the flux-form or
         // the per-cell kernel; the tiled kernel hands it to the flux form.
-        const int var = o.tend < 0 ? 2 : o.tend;
+        // The marching kernels index fields with 32 bits; larger grids run per cell.
+        const int var = d.ncells >= (1LL << 32) ? 0 : (o.tend < 0 ? 2 : o.tend);
         const bool lim = adv == ADVEC_2I5_LIM && scal;
         if (adv == ADVEC_2I5_LIM && !scal) adv = MHH_ADVEC_2I5;
         if (var >= 1 && (adv == MHH_ADVEC_2I5 || lim) && dif == MHH_DIFF_SMAG2 && !force && d.igc >= 3 && d.jgc >= 3)

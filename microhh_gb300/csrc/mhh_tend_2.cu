@@ -230,8 +230,9 @@ namespace mhh
     {
         constexpr size_t smem = tend2_smem<TF, SCAL>();
         const int nx = (d.itot + DTX - 1)/DTX, ny = (d.jtot + DTY - 1)/DTY;
-        kchunk = min(auto_kchunk(kchunk, (long long)nx*ny, d.ktot), DKCHUNK_MAX);
-        launch_body<Tend2P<TF>, tend2_body<TF, SCAL, BUOY>, DNT, (sizeof(TF) == 4 ? 3 : 2)>(
+        constexpr int occ = sizeof(TF) == 4 ? 3 : 2;
+        kchunk = auto_kchunk(kchunk, (long long)nx*ny, d.ktot, sizeof(TF) == 8, DKCHUNK_MAX);
+        launch_body<Tend2P<TF>, tend2_body<TF, SCAL, BUOY>, DNT, occ>(
             dim3(nx, ny, (d.ktot + kchunk - 1)/kchunk), dim3(DNT), smem, s, Tend2P<TF>{d, pr, a, kchunk});
         count_launch();
     }

@@ -532,8 +532,8 @@ namespace mhh
     static void launch_flux_t(const Dims& d, const Prof<TF>& pr, const TendArgs<TF>& a, int kchunk, cudaStream_t s)
     {
         const size_t smem = flux_smem<TF>();
-        kchunk = min(auto_kchunk(kchunk, (long long)((d.itot + FTX - 1)/FTX)*((d.jtot + FTY - 1)/FTY), d.ktot),
-                     FKCHUNK_MAX);
+        kchunk = auto_kchunk(kchunk, (long long)((d.itot + FTX - 1)/FTX)*((d.jtot + FTY - 1)/FTY), d.ktot,
+                             sizeof(TF) == 8, FKCHUNK_MAX);
         dim3 grid((d.itot + FTX - 1)/FTX, (d.jtot + FTY - 1)/FTY, (d.ktot + kchunk - 1)/kchunk);
         launch_body<TendFluxP<TF>, tend_flux_body<TF, SURF, SCAL, BUOY, LIM>, NTHR, FluxOcc<TF>::v>(
             grid, dim3(NTHR), smem, s, TendFluxP<TF>{d, pr, a, kchunk});

@@ -301,8 +301,7 @@ namespace mhh
                             double tpr, int kchunk, cudaStream_t s)
     {
         const size_t smem = visc_smem<TF>();
-        kchunk = min(auto_kchunk(kchunk, (long long)((d.itot + VTX - 1)/VTX)*((d.jtot + VTY - 1)/VTY), d.ktot),
-                     VKCHUNK_MAX);
+        kchunk = auto_kchunk(kchunk, (long long)((d.itot + VTX - 1)/VTX)*((d.jtot + VTY - 1)/VTY), d.ktot, sizeof(TF) == 8, VKCHUNK_MAX);
         dim3 grid((d.itot + VTX - 1)/VTX, (d.jtot + VTY - 1)/VTY, (d.ktot + kchunk - 1)/kchunk);
         // Three blocks per SM in float (64 registers).
         launch_body<ViscPlanesP<TF>, visc_planes_body<TF, SURF, THERMO>, VNT, (sizeof(TF) == 4 ? 3 : 1)>(grid, dim3(VNT), smem, s,
