@@ -144,15 +144,13 @@ int mhh_ctx_estimate_bytes(const mhh_grid_desc* desc, int precision, size_t* byt
    1 in FP64 contexts and for columns above about 8000 levels), -1 =
    automatic (0 for FP64 contexts, 3 for FP32 contexts; the default). */
 int mhh_set_option(const char* name, int value);
-/* "fft_pipeline": 1 (the default) runs the fixed-length FFTs as persistent
-   blocks that load their next tile while transforming the current one; 0
-   runs one tile per block.  Both give identical results.
-   "fft_column_pairs": complex sequence pairs per tile of the y FFT, 8 (the
-   default: 16 adjacent columns, 512 threads per block, float fields; 256
-   threads for the 512-point warp-synchronous schedule, one warp per pair)
-   or 4.  "pres_fuse": 1 (the default) computes the Poisson
-   right-hand side inside the forward x FFT and stores the inverse x FFT into
-   the ghost layout of p; 0 runs them as separate kernels. */
+/* "fft_pipeline": 0 or 1, without effect (the transforms have one schedule;
+   it chose between two that gave identical results).
+   "fft_column_pairs": complex sequence pairs per tile of the y FFT of float
+   fields at jtot = 32, 8 (the default) or 4.
+   "pres_fuse": 1 (the default) computes the Poisson right-hand side inside the
+   forward x FFT and stores the inverse x FFT into the ghost layout of p; 0
+   runs them as separate kernels. */
 /* "tendency_kchunk" / "viscosity_kchunk": levels per block of the marching
    kernels, 4, 8, 16, 32 or 64, or 0 (the default: at most 64, the height that
    keeps the busiest SM least busy). */

@@ -77,8 +77,6 @@ namespace mhh
     static int g_pres_fuse = 1;
     int pres_fuse() { return g_pres_fuse; }
     int fft_column_pairs() { return g_fft_col_pairs; }
-    static int g_fft_pipeline = 1;
-    int fft_pipeline() { return g_fft_pipeline; }
     void set_fft_column_pairs(int p) { g_fft_col_pairs = p; }
     static int g_tdma_variant = -1;
     int tdma_variant() { return g_tdma_variant; }
@@ -658,7 +656,6 @@ int mhh_set_option(const char* name, int value)
     if (!std::strcmp(name, "fft_pipeline"))
     {
         if (value != 0 && value != 1) return fail(MHH_ERR_ARG, "fft_pipeline is 0 or 1");
-        g_fft_pipeline = value;
         return MHH_OK;
     }
     if (!std::strcmp(name, "fft_column_pairs"))

@@ -127,8 +127,10 @@ namespace mhh
     struct FftPlan
     {
         int n;
-        int ngfac;        // radices (2 to 10) of the run-time plan
+        int ngfac;        // radices (2 to 10) of the double plan
         int gfac[16];
+        int nffac;        // stage codes of the float plan
+        int ffac[16];
         double* tw_d;     // exp(-2 pi i k/n), k < n, as (re, im) pairs (double)
         float* tw_f;      // the same in float
     };
@@ -178,9 +180,9 @@ namespace mhh
     // fields); -1 = automatic (0 for double fields, 3 for float fields).
     int tdma_variant();
     void set_tdma_variant(int v);
-    // Complex sequence pairs per block of the column (y) FFT: 4 or 8.
+    // Complex sequence pairs per block of the column (y) FFT with compile-time
+    // stages: 4 or 8.
     int fft_column_pairs();
-    int fft_pipeline();
     // 1 (default): the pressure right-hand side and the scatter into p are
     // fused into the x transforms; 0: separate kernels.
     int pres_fuse();

@@ -6,11 +6,10 @@
 //
 // FFT: two real sequences x, y of length n are transformed together as
 // z = x + i y with a mixed-radix Stockham autosort FFT in shared memory
-// (ping-pong buffers, one barrier per stage; compile-time stages for the common
-// lengths, run-time plans of radices 2 to 10 for the others), or for n = 128,
-// 256 and 512 with a warp-synchronous schedule (one warp per sequence), then
-// separated by Hermitian symmetry into FFTW's halfcomplex order r_0 ..
-// r_{n/2}, i_{(n+1)/2-1} .. i_1 (the convention of src/fft.cxx:145-206).
+// (ping-pong buffers, one barrier per stage; run-time plans of radices 2 to 12,
+// compile-time stages for n = 32 in float), then separated by Hermitian
+// symmetry into FFTW's halfcomplex order r_0 .. r_{n/2}, i_{(n+1)/2-1} .. i_1
+// (the convention of src/fft.cxx:145-206).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -35,6 +34,10 @@ namespace mhh
     }
     template<typename T2> __device__ __forceinline__ T2 cadd(T2 a, T2 b) { T2 r; r.x = a.x + b.x; r.y = a.y + b.y; return r; }
     template<typename T2> __device__ __forceinline__ T2 csub(T2 a, T2 b) { T2 r; r.x = a.x - b.x; r.y = a.y - b.y; return r; }
+
+    // Packed in float: one instruction per complex sum.
+    __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+    __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 
     template<typename TF> __device__ __forceinline__ const TF* twtab(const FftPlan& pl);
     template<> __device__ __forceinline__ const double* twtab<double>(const FftPlan& pl) { return pl.tw_d; }
@@ -61,9 +64,9 @@ namespace mhh
     }
 
     // ---- fixed-length transforms -----------------------------------------
-    // For the common lengths the radices are compile-time constants (8 first,
-    // then 4, 2, 3, 5), so all index arithmetic folds into shifts and
-    // multiplications and each stage is unrolled.
+    // The radices are compile-time constants (8 first, then 4, 2, 3, 5), so all
+    // index arithmetic folds into shifts and multiplications and each stage is
+    // unrolled.
     __host__ __device__ constexpr int fixed_radix(int n, int s)
     {
         int r = n;
@@ -97,7 +100,10 @@ namespace mhh
         T2 t7; t7.x = h*(a7.y - a7.x); t7.y = -h*(a7.x + a7.y);
         // Stage 2: radix-4 on (a0,a1,a2,a3) and (a4,t5,t6,t7)
         T2 b0 = cadd(a0, a2), b2 = csub(a0, a2), b1 = cadd(a1, a3), b3 = mul_mi<T2>(csub(a1, a3));
-        T2 c0 = cadd(a4, t6), c2 = csub(a4, t6), c1 = cadd(t5, t7), c3 = mul_mi<T2>(csub(t5, t7));
+        T2 c0 = cadd(a4, t6), c2 = csub(a4, t6), c1, c3;
+        // By component: the products of t5, t7 are contracted into these sums.
+        c1.x = t5.x + t7.x; c1.y = t5.y + t7.y;
+        c3.x = t5.y - t7.y; c3.y = -(t5.x - t7.x);
         u[0] = cadd(b0, b1); u[4] = csub(b0, b1);
         u[2] = cadd(b2, b3); u[6] = csub(b2, b3);
         u[1] = cadd(c0, c1); u[5] = csub(c0, c1);
@@ -147,15 +153,8 @@ namespace mhh
         }
     }
 
-    // Shared-memory position of complex element idx of a stage buffer: with
-    // SWZ one element of padding per 16, so that the strided writes of the
-    // first stages (element i*R + r of thread i) spread over all banks.
-    template<bool SWZ> __device__ __forceinline__ int swz(int idx) { return SWZ ? idx + (idx >> 4) : idx; }
-
-    // Stockham stages S.. of P sequences of length N, sequence q at
-    // src + q*SS (SS >= N: a padded stride keeps column stores free of bank
-    // conflicts).
-    template<typename TF, int N, int P, int S, int PACC, int SS = N, bool SWZ = false>
+    // Stockham stages S.. of P sequences of length N, sequence q at src + q*N.
+    template<typename TF, int N, int P, int S, int PACC>
     struct FixedStages
     {
         using T2 = typename C2<TF>::T;
@@ -170,25 +169,25 @@ namespace mhh
                 const int seq = it / T;
                 const int i = it - seq*T;
                 const int k = i % PACC;
-                const int xb = seq*SS + i;
-                const int j = seq*SS + (i - k)*R + k;
+                const int xb = seq*N + i;
+                const int j = seq*N + (i - k)*R + k;
                 T2 u[R];
-                u[0] = src[swz<SWZ>(xb)];
+                u[0] = src[xb];
                 #pragma unroll
                 for (int q=1; q<R; ++q)
-                    u[q] = (PACC == 1) ? src[swz<SWZ>(xb + q*T)] : cmul(src[swz<SWZ>(xb + q*T)], tws[(q*k*step) % N]);
+                    u[q] = (PACC == 1) ? src[xb + q*T] : cmul(src[xb + q*T], tws[(q*k*step) % N]);
                 radix_bfly<TF, N, R, T>(u, tws);
                 #pragma unroll
-                for (int r=0; r<R; ++r) dst[swz<SWZ>(j + r*PACC)] = u[r];
+                for (int r=0; r<R; ++r) dst[j + r*PACC] = u[r];
             }
             __syncthreads();
             T2* t = src; src = dst; dst = t;
-            FixedStages<TF, N, P, S+1, PACC*R, SS, SWZ>::run(src, dst, tws);
+            FixedStages<TF, N, P, S+1, PACC*R>::run(src, dst, tws);
         }
     };
 
-    template<typename TF, int N, int P, int S, int SS, bool SWZ>
-    struct FixedStages<TF, N, P, S, N, SS, SWZ>
+    template<typename TF, int N, int P, int S>
+    struct FixedStages<TF, N, P, S, N>
     {
         using T2 = typename C2<TF>::T;
         static __device__ __forceinline__ void run(T2*&, T2*&, const T2*) {}
@@ -247,7 +246,10 @@ namespace mhh
     __device__ __forceinline__ long long seq_base(const SeqLayout& L, long long s, int n)
     {
         if (L.rows) return s*(long long)n;
-        return (s / L.itot)*(long long)L.itot*n + (s % L.itot);
+        // 32-bit division where the sequence number allows (all but the largest
+        // grids): a 64-bit one takes longer than a small tile's load.
+        const long long k = L.nseq <= 0xffffffffLL ? (long long)((unsigned)s/(unsigned)L.itot) : s/L.itot;
+        return k*(long long)L.itot*n + (s - k*L.itot);
     }
 
     template<typename TF>
@@ -261,7 +263,8 @@ namespace mhh
             ti.sb[ls] = seq_base(L, s, n);
             if (fused)
             {
-                const int kr = (int)(s / fz.d.jtot), jr = (int)(s - (long long)kr*fz.d.jtot);
+                const int kr = (int)(L.nseq <= 0xffffffffLL ? (unsigned)s/(unsigned)fz.d.jtot : s/fz.d.jtot);
+                const int jr = (int)(s - (long long)kr*fz.d.jtot);
                 ti.sc[ls] = ijk(fz.d, fz.d.igc, jr + fz.d.jgc, kr + fz.d.kgc);
                 ti.sk[ls] = kr;
             }
@@ -286,159 +289,6 @@ namespace mhh
     // The float transform with the fused right-hand side keeps five blocks
     // per SM (at most 51 registers): its batched loads need the residency to
     // cover the latency of HBM.
-    // ---- warp-synchronous schedule for n = 64 R (R = 2, 4, 8) --------------
-    // For n = 128, 256 and 512 one warp transforms one complex sequence with
-    // a single block-wide dependency (its input tile): a decimation-in-
-    // frequency radix-R stage splits the sequence into R 64-point
-    // sub-sequences,
-    //   s_r[i] = wn^(i r) DFT_R,q(z[i + 64 q])[r],  X[R K + r] = DFT64(s_r)[K],
-    // and each 64-point transform runs as 8 x 8 within the warp:
-    //   A[t][k1] = w64^(t k1) DFT8_m(s_r[t + 8 m])[k1],
-    //   X_r[k1 + 8 k2] = DFT8_t(A[t][k1])[k2].
-    // The exchanges between the three passes go through the warp's own
-    // shared-memory region with __syncwarp (an 8 x 8 transpose among eight
-    // lanes is 16 shared accesses per lane; with __shfl_xor_sync it is 24
-    // shuffles and 48 selects), so a tile needs block barriers only after its
-    // load and before its store, against one per stage in the Stockham
-    // schedule.  The last pass writes its result over the warp's own real
-    // input, which no other warp reads.
-    //
-    // Positions within a sub-sequence block: rows of eight complex elements,
-    // row index XOR (r & 1) and column index XOR row, so that eight lanes
-    // reading a row or a column, and the sub-blocks a warp touches at once,
-    // spread over all banks.
-    __device__ __forceinline__ int warp_pos(int r, int row, int col)
-    {
-        return r*64 + ((row ^ (r & 1)) << 3) + (col ^ row);
-    }
-
-    // Twiddles of the schedule, n = 64 R entries in shared memory: wn^(i r)
-    // at (r-1)*64 + i for r = 1..R-1, i = 0..63, then w64^(t k1) = wn^(R t k1)
-    // at (R-1)*64 + k1*8 + t.
-    template<typename TF, int R>
-    __device__ __forceinline__ void warp_twiddles(typename C2<TF>::T* tw, const TF* __restrict__ twt)
-    {
-        using T2 = typename C2<TF>::T;
-        constexpr int N = 64*R, B = (R - 1)*64;
-        for (int e = threadIdx.x; e < N; e += blockDim.x)
-        {
-            const int idx = e < B ? ((e & 63)*((e >> 6) + 1)) % N : (R*(e & 7)*((e - B) >> 3)) % N;
-            T2 w; w.x = twt[2*idx]; w.y = twt[2*idx + 1];
-            tw[e] = w;
-        }
-    }
-
-    // Complex input element k of the pair (hx, hy): z = x + i y (forward) or
-    // the conjugated halfcomplex pair (inverse), as in the first Stockham
-    // stage.
-    template<typename TF, bool INV, int N>
-    __device__ __forceinline__ typename C2<TF>::T pair_in(const TF* __restrict__ hx, const TF* __restrict__ hy, int k)
-    {
-        typename C2<TF>::T u;
-        if (!INV)
-        {
-            u.x = hx[k]; u.y = hy[k];
-        }
-        else
-        {
-            const int kk = k <= N/2 ? k : N - k;
-            const bool real_only = (kk == 0) || (2*kk == N);
-            const TF sg = k <= N/2 ? TF(1) : TF(-1);
-            const int km = real_only ? kk : N - kk;
-            const TF xr = hx[kk], yr = hy[kk];
-            const TF xi = real_only ? TF(0) : sg*hx[km];
-            const TF yi = real_only ? TF(0) : sg*hy[km];
-            u.x = xr - yi;
-            u.y = -(xi + yr);
-        }
-        return u;
-    }
-
-    // Position of X[k] in the result of fft_warp: natural order, or with
-    // SWAP the sub-sequence index r = k mod R and the next octal digit k1
-    // exchanged (pass 3 then stores lane-consecutive elements; the column
-    // stores read pairs of adjacent k, which this order keeps in different
-    // banks).
-    template<int R, bool SWAP> __device__ __forceinline__ int warp_res(int k)
-    {
-        if (!SWAP) return k;
-        const int r = k % R, k1 = (k / R) & 7, k2 = k / (8*R);
-        return r*8 + k1 + 8*R*k2;
-    }
-
-    // The transform of complex sequence q (warp q; q < P) of a tile whose
-    // 2P real sequences sit at rin + s*ns.  work holds P regions of 64 R
-    // complex elements at stride ss.  On return (after __syncwarp) X[k] of
-    // sequence q is at element warp_res<R, SWAP>(k) of
-    // reinterpret_cast<T2*>(rin + 2q*ns).
-    template<typename TF, bool INV, bool SWAP, int R>
-    __device__ __forceinline__ void fft_warp(TF* rin, int ns, typename C2<TF>::T* work, int ss,
-                                             const typename C2<TF>::T* __restrict__ tw, int P)
-    {
-        using T2 = typename C2<TF>::T;
-        constexpr int N = 64*R, NPAIR = 8*R;
-        const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (q >= P) return;
-        const TF* hx = rin + (2*q)*ns;
-        const TF* hy = hx + ns;
-        T2* z = work + q*ss;
-        // Pass 1: radix R over stride 64, twiddles wn^(i r).
-        #pragma unroll
-        for (int h=0; h<2; ++h)
-        {
-            const int i = lane + 32*h;
-            T2 u[R];
-            #pragma unroll
-            for (int b=0; b<R; ++b) u[b] = pair_in<TF, INV, N>(hx, hy, i + 64*b);
-            radix_bfly<TF, N, R, 64>(u, tw);
-            #pragma unroll
-            for (int r=1; r<R; ++r) u[r] = cmul(u[r], tw[(r - 1)*64 + i]);
-            #pragma unroll
-            for (int r=0; r<R; ++r) z[warp_pos(r, i >> 3, i & 7)] = u[r];
-        }
-        __syncwarp();
-        // Pass 2: radix 8 over m within each sub-sequence, twiddles w64^(t k1),
-        // in place (a lane's writes are the elements it read).
-        #pragma unroll
-        for (int h=0; h<(NPAIR + 31)/32; ++h)
-        {
-            const int pp = lane + 32*h, r = pp >> 3, t = pp & 7;
-            if (pp < NPAIR)
-            {
-                T2 a[8];
-                #pragma unroll
-                for (int m=0; m<8; ++m) a[m] = z[warp_pos(r, m, t)];
-                dft8<TF, T2>(a);
-                #pragma unroll
-                for (int k1=1; k1<8; ++k1) a[k1] = cmul(a[k1], tw[(R - 1)*64 + k1*8 + t]);
-                #pragma unroll
-                for (int k1=0; k1<8; ++k1) z[warp_pos(r, k1, t)] = a[k1];
-            }
-        }
-        __syncwarp();
-        // Pass 3: radix 8 over t; X[r + R k1 + 8 R k2] at warp_res over the
-        // warp's real input (read only by this warp, in pass 1).
-        T2* out = reinterpret_cast<T2*>(rin + (2*q)*ns);
-        #pragma unroll
-        for (int h=0; h<(NPAIR + 31)/32; ++h)
-        {
-            const int pp = lane + 32*h, r = pp >> 3, k1 = pp & 7;
-            if (pp < NPAIR)
-            {
-                T2 a[8];
-                #pragma unroll
-                for (int t=0; t<8; ++t) a[t] = z[warp_pos(r, k1, t)];
-                dft8<TF, T2>(a);
-                #pragma unroll
-                for (int k2=0; k2<8; ++k2) out[SWAP ? pp + 8*R*k2 : r + R*k1 + 8*R*k2] = a[k2];
-            }
-        }
-        __syncwarp();
-    }
-
-    // Lengths that run the warp-synchronous schedule.
-    __host__ __device__ constexpr bool warp_len(int n) { return n == 128 || n == 256 || n == 512; }
-
     template<typename TF> struct FftP { FftPlan pl; TF* data; SeqLayout L; TF scale; FftFuse<TF> fz; };
     template<typename TF, int FUSE> struct FftOcc { static constexpr int v = (FUSE == 1 && sizeof(TF) == 4) ? 5 : 1; };
 
@@ -464,14 +314,9 @@ namespace mhh
         const long long s0 = (long long)vb.x*2*P;
         const int nloc = (int)min((long long)2*P, L.nseq - s0);
 
-        constexpr bool WARP = warp_len(NFIX);
-        if constexpr (WARP) warp_twiddles<TF, NFIX/64>(tws, twtab<TF>(pl));
-        else
-        {
-            const TF* tt = twtab<TF>(pl);
-            for (int e = threadIdx.x; e < n; e += blockDim.x)
-            { T2 w; w.x = tt[2*e]; w.y = tt[2*e+1]; tws[e] = w; }
-        }
+        const TF* tt = twtab<TF>(pl);
+        for (int e = threadIdx.x; e < n; e += blockDim.x)
+        { T2 w; w.x = tt[2*e]; w.y = tt[2*e+1]; tws[e] = w; }
 
         // 1. Load 2P real sequences into buf1 viewed as real [2P][n], with
         //    asynchronous copies so that all of a thread's loads are in
@@ -571,19 +416,6 @@ namespace mhh
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
 
-        // 2-3. With n = 128, 256 or 512 the warp-synchronous schedule, whose
-        //      result is the natural order over each sequence pair's real
-        //      input.
-        T2* res;
-        T2* other;
-        if constexpr (WARP)
-        {
-            fft_warp<TF, INV, false, NFIX/64>(r1, ns, buf0, n, tws, P);
-            __syncthreads();
-            res = nullptr; other = buf0;
-        }
-        else
-        {
         // 2. Complex input: z = x + i y (forward) or conj(X + i Y) (inverse).
         for (int e = threadIdx.x; e < P*n; e += blockDim.x)
         {
@@ -611,11 +443,9 @@ namespace mhh
         __syncthreads();
 
         // 3. FFT.
-        T2* src = buf0;
-        T2* dst = buf1;
-        FixedStages<TF, NFIX, PFIX, 0, 1>::run(src, dst, tws);
-        res = src; other = dst;
-        }
+        T2* res = buf0;
+        T2* other = buf1;
+        FixedStages<TF, NFIX, PFIX, 0, 1>::run(res, other, tws);
         TF* rout = reinterpret_cast<TF*>(other);
 
         // 4. Real outputs into the other buffer, [2P][n].
@@ -624,7 +454,7 @@ namespace mhh
             const int q = e / n, k = e - q*n;
             TF* ox = rout + (2*q)*ns;
             TF* oy = rout + (2*q+1)*ns;
-            const T2* rq = WARP ? reinterpret_cast<const T2*>(r1 + (2*q)*ns) : res + q*n;
+            const T2* rq = res + q*n;
             if (!INV)
             {
                 if (k <= n/2)
@@ -690,281 +520,6 @@ namespace mhh
         }
     }
 
-    // ---- pipelined fixed-length transforms ----------------------------------
-    // A persistent block loops over tiles of 2P real sequences.  While it
-    // transforms tile t, the asynchronous copies of its next tile are already
-    // in flight into a second input buffer, so the loads of HBM overlap the
-    // shared-memory work of the stages (one tile per block left the memory
-    // system idle between a block's load and its store).  The packing of two
-    // real sequences into one complex one is folded into the first stage and
-    // the separation into halfcomplex order into the store.
-    //
-    // Shared memory: two input buffers and one work buffer of P*SS + P
-    // complex elements, plus the twiddle table.  Tile t's input buffer also
-    // serves as the second stage buffer; the other input buffer receives
-    // tile t + (the number of blocks).
-
-    // Complex elements of one buffer of the pipelined kernel: P sequences at
-    // stride SS (N for rows, N + 4 for columns) with the swizzle padding, and
-    // at least the real input view of 2P sequences at stride NS.
-    __host__ __device__ constexpr int fftp_buf(int N, int P, bool rows)
-    {
-        return (P*(rows ? N : N + 4)*17)/16 + 16 + P;
-    }
-
-    // First Stockham stage (radix R0, no twiddles) with the complex input
-    // formed from the real sequences: z = x + i y (forward) or the
-    // conjugated halfcomplex pair (inverse).  Real sequence s sits at
-    // r + s*NS.
-    template<typename TF, bool INV, int N, int P, int NS, int SS, bool SWZ>
-    __device__ __forceinline__ void fft_first_stage(const TF* __restrict__ r, typename C2<TF>::T* __restrict__ y,
-                                                    const typename C2<TF>::T* __restrict__ tws)
-    {
-        using T2 = typename C2<TF>::T;
-        constexpr int R = fixed_radix(N, 0);
-        constexpr int T = N / R;
-        for (int it = threadIdx.x; it < P*T; it += blockDim.x)
-        {
-            const int seq = it / T, i = it - seq*T;
-            const TF* hx = r + (2*seq)*NS;
-            const TF* hy = hx + NS;
-            T2 u[R];
-            #pragma unroll
-            for (int q=0; q<R; ++q)
-            {
-                const int k = i + q*T;
-                if (!INV)
-                {
-                    u[q].x = hx[k]; u[q].y = hy[k];
-                }
-                else
-                {
-                    const int kk = k <= N/2 ? k : N - k;
-                    const bool real_only = (kk == 0) || (2*kk == N);
-                    const TF sg = k <= N/2 ? TF(1) : TF(-1);
-                    const int km = real_only ? kk : N - kk;
-                    const TF xr = hx[kk], yr = hy[kk];
-                    const TF xi = real_only ? TF(0) : sg*hx[km];
-                    const TF yi = real_only ? TF(0) : sg*hy[km];
-                    u[q].x = xr - yi;
-                    u[q].y = -(xi + yr);
-                }
-            }
-            radix_bfly<TF, N, R, T>(u, tws);
-            const int yb = seq*SS + i*R;
-            #pragma unroll
-            for (int q=0; q<R; ++q) y[swz<SWZ>(yb + q)] = u[q];
-        }
-        __syncthreads();
-    }
-
-    // Real output k of real sequence ls of a tile from the transformed pairs:
-    // halfcomplex separation (forward) or real/imaginary parts (inverse).
-    template<typename TF, bool INV, int N, int SS, bool SWZ>
-    __device__ __forceinline__ TF fft_real_out(const typename C2<TF>::T* __restrict__ res, int ls, int k, TF scale)
-    {
-        using T2 = typename C2<TF>::T;
-        const int qb = (ls >> 1)*SS;
-        const bool yseq = ls & 1;
-        if (INV)
-        {
-            const T2 a = res[swz<SWZ>(qb + k)];
-            return yseq ? -a.y*scale : a.x*scale;
-        }
-        const int kk = k <= N/2 ? k : N - k;
-        const T2 a = res[swz<SWZ>(qb + kk)], b = res[swz<SWZ>(qb + (kk == 0 ? 0 : N - kk))];
-        if (k <= N/2) return yseq ? TF(0.5)*(a.y + b.y) : TF(0.5)*(a.x + b.x);
-        return yseq ? TF(-0.5)*(a.x - b.x) : TF(0.5)*(a.y - b.y);
-    }
-
-    // The same from the result rq of the pair from fft_warp (yseq: the
-    // pair's second real sequence).
-    template<typename TF, bool INV, int N, bool SWAP>
-    __device__ __forceinline__ TF fft_real_nat(const typename C2<TF>::T* __restrict__ rq, int yseq, int k, TF scale)
-    {
-        using T2 = typename C2<TF>::T;
-        if (INV)
-        {
-            const T2 a = rq[warp_res<N/64, SWAP>(k)];
-            return yseq ? -a.y*scale : a.x*scale;
-        }
-        const int kk = k <= N/2 ? k : N - k;
-        const T2 a = rq[warp_res<N/64, SWAP>(kk)], b = rq[warp_res<N/64, SWAP>(kk == 0 ? 0 : N - kk)];
-        if (k <= N/2) return yseq ? TF(0.5)*(a.y + b.y) : TF(0.5)*(a.x + b.x);
-        return yseq ? TF(-0.5)*(a.x - b.x) : TF(0.5)*(a.y - b.y);
-    }
-
-    template<typename TF> struct FftpP { TF* data; SeqLayout L; TF scale; FftFuse<TF> fz; const TF* twt; long long ntiles; };
-
-    template<typename TF, bool INV, int N, int P, int FUSE, bool ROWS>
-    __device__ __forceinline__ void fftp_body(const FftpP<TF>& A, const VBlock& vb)
-    {
-        TF* __restrict__ data = A.data;
-        const SeqLayout& L = A.L;
-        const TF scale = A.scale;
-        const FftFuse<TF>& fz = A.fz;
-        const TF* __restrict__ twt = A.twt;
-        const long long ntiles = A.ntiles;
-        using T2 = typename C2<TF>::T;
-        constexpr int NS = ROWS ? N : N + 1;      // real stride of the input view
-        constexpr int SS = ROWS ? N : N + 4;      // complex stride of the stages
-        constexpr int BUF = fftp_buf(N, P, ROWS);
-        extern __shared__ __align__(16) unsigned char smem_raw[];
-        T2* bufs = reinterpret_cast<T2*>(smem_raw);
-        T2* work = bufs + BUF;
-        T2* tws = bufs + 3*BUF;
-        constexpr bool WARP = warp_len(N);
-        if constexpr (WARP) warp_twiddles<TF, N/64>(tws, twt);
-        else
-            for (int e = threadIdx.x; e < N; e += blockDim.x)
-            { T2 w; w.x = twt[2*e]; w.y = twt[2*e+1]; tws[e] = w; }
-
-        // Asynchronous copies of tile t into input buffer b (a missing
-        // sequence reads as zero).  Each thread computes the base of the
-        // sequence it copies once per tile.
-        auto issue = [&](long long t, T2* b)
-        {
-            TF* r = reinterpret_cast<TF*>(b);
-            const long long s0 = t*2*P;
-            const int nloc = (int)min((long long)2*P, L.nseq - s0);
-            if (ROWS)
-            {
-                for (int e = threadIdx.x; e < 2*P*N; e += blockDim.x)
-                {
-                    const int ls = e / N, j = e - ls*N;
-                    const bool ok = ls < nloc;
-                    fft_cp_async(r + ls*NS + j, ok ? data + (s0 + ls)*(long long)N + j : data, ok);
-                }
-            }
-            else
-            {
-                const int ls = threadIdx.x % (2*P);
-                const bool ok = ls < nloc;
-                const long long st = (long long)(blockDim.x/(2*P))*L.itot;
-                const TF* sp = data + (ok ? seq_base(L, s0 + ls, N) : 0) + (long long)(threadIdx.x/(2*P))*L.itot;
-                for (int j = threadIdx.x/(2*P); j < N; j += blockDim.x/(2*P), sp += st)
-                    fft_cp_async(r + ls*NS + j, ok ? sp : data, ok);
-            }
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-        };
-        // Ghost-layout offsets of the current tile's rows (FUSE == 2),
-        // written after the barrier that ends the previous tile and read
-        // after the barriers of the stages.
-        __shared__ TileIdx x;
-
-        long long t = vb.x;
-        int cur = 0;
-        if (t < ntiles) issue(t, bufs);
-        for (; t < ntiles; t += vb.gx)
-        {
-            T2* in = cur ? bufs + 2*BUF : bufs;
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-            __syncthreads();
-            // The other input buffer was last read by the previous tile,
-            // which every thread has finished (barrier above).
-            if (t + vb.gx < ntiles) issue(t + vb.gx, cur ? bufs : bufs + 2*BUF);
-            if (FUSE == 2)
-            {
-                const long long s0 = t*2*P;
-                tile_index<TF>(x, L, fz, s0, (int)min((long long)2*P, L.nseq - s0), N, true);
-            }
-
-            const T2* res = work;
-            TF* inr = reinterpret_cast<TF*>(in);
-            if constexpr (WARP)
-            {
-                fft_warp<TF, INV, !ROWS, N/64>(inr, NS, work, SS, tws, P);
-                __syncthreads();
-            }
-            else
-            {
-                // The swizzle pays off for rows; the padded column stride
-                // already spreads the column stores.
-                fft_first_stage<TF, INV, N, P, NS, SS, ROWS>(inr, work, tws);
-                T2* src = work;
-                T2* dst = in;
-                FixedStages<TF, N, P, 1, fixed_radix(N, 0), SS, ROWS>::run(src, dst, tws);
-                res = src;
-            }
-            // Real output k of real sequence ls of the tile.
-            auto out_at = [&](int ls, int k) -> TF
-            {
-                if constexpr (WARP)
-                    return fft_real_nat<TF, INV, N, !ROWS>(reinterpret_cast<const T2*>(inr + (ls & ~1)*NS), ls & 1, k, scale);
-                else
-                    return fft_real_out<TF, INV, N, SS, ROWS>(res, ls, k, scale);
-            };
-
-            const long long s0 = t*2*P;
-            const int nloc = (int)min((long long)2*P, L.nseq - s0);
-            if (FUSE == 2)
-            {
-                // Straight into the ghost layout of p, with the bottom ghost
-                // level p[kstart-1] = p[kstart] (src/pres_2.cxx:330-358).
-                for (int e = threadIdx.x; e < 2*P*N; e += blockDim.x)
-                {
-                    const int ls = e / N, i = e - ls*N;
-                    if (ls < nloc)
-                    {
-                        TF val = out_at(ls, i);
-                        if (fz.dcm) val = add_rn(val, fz.dcm[x.sk[ls]]);
-                        const long long c = x.sc[ls] + i;
-                        fz.p[c] = val;
-                        if (x.sk[ls] == 0) fz.p[c - fz.d.ijcells] = val;
-                    }
-                }
-            }
-            else if (ROWS)
-            {
-                for (int e = threadIdx.x; e < 2*P*N; e += blockDim.x)
-                {
-                    const int ls = e / N, j = e - ls*N;
-                    if (ls < nloc) data[(s0 + ls)*(long long)N + j] = out_at(ls, j);
-                }
-            }
-            else
-            {
-                const int ls = threadIdx.x % (2*P);
-                if (ls < nloc)
-                {
-                    const long long st = (long long)(blockDim.x/(2*P))*L.itot;
-                    TF* dp = data + seq_base(L, s0 + ls, N) + (long long)(threadIdx.x/(2*P))*L.itot;
-                    for (int j = threadIdx.x/(2*P); j < N; j += blockDim.x/(2*P), dp += st)
-                        *dp = out_at(ls, j);
-                }
-            }
-            cur ^= 1;
-        }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    }
-
-    template<typename TF, bool INV, int N, int P, int FUSE, bool ROWS>
-    static void launch_fftp(const FftPlan& pl, TF* data, SeqLayout L, TF scale, const FftFuse<TF>& fz, cudaStream_t s)
-    {
-        using T2 = typename C2<TF>::T;
-        // 8 pairs (16 columns, 64-byte rows of a tile) run with 512 threads;
-        // the warp-synchronous schedule with one warp per pair.
-        constexpr int NT = warp_len(N) ? 32*P : (P == 8 ? 512 : 256);
-        const size_t smem = sizeof(T2)*((size_t)3*fftp_buf(N, P, ROWS) + N);
-        const long long ntiles = (L.nseq + 2*P - 1) / (2*P);
-        // Attribute and residency are set once per kernel, outside any stream
-        // capture that a later call may be part of.
-        using B = FftpP<TF>;
-        constexpr auto body = fftp_body<TF, INV, N, P, FUSE, ROWS>;
-        static const int resident = [&]
-        {
-            set_smem_limit<B, body, NT, 1>(smem);
-            int per_sm = 0, dev = 0, sms = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_one<B, body, NT, 1>, NT, smem);
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            return (per_sm > 0 ? per_sm : 1)*(sms > 0 ? sms : 1);
-        }();
-        const long long nblk = ntiles < resident ? ntiles : resident;
-        const TF* twt = sizeof(TF) == 8 ? reinterpret_cast<const TF*>(pl.tw_d) : reinterpret_cast<const TF*>(pl.tw_f);
-        launch_body<B, body, NT, 1>(dim3((unsigned)nblk), dim3(NT), smem, s, B{data, L, scale, fz, twt, ntiles});
-    }
-
     template<typename TF, bool INV, int NF, int PF, int FUSE>
     static void launch_fixed(const FftPlan& pl, TF* data, SeqLayout L, TF scale, const FftFuse<TF>& fz, cudaStream_t s)
     {
@@ -979,44 +534,27 @@ namespace mhh
     {
         if (pl.n != NF) return false;
         // Rows: 4 pairs per block; columns: 4 or 8 (float) pairs per block.
-        constexpr int PR = (2*sizeof(typename C2<TF>::T)*4*NF <= 96*1024) ? 4 : 1;
-        constexpr int PC = (sizeof(TF) == 4 && 2*sizeof(typename C2<TF>::T)*8*NF <= 96*1024) ? 8 : PR;
-        // Pipelined transforms (three buffers) where they fit in 96 KB.
-        constexpr bool PIPE_R = sizeof(typename C2<TF>::T)*(3*fftp_buf(NF, PR, true) + NF) <= 96*1024;
-        constexpr bool PIPE_C = sizeof(typename C2<TF>::T)*(3*fftp_buf(NF, PR, false) + NF) <= 96*1024;
-        constexpr bool PIPE_C8 = sizeof(TF) == 4 && sizeof(typename C2<TF>::T)*(3*fftp_buf(NF, 8, false) + NF) <= 200*1024;
-        const bool pipe = fft_pipeline() != 0;
+        constexpr int PR = 4, PC = sizeof(TF) == 4 ? 8 : 4;
         if (L.rows)
         {
             if constexpr (!INV) { if (fz.mode == 1) { launch_fixed<TF, INV, NF, PR, 1>(pl, data, L, scale, fz, s); return true; } }
-            else
-            {
-                if (fz.mode == 2)
-                {
-                    if (PIPE_R && pipe) launch_fftp<TF, INV, NF, PR, 2, true>(pl, data, L, scale, fz, s);
-                    else launch_fixed<TF, INV, NF, PR, 2>(pl, data, L, scale, fz, s);
-                    return true;
-                }
-            }
-            if (PIPE_R && pipe) launch_fftp<TF, INV, NF, PR, 0, true>(pl, data, L, scale, fz, s);
-            else launch_fixed<TF, INV, NF, PR, 0>(pl, data, L, scale, fz, s);
+            else { if (fz.mode == 2) { launch_fixed<TF, INV, NF, PR, 2>(pl, data, L, scale, fz, s); return true; } }
+            launch_fixed<TF, INV, NF, PR, 0>(pl, data, L, scale, fz, s);
         }
-        else if (PIPE_C8 && pipe && fft_column_pairs() == 8) launch_fftp<TF, INV, NF, 8, 0, false>(pl, data, L, scale, fz, s);
-        else if (PIPE_C && pipe) launch_fftp<TF, INV, NF, PR, 0, false>(pl, data, L, scale, fz, s);
         else if (fft_column_pairs() == 4 || PC == PR) launch_fixed<TF, INV, NF, PR, 0>(pl, data, L, scale, fz, s);
         else launch_fixed<TF, INV, NF, PC, 0>(pl, data, L, scale, fz, s);
         return true;
     }
 
+    // The length with compile-time stages: 32 in float, whose launches are bound
+    // by latency and instruction fetches (32^3: 0.088 ms of transforms per step
+    // against 0.099 with the run-time plan).  At 16 and from 48 on the run-time
+    // plan is as fast or faster, in double at every length.
     template<typename TF, bool INV>
     static bool launch_fixed_any(const FftPlan& pl, TF* data, SeqLayout L, TF scale, const FftFuse<TF>& fz, cudaStream_t s)
     {
-        return try_fixed_n<TF, INV, 512>(pl, data, L, scale, fz, s) || try_fixed_n<TF, INV, 256>(pl, data, L, scale, fz, s)
-            || try_fixed_n<TF, INV, 128>(pl, data, L, scale, fz, s) || try_fixed_n<TF, INV, 64>(pl, data, L, scale, fz, s)
-            || try_fixed_n<TF, INV, 32>(pl, data, L, scale, fz, s) || try_fixed_n<TF, INV, 1024>(pl, data, L, scale, fz, s)
-            || try_fixed_n<TF, INV, 192>(pl, data, L, scale, fz, s) || try_fixed_n<TF, INV, 96>(pl, data, L, scale, fz, s)
-            || try_fixed_n<TF, INV, 48>(pl, data, L, scale, fz, s) || try_fixed_n<TF, INV, 384>(pl, data, L, scale, fz, s)
-            || try_fixed_n<TF, INV, 768>(pl, data, L, scale, fz, s) || try_fixed_n<TF, INV, 16>(pl, data, L, scale, fz, s);
+        if constexpr (sizeof(TF) == 4) return try_fixed_n<TF, INV, 32>(pl, data, L, scale, fz, s);
+        else return false;
     }
 
     // ---- run-time plans -----------------------------------------------------
@@ -1025,14 +563,18 @@ namespace mhh
     // pair q at j*S + q: consecutive threads take the pairs of one element, so
     // the index of a butterfly is a shift, its twiddles are broadcasts, and for
     // columns (y) the pair of adjacent real columns is the complex element as it
-    // lies in memory.  Stages of radix 2 to 10 (as few as the length allows) run
+    // lies in memory.  Stages of radix 2 to 12 (as few as the length allows) run
     // in registers between two buffers, one barrier each; the first forms the
-    // complex input and the store separates the result.  The schedule it
-    // replaces ran radices 2 to 7 with separate packing and separation passes,
-    // global twiddle loads and two integer divisions per element: x and y
-    // transforms per step at 150^3 0.80 -> 0.30 ms in float, 189 x 105 x 90
-    // 0.45 -> 0.20 (what bounds it now is shared-memory latency with a barrier
-    // per stage).
+    // complex input and the store separates the result.  Small tiles, several
+    // blocks per SM: what bounds a transform is the latency of its loads and
+    // shared-memory stages in float, the FP64 pipe in double.  Transforms in ms
+    // per step (x, y), before: one stage per factor with packing and separation
+    // passes and two integer divisions per element at 150^3 0.395, 0.313, now
+    // 0.193, 0.124; 189 x 105 x 90 0.204, 0.190, now 0.101, 0.104; compile-time
+    // stages at 192 (channel 256 x 192 x 128) y 0.181, now 0.156, FP64 1.21, now
+    // 1.06; a warp-synchronous schedule at 512 x 512 x 256 2.17, 1.32, now 1.80,
+    // 1.31, 256 x 256 x 128 0.333, 0.186, now 0.311, 0.183.  256 threads a block:
+    // -3 % at 512, +2 to +15 % at other lengths.
     constexpr int FG_NT = 128;
     constexpr int FG_SMEM = 200*1024;
 
@@ -1164,13 +706,29 @@ namespace mhh
         TF* data; SeqLayout L; TF scale; FftFuse<TF> fz; const TF* twt;
         int n, lp, nst;
         int pairs;              // columns: the pairs of a tile are adjacent in memory
-        unsigned long long fac; // radices, four bits each, first stage lowest
+        unsigned long long fac; // the stages' codes, eight bits each, first stage lowest
     };
+
+    // Complex input element e of a pair: as it lies (forward) or the conjugated
+    // halfcomplex pair (inverse).
+    template<bool INV, typename T2>
+    __device__ __forceinline__ T2 fg_in(const T2* __restrict__ src, int e, int n, int S, int q)
+    {
+        if (!INV) return src[e*S + q];
+        const int kk = 2*e <= n ? e : n - e;
+        const bool real_only = kk == 0 || 2*kk == n;
+        const T2 a = src[kk*S + q], b = src[(real_only ? kk : n - kk)*S + q];
+        using TF = std::remove_cv_t<decltype(T2::x)>;
+        const TF sg = real_only ? TF(0) : (2*e <= n ? TF(1) : TF(-1));
+        T2 u;
+        u.x = a.x - sg*b.y;
+        u.y = -(sg*b.x + a.y);
+        return u;
+    }
 
     // One Stockham stage of radix R (p = the product of the radices before):
     // item (i, q), k = i mod p, reads src[i + r T] times w^(r k step) and writes
-    // dst[(i - k) R + k + r p].  FIRST: p = 1, no twiddles; with INV the input
-    // is the conjugated halfcomplex pair.
+    // dst[(i - k) R + k + r p].  FIRST: p = 1, no twiddles.
     template<typename TF, int R, bool FIRST, bool INV>
     __device__ __forceinline__ void fg_stage(const typename C2<TF>::T* __restrict__ src, typename C2<TF>::T* __restrict__ dst,
                                              const typename C2<TF>::T* __restrict__ tw, int n, int p, int S, int lp)
@@ -1188,17 +746,8 @@ namespace mhh
             for (int r=0; r<R; ++r)
             {
                 const int e = i + r*T;
-                if (FIRST && INV)
-                {
-                    const int kk = 2*e <= n ? e : n - e;
-                    const bool real_only = kk == 0 || 2*kk == n;
-                    const T2 a = src[kk*S + q], b = src[(real_only ? kk : n - kk)*S + q];
-                    const TF sg = real_only ? TF(0) : (2*e <= n ? TF(1) : TF(-1));
-                    u[r].x = a.x - sg*b.y;
-                    u[r].y = -(sg*b.x + a.y);
-                }
-                else
-                    u[r] = (FIRST || r == 0) ? src[e*S + q] : cmul(src[e*S + q], tw[r*k*step]);
+                if (FIRST) u[r] = fg_in<INV>(src, e, n, S, q);
+                else u[r] = r == 0 ? src[e*S + q] : cmul(src[e*S + q], tw[r*k*step]);
             }
             gdft<TF, R>(u);
             T2* y = dst + ((i - k)*R + k)*S + q;
@@ -1207,22 +756,150 @@ namespace mhh
         }
     }
 
+    // ---- the float plan ------------------------------------------------------
+    // In float a transform's rounding shows in every field, so the operations of
+    // a length are fixed by its list of elementary radices (plan_floats) and do
+    // not depend on how its stages are grouped: two elementary stages RA, RB run
+    // in registers as one, with the twiddles of both as if each had been stored.
+    //   one stage:  as fg_stage with R = RA;
+    //   two:        x[i + r T + q RB T] over q in radix RA (r < RB, twiddles
+    //               w^(q k RB step)), then over r in radix RB (m < RA, twiddles
+    //               w^(r (k + m p) step)), stored at (i - k) R + k + (m + RA r) p;
+    //   RB = 0:     decimation in frequency, the twiddles w^(r (i - k)) on the
+    //               results (lengths 128, 256 and 512).
+    // Radices 5 and 7 by the direct sum, 8 by dft8.  Sums two at a time in packed
+    // instructions, the same roundings: 512 x 512 x 256 x 1.95 ms, now 1.80;
+    // 150^3 0.213, 0.138 (x, y), now 0.193, 0.124.
+    // The product with its roundings spelled out, so that the sign folded into
+    // an operand cannot change which product is contracted.
+    __device__ __forceinline__ float2 fe_mul(float2 a, float2 b)
+    {
+        return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y)));
+    }
+
+    template<int R>
+    __device__ __forceinline__ void fe_dft(float2* u, const float2* __restrict__ tw, int n)
+    {
+        if constexpr (R == 2) gdft2(u);
+        else if constexpr (R == 3) gdft3<float>(u[0], u[1], u[2]);
+        else if constexpr (R == 4) gdft4(u[0], u[1], u[2], u[3]);
+        else if constexpr (R == 8) dft8<float, float2>(u);
+        else
+        {
+            // Packed: (x, y) of u_q w = (u.x, u.y) (w.x, w.x) + (u.y, u.x) (-w.y, w.y).
+            float2 wx[R], wy[R], v[R];
+            #pragma unroll
+            for (int m=0; m<R; ++m)
+            {
+                const float2 w = tw[m*(n/R)];
+                wx[m] = make_float2(w.x, w.x);
+                wy[m] = make_float2(-w.y, w.y);
+            }
+            #pragma unroll
+            for (int r=0; r<R; ++r) v[r] = u[0];
+            #pragma unroll
+            for (int q=1; q<R; ++q)
+            {
+                const float2 t = make_float2(u[q].y, u[q].x);
+                #pragma unroll
+                for (int r=0; r<R; ++r)
+                    v[r] = __fadd2_rn(v[r], __ffma2_rn(u[q], wx[(q*r) % R], __fmul2_rn(t, wy[(q*r) % R])));
+            }
+            #pragma unroll
+            for (int r=0; r<R; ++r) u[r] = v[r];
+        }
+    }
+
+    template<int RA, int RB, bool FIRST, bool INV>
+    __device__ __forceinline__ void fe_stage(const float2* __restrict__ src, float2* __restrict__ dst,
+                                             const float2* __restrict__ tw, int n, int p, int S, int lp)
+    {
+        constexpr bool DIF = RB == 0;
+        constexpr int B = RB > 1 ? RB : 1, R = RA*B;
+        const int T = n/R, step = T/p;
+        const float rp = 1.f/(float)p;
+        const int q = threadIdx.x & ((1 << lp) - 1);
+        for (int i = threadIdx.x >> lp; i < T; i += FG_NT >> lp)
+        {
+            int k = 0;
+            if (!FIRST) div_rcp(i, p, rp, k);
+            float2 u[B][RA];
+            #pragma unroll
+            for (int r=0; r<B; ++r)
+            {
+                #pragma unroll
+                for (int a=0; a<RA; ++a)
+                {
+                    const int e = i + (r + a*B)*T;
+                    if (FIRST) u[r][a] = fg_in<INV>(src, e, n, S, q);
+                    else u[r][a] = DIF || a == 0 ? src[e*S + q] : fe_mul(src[e*S + q], tw[a*k*B*step]);
+                }
+                fe_dft<RA>(u[r], tw, n);
+            }
+            float2* y = dst + ((i - k)*R + k)*S + q;
+            if (DIF)
+            {
+                if (p != T)
+                {
+                    #pragma unroll
+                    for (int a=1; a<RA; ++a) u[0][a] = fe_mul(u[0][a], tw[a*(i - k)]);
+                }
+                #pragma unroll
+                for (int a=0; a<RA; ++a) y[a*p*S] = u[0][a];
+            }
+            else
+            {
+                #pragma unroll
+                for (int m=0; m<RA; ++m)
+                {
+                    float2 v[B];
+                    v[0] = u[0][m];
+                    #pragma unroll
+                    for (int r=1; r<B; ++r) v[r] = FIRST && m == 0 ? u[r][m] : fe_mul(u[r][m], tw[r*(k + m*p)*step]);
+                    if constexpr (B > 1) fe_dft<B>(v, tw, n);
+                    #pragma unroll
+                    for (int r=0; r<B; ++r) y[(m + RA*r)*p*S] = v[r];
+                }
+            }
+        }
+    }
+
+    // A stage of the plan: code R in double, RA + 16 RB in float.
     template<typename TF, bool FIRST, bool INV>
-    __device__ __forceinline__ void fg_any(int R, const typename C2<TF>::T* src, typename C2<TF>::T* dst,
+    __device__ __forceinline__ void fg_any(int code, const typename C2<TF>::T* src, typename C2<TF>::T* dst,
                                            const typename C2<TF>::T* tw, int n, int p, int S, int lp)
     {
-        switch (R)
-        {
-            case 2: fg_stage<TF, 2, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-            case 3: fg_stage<TF, 3, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-            case 4: fg_stage<TF, 4, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-            case 5: fg_stage<TF, 5, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-            case 6: fg_stage<TF, 6, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-            case 7: fg_stage<TF, 7, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-            case 8: fg_stage<TF, 8, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-            case 9: fg_stage<TF, 9, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-            default: fg_stage<TF, 10, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
-        }
+        if constexpr (sizeof(TF) == 8)
+            switch (code)
+            {
+                case 2: fg_stage<TF, 2, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 3: fg_stage<TF, 3, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 4: fg_stage<TF, 4, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 5: fg_stage<TF, 5, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 6: fg_stage<TF, 6, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 7: fg_stage<TF, 7, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 8: fg_stage<TF, 8, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 9: fg_stage<TF, 9, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                default: fg_stage<TF, 10, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            }
+        else
+            switch (code)
+            {
+                case 0x02: if (FIRST) fe_stage<2, 0, true, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x04: if (FIRST) fe_stage<4, 0, true, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x08: fe_stage<8, 0, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x12: fe_stage<2, 1, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x13: fe_stage<3, 1, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x14: fe_stage<4, 1, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x15: fe_stage<5, 1, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x17: fe_stage<7, 1, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x18: fe_stage<8, 1, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x32: fe_stage<2, 3, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x52: fe_stage<2, 5, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x24: fe_stage<4, 2, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                case 0x33: fe_stage<3, 3, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+                default:   fe_stage<4, 3, FIRST, INV>(src, dst, tw, n, p, S, lp); break;
+            }
     }
 
     template<typename T2>
@@ -1269,7 +946,7 @@ namespace mhh
                     const TF dzi = ld(fz.pr.dzi, kg), dti = fz.dti;
                     const TF *u = fz.u + c, *v = fz.v + c, *w = fz.w + c, *ut = fz.ut + c, *vt = fz.vt + c, *wt = fz.wt + c;
                     const int jj = d.icells, kk = d.ijcells;
-                    #pragma unroll 2
+                    #pragma unroll 4
                     for (int i = lane; i < n; i += 32)
                     {
                         const TF du = (ld(ut, i+1) + mulx(ld(u, i+1), dti)) - (ld(ut, i) + mulx(ld(u, i), dti));
@@ -1320,10 +997,10 @@ namespace mhh
         int p = 1;
         for (int st=0; st<A.nst; ++st)
         {
-            const int R = (int)(A.fac >> 4*st) & 15;
-            if (st == 0) fg_any<TF, true, INV>(R, src, dst, tw, n, 1, S, lp);
-            else fg_any<TF, false, INV>(R, src, dst, tw, n, p, S, lp);
-            p *= R;
+            const int code = (int)(A.fac >> 8*st) & 255;
+            if (st == 0) fg_any<TF, true, INV>(code, src, dst, tw, n, 1, S, lp);
+            else fg_any<TF, false, INV>(code, src, dst, tw, n, p, S, lp);
+            p *= code < 32 ? code & 15 : (code & 15)*(code >> 4);
             __syncthreads();
             T2* t = src; src = dst; dst = t;
         }
@@ -1349,28 +1026,47 @@ namespace mhh
         };
         if (ROWS)
         {
-            for (int ls = warp; ls < nloc; ls += FG_NT/32)
+            // A warp (or, with fewer pairs than warps, several) per pair of rows.
+            constexpr int NW = FG_NT/32;
+            const int wpp = P < NW ? NW/P : 1;
+            for (int q = warp/wpp; 2*q < nloc; q += NW/wpp)
             {
+                const bool two = 2*q + 1 < nloc;
                 if (FUSE == 2)
                 {
                     // Straight into the ghost layout of p, with the bottom
                     // ghost level p[kstart-1] = p[kstart]
                     // (src/pres_2.cxx:330-358).
-                    const TF mean = fz.dcm ? fz.dcm[ti.sk[ls]] : TF(0);
-                    for (int i = lane; i < n; i += 32)
+                    const int l0 = 2*q, l1 = two ? 2*q + 1 : 2*q;
+                    TF* x = fz.p + ti.sc[l0];
+                    TF* y = fz.p + ti.sc[l1];
+                    const TF m0 = fz.dcm ? fz.dcm[ti.sk[l0]] : TF(0), m1 = fz.dcm ? fz.dcm[ti.sk[l1]] : TF(0);
+                    const bool g0 = ti.sk[l0] == 0, g1 = ti.sk[l1] == 0;
+                    #pragma unroll 4
+                    for (int i = lane + 32*(warp % wpp); i < n; i += 32*wpp)
                     {
-                        const T2 o = pair_out(i, ls >> 1);
-                        TF val = ls & 1 ? o.y : o.x;
-                        if (fz.dcm) val = add_rn(val, mean);
-                        const long long c = ti.sc[ls] + i;
-                        fz.p[c] = val;
-                        if (ti.sk[ls] == 0) fz.p[c - fz.d.ijcells] = val;
+                        T2 o = pair_out(i, q);
+                        if (fz.dcm) { o.x = add_rn(o.x, m0); o.y = add_rn(o.y, m1); }
+                        x[i] = o.x;
+                        if (g0) x[i - fz.d.ijcells] = o.x;
+                        if (two)
+                        {
+                            y[i] = o.y;
+                            if (g1) y[i - fz.d.ijcells] = o.y;
+                        }
                     }
                 }
                 else
                 {
-                    TF* out = A.data + ti.sb[ls];
-                    for (int i = lane; i < n; i += 32) { const T2 o = pair_out(i, ls >> 1); out[i] = ls & 1 ? o.y : o.x; }
+                    TF* x = A.data + ti.sb[2*q];
+                    TF* y = A.data + ti.sb[two ? 2*q + 1 : 2*q];
+                    #pragma unroll 4
+                    for (int i = lane + 32*(warp % wpp); i < n; i += 32*wpp)
+                    {
+                        const T2 o = pair_out(i, q);
+                        x[i] = o.x;
+                        if (two) y[i] = o.y;
+                    }
                 }
             }
         }
@@ -1404,13 +1100,19 @@ namespace mhh
         A.data = data; A.L = L; A.scale = scale; A.fz = fz;
         A.twt = sizeof(TF) == 8 ? reinterpret_cast<const TF*>(pl.tw_d) : reinterpret_cast<const TF*>(pl.tw_f);
         A.n = pl.n;
-        A.nst = pl.ngfac;
-        for (int q=0; q<pl.ngfac; ++q) A.fac |= (unsigned long long)pl.gfac[q] << 4*q;
-        // Eight pairs (64- or 128-byte runs of columns), fewer where two
-        // buffers of them do not fit.
+        A.nst = sizeof(TF) == 8 ? pl.ngfac : pl.nffac;
+        for (int q=0; q<A.nst && q<8; ++q) A.fac |= (unsigned long long)(sizeof(TF) == 8 ? pl.gfac[q] : pl.ffac[q]) << 8*q;
+        // Pairs per tile, at most eight: columns as many as leave two (float) or
+        // more (double, bound by the FP64 pipe) blocks on an SM, so that a run is
+        // 64 bytes or more; rows, which need no runs, few enough that five
+        // blocks' loads overlap (512 x 512 x 256, 8, 4, 2
+        // pairs: 2.48, 1.85, 2.06 ms per step for x; 150^3 0.177, 0.192, 0.239;
+        // with scalar sums).
         auto bytes = [&](int lp) { return sizeof(T2)*(size_t)pl.n*(2*((1 << lp) + (lp ? 1 : 0)) + 1); };
-        A.lp = 3;
-        while (A.lp > 0 && bytes(A.lp) > (size_t)FG_SMEM) --A.lp;
+        const size_t most = (ROWS ? 46 : (sizeof(TF) == 4 ? 80 : 48))*1024;
+        A.lp = ROWS && sizeof(TF) == 8 ? 2 : 3;
+        while (A.lp > 1 && bytes(A.lp) > most) --A.lp;
+        if (bytes(A.lp) > (size_t)FG_SMEM) A.lp = 0;
         // Pairs of columns move as one element where they are adjacent and the
         // data is aligned for it.
         A.pairs = !ROWS && L.itot % 2 == 0 && reinterpret_cast<size_t>(data) % sizeof(T2) == 0;
@@ -1496,6 +1198,35 @@ namespace mhh
         std::sort(pl->gfac, pl->gfac + pl->ngfac, [](int x, int y) { return x > y; });
     }
 
+    // The float plan: elementary radices 8, 4, 2, 3 for 2^a 3 (a >= 4), 8 after
+    // 2, 4 or 8 in frequency for 128, 256 and 512, and 4, 2, 3, 5, 7 for other
+    // lengths; neighbours grouped where a stage of the product is at hand.
+    static void plan_floats(FftPlan* pl)
+    {
+        const int n = pl->n;
+        pl->nffac = 0;
+        if (n == 128 || n == 256 || n == 512)
+        {
+            pl->ffac[0] = n/64; pl->ffac[1] = pl->ffac[2] = 8;
+            pl->nffac = 3;
+            return;
+        }
+        bool eights = false;
+        for (int m : {16, 32, 48, 64, 96, 192, 384, 768, 1024}) eights = eights || n == m;
+        std::vector<int> rad;
+        int r = n;
+        for (int f : {8, 4, 2, 3, 5, 7})
+            while ((f < 8 || eights) && r % f == 0) { rad.push_back(f); r /= f; }
+        for (size_t q=0; q<rad.size(); ++q)
+        {
+            int code = rad[q] + 16;
+            if (q + 1 < rad.size())
+                for (int pair : {0x32, 0x52, 0x24, 0x33, 0x34})
+                    if (rad[q] == (pair & 15) && rad[q+1] == pair >> 4) { code = pair; ++q; break; }
+            pl->ffac[pl->nffac++] = code;
+        }
+    }
+
     int fft_plan_init(FftPlan* pl, int n, cudaStream_t s)
     {
         std::memset(pl, 0, sizeof(*pl));
@@ -1504,6 +1235,7 @@ namespace mhh
         for (int f : {2, 3, 5, 7}) while (r % f == 0) r /= f;
         if (r != 1) return MHH_ERR_UNSUPPORTED;
         plan_radices(pl);
+        plan_floats(pl);
         std::vector<double> td(2*(size_t)n);
         std::vector<float> tf(2*(size_t)n);
         const long double twopi = 6.283185307179586476925286766559005768L;

@@ -1,5 +1,5 @@
-"""The run-time-plan transforms (lengths without a compile-time schedule, radices
-2 to 10) against numpy's DFT in halfcomplex order and back."""
+"""The run-time-plan transforms (every length but 32 in float; stages of radix
+2 to 12) against numpy's DFT in halfcomplex order and back."""
 import ctypes
 import math
 
@@ -70,3 +70,13 @@ def test_plan(mhh, itot, jtot, precision, offset):
     n = itot * jtot
     assert np.abs(t.double().cpu().numpy() / n - x).max() <= 2 * tol * np.abs(x).max()
     kern.mhh_ctx_destroy(h)
+
+
+# The lengths of radix 8: 2^a, 2^a 3, and 128, 256 and 512 in frequency.
+EIGHTS = [(16, 48), (64, 96), (128, 192), (256, 384), (512, 128), (768, 256), (1024, 512)]
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("itot,jtot", EIGHTS)
+def test_eights(mhh, itot, jtot, precision):
+    test_plan(mhh, itot, jtot, precision, 0)
