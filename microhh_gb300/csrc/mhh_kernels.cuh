@@ -106,6 +106,9 @@ namespace mhh
     template<typename TF> void launch_tendency_flux(const Dims& d, const Prof<TF>& pr, const TendArgs<TF>& a,
                                                     bool surf, bool scal, bool buoy, bool lim, int kchunk,
                                                     cudaStream_t s);
+    // Advec_2i5 (adv) or Diff_smag2 alone in flux form.
+    template<typename TF> void launch_tendency_flux_term(const Dims& d, const Prof<TF>& pr, const TendArgs<TF>& a, bool adv,
+                                                         bool surf, bool scal, bool lim, int kchunk, cudaStream_t s);
     // Advec_2 + Diff_2 in flux form; force: a.fbody is added to u.
     template<typename TF> void launch_tendency_2(const Dims& d, const Prof<TF>& pr, const TendArgs<TF>& a, bool scal,
                                                  bool buoy, bool force, int kchunk, cudaStream_t s);

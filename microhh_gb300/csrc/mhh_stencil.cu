@@ -413,8 +413,11 @@ namespace mhh
         const TF dxi = dxi_of<TF>(d), dyi = dyi_of<TF>(d);
         const TF* u = a.u; const TF* v = a.v; const TF* w = a.w;
 
+        // A field that no term changes is not touched.
         constexpr bool A2I5 = ADV == MHH_ADVEC_2I5 || ADV == ADVEC_2I5_LIM;
+        constexpr bool TERM = ADV != 0 || DIF != 0;
         // u
+        if (TERM || FORCE)
         {
             TF t = TF(0);
             if (A2I5) t += advec_2i5_u(d, pr, u, v, w, c, k, dxi, dyi);
@@ -425,6 +428,7 @@ namespace mhh
             a.ut[c] += t;
         }
         // v
+        if (TERM)
         {
             TF t = TF(0);
             if (A2I5) t += advec_2i5_v(d, pr, u, v, w, c, k, dxi, dyi);
@@ -434,7 +438,7 @@ namespace mhh
             a.vt[c] += t;
         }
         // w (half levels above the wall)
-        if (k > d.kstart)
+        if ((TERM || BUOY) && k > d.kstart)
         {
             TF t = TF(0);
             if (BUOY) t += TF(GRAV)/ld(pr.threfh, k)*(i2(ld(a.s, c-d.ijcells), ld(a.s, c)) - ld(pr.thbh, k));
@@ -445,7 +449,7 @@ namespace mhh
             a.wt[c] += t;
         }
         // scalar
-        if (SCAL)
+        if (TERM && SCAL)
         {
             TF t = TF(0);
             if (ADV == ADVEC_2I5_LIM) t += advec_2i5_s_lim(d, pr, a.s, u, v, w, c, k, dxi, dyi);
@@ -522,8 +526,15 @@ namespace mhh
             else launch_tendency_les<TF>(d, pr, a, surf, scal, buoy, s);
             return;
         }
-        // The DNS combination in flux form (mhh_tend_2.cu); its terms alone (the
-        // module calls) and every other combination run per cell.
+        // Advec_2i5 or Diff_smag2 alone (the module calls) in the flux form too.
+        if (var == 2 && !force && !buoy && d.igc >= 3 && d.jgc >= 3
+            && (((adv == MHH_ADVEC_2I5 || lim) && dif == 0) || (adv == 0 && dif == MHH_DIFF_SMAG2)))
+        {
+            launch_tendency_flux_term<TF>(d, pr, a, adv != 0, surf, scal, lim, o.tend_kchunk, s);
+            return;
+        }
+        // The DNS combination in flux form (mhh_tend_2.cu); its terms alone and
+        // every other combination run per cell.
         if (var == 2 && adv == MHH_ADVEC_2 && dif == MHH_DIFF_2)
         {
             launch_tendency_2<TF>(d, pr, a, scal, buoy, force, o.tend_kchunk, s);
@@ -565,11 +576,11 @@ namespace mhh
     template<typename TF>
     __global__ void k_rk3(TF* __restrict__ a, TF* __restrict__ at, Dims d, TF cbdt, TF ca, int last)
     {
-        const long long n = blockIdx.x*(long long)blockDim.x + threadIdx.x;
-        if (n >= d.ncells) return;
-        const int i = (int)(n % d.icells);
-        const int j = (int)((n / d.icells) % d.jcells);
-        const int k = (int)(n / d.ijcells);
+        const int i = blockIdx.x*blockDim.x + threadIdx.x;
+        const int j = blockIdx.y*blockDim.y + threadIdx.y;
+        const int k = blockIdx.z;
+        if (i >= d.icells || j >= d.jcells) return;
+        const long long n = ijk(d, i, j, k);
         const bool interior = i >= d.istart && i < d.iend && j >= d.jstart && j < d.jend && k >= d.kstart && k < d.kend;
         if (interior)
         {
@@ -634,8 +645,8 @@ namespace mhh
         const double cA[3] = {0., -5./9., -153./128.};
         const double cB[3] = {1./3., 15./16., 8./15.};
         const int sn = (substep + 1) % 3;
-        const long long n = d.ncells;
-        k_rk3<TF><<<(unsigned)((n + 255)/256), 256, 0, s>>>(a, at, d, TF(cB[substep]*dt), TF(cA[sn]), sn == 0);
+        dim3 block(32, 8), grid((d.icells + 31)/32, (d.jcells + 7)/8, d.kcells);
+        k_rk3<TF><<<grid, block, 0, s>>>(a, at, d, TF(cB[substep]*dt), TF(cA[sn]), sn == 0);
         count_launch();
     }
 

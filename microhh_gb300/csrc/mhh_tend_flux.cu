@@ -64,7 +64,12 @@ namespace mhh
 
     template<typename TF> struct TendFluxP { Dims d; Prof<TF> pr; TendArgs<TF> a; int kchunk; };
 
-    template<typename TF, bool SURF, bool SCAL, bool BUOY, bool LIM>
+    // ADV, DIF: with one of them false the other term alone (the module calls of
+    // Advec_2i5 and Diff_smag2; the per-cell kernels they replace evaluate every
+    // flux from both sides.  Step by modules, ms: float 96 x 96 x 64 0.686, now
+    // 0.663, 256 x 256 x 128 4.66, now 3.33; FP64 3.52, now 2.05 and 42.1, now
+    // 21.5).
+    template<typename TF, bool SURF, bool SCAL, bool BUOY, bool LIM, bool ADV = true, bool DIF = true>
     __device__ __forceinline__ void tend_flux_body(const TendFluxP<TF>& P, const VBlock& vb)
     {
         const Dims& d = P.d;
@@ -154,7 +159,8 @@ namespace mhh
         {
             const unsigned lo = level(l);
             const int so = (l & 3)*FPS;
-            plane(SU, u, lo, so); plane(SV, v, lo, so); plane(SE, ev, lo, so); plane(SW, w, lo, so);
+            plane(SU, u, lo, so); plane(SV, v, lo, so); plane(SW, w, lo, so);
+            if (DIF) plane(SE, ev, lo, so);
             if (SCAL && l < m0+3) plane(SS, s, lo, so);
         }
         cp_async_commit();
@@ -191,7 +197,7 @@ namespace mhh
 
         // Double form: the viscosity sums of the own faces at levels m and m+1.
         TF ex0 = 0, ey0 = 0, ex1 = 0, ey1 = 0;
-        if (sizeof(TF) == 8 && face)
+        if (sizeof(TF) == 8 && DIF && face)
         {
             const TF* E = sm + SE*FPS + (m0 & 3)*FPS + pc;
             ex0 = E[-1] + E[0];
@@ -243,7 +249,8 @@ namespace mhh
             {
                 if constexpr (sizeof(TF) == 4)
                 {
-                    const TF txy = (TF(0.25)*(PL(E0,-1,-1) + PL(E0,0,-1) + PL(E0,-1,0) + PL(E0,0,0)) + visc)
+                    const float2 zero = make_float2(0.f, 0.f);
+                    const TF txy = !DIF ? TF(0) : (TF(0.25)*(PL(E0,-1,-1) + PL(E0,0,-1) + PL(E0,-1,0) + PL(E0,0,0)) + visc)
                                  * ((PL(U0,0,0) - PL(U0,0,-1))*dyi + (PL(V0,0,0) - PL(V0,-1,0))*dxi);
                     // tau_xz and tau_yz in one packed pair.
                     const float2 ez = __ffma2_rn(__fadd2_rn(__fadd2_rn(f2(PL(E0,-1,0), PL(E0,0,-1)), f2(PL(E0,0,0), PL(E0,0,0))),
@@ -252,25 +259,25 @@ namespace mhh
                     const float2 gz = __ffma2_rn(sub2(f2(PL(U1,0,0), PL(V1,0,0)), f2(PL(U0,0,0), PL(V0,0,0))), f2(dzhi1, dzhi1),
                                                  __fmul2_rn(sub2(f2(PL(W1,0,0), PL(W1,0,0)), f2(PL(W1,-1,0), PL(W1,0,-1))),
                                                             f2(dxi, dyi)));
-                    const float2 tz = __fmul2_rn(ez, gz);
+                    const float2 tz = DIF ? __fmul2_rn(ez, gz) : zero;
                     txz = tz.x; tyz = tz.y;
                     // Float form: the x- and y-face advective fluxes of each
                     // field in packed pairs (both computed by every face
                     // thread; the plane holds the stencils of the edge faces).
-                    const float2 Au = adv6x2(make_float2(i2(PL(U0,-1,0), PL(U0,0,0)), i2(PL(V0,-1,0), PL(V0,0,0))),
+                    const float2 Au = !ADV ? zero : adv6x2(make_float2(i2(PL(U0,-1,0), PL(U0,0,0)), i2(PL(V0,-1,0), PL(V0,0,0))),
                                              make_float2(PL(U0,-3,0), PL(U0,0,-3)), make_float2(PL(U0,-2,0), PL(U0,0,-2)),
                                              make_float2(PL(U0,-1,0), PL(U0,0,-1)), make_float2(PL(U0,0,0), PL(U0,0,0)),
                                              make_float2(PL(U0,1,0), PL(U0,0,1)), make_float2(PL(U0,2,0), PL(U0,0,2)));
-                    const float2 Av = adv6x2(make_float2(i2(PL(U0,0,-1), PL(U0,0,0)), i2(PL(V0,0,-1), PL(V0,0,0))),
+                    const float2 Av = !ADV ? zero : adv6x2(make_float2(i2(PL(U0,0,-1), PL(U0,0,0)), i2(PL(V0,0,-1), PL(V0,0,0))),
                                              make_float2(PL(V0,-3,0), PL(V0,0,-3)), make_float2(PL(V0,-2,0), PL(V0,0,-2)),
                                              make_float2(PL(V0,-1,0), PL(V0,0,-1)), make_float2(PL(V0,0,0), PL(V0,0,0)),
                                              make_float2(PL(V0,1,0), PL(V0,0,1)), make_float2(PL(V0,2,0), PL(V0,0,2)));
-                    const float2 Aw = adv6x2(make_float2(i2(PL(U0,0,0), PL(U1,0,0)), i2(PL(V0,0,0), PL(V1,0,0))),
+                    const float2 Aw = !ADV ? zero : adv6x2(make_float2(i2(PL(U0,0,0), PL(U1,0,0)), i2(PL(V0,0,0), PL(V1,0,0))),
                                              make_float2(PL(W1,-3,0), PL(W1,0,-3)), make_float2(PL(W1,-2,0), PL(W1,0,-2)),
                                              make_float2(PL(W1,-1,0), PL(W1,0,-1)), make_float2(PL(W1,0,0), PL(W1,0,0)),
                                              make_float2(PL(W1,1,0), PL(W1,0,1)), make_float2(PL(W1,2,0), PL(W1,0,2)));
-                    float2 As = make_float2(0.f, 0.f);
-                    if (SCAL)
+                    float2 As = zero;
+                    if (SCAL && ADV)
                     {
                         if (LIM)
                             As = make_float2(lim_flux(PL(U0,0,0), PL(S0,-2,0), PL(S0,-1,0), PL(S0,0,0), PL(S0,1,0), 0),
@@ -285,10 +292,10 @@ namespace mhh
                     // x and y, in packed pairs.
                     const float2 eo = f2(PL(E0,-1,0), PL(E0,0,-1));
                     const float2 h2 = f2(dxi, dyi);
-                    const float2 Duv = __fmul2_rn(__fmul2_rn(__fadd2_rn(eo, f2(visc, visc)), f2(2.f, 2.f)),
+                    const float2 Duv = !DIF ? zero : __fmul2_rn(__fmul2_rn(__fadd2_rn(eo, f2(visc, visc)), f2(2.f, 2.f)),
                                                   __fmul2_rn(sub2(f2(PL(U0,0,0), PL(V0,0,0)), f2(PL(U0,-1,0), PL(V0,0,-1))), h2));
-                    float2 Ds = f2(0.f, 0.f);
-                    if (SCAL)
+                    float2 Ds = zero;
+                    if (SCAL && DIF)
                         Ds = __fmul2_rn(__ffma2_rn(__fmul2_rn(__fadd2_rn(eo, f2(PL(E0,0,0), PL(E0,0,0))), f2(0.5f, 0.5f)),
                                                    f2(tpri, tpri), f2(svisc, svisc)),
                                         __fmul2_rn(sub2(f2(PL(S0,0,0), PL(S0,0,0)), f2(PL(S0,-1,0), PL(S0,0,-1))), h2));
@@ -307,64 +314,63 @@ namespace mhh
                     // viscosity at the face's two cells shared between the
                     // stresses and carried up a level, constant factors
                     // folded, each flux one FMA off its advective part.
-                    ex1 = PL(E1,-1,0) + PL(E1,0,0);
-                    ey1 = PL(E1,0,-1) + PL(E1,0,0);
-                    const TF txy = fma(ex0 + (PL(E0,-1,-1) + PL(E0,0,-1)), TF(0.25), visc)
+                    if (DIF) { ex1 = PL(E1,-1,0) + PL(E1,0,0); ey1 = PL(E1,0,-1) + PL(E1,0,0); }
+                    const TF txy = !DIF ? TF(0) : fma(ex0 + (PL(E0,-1,-1) + PL(E0,0,-1)), TF(0.25), visc)
                                  * fma(PL(V0,0,0) - PL(V0,-1,0), dxi, (PL(U0,0,0) - PL(U0,0,-1))*dyi);
                     if (face_x)
                     {
-                        txz = fma(ex0 + ex1, TF(0.25), visc)
+                        if (DIF) txz = fma(ex0 + ex1, TF(0.25), visc)
                             * fma(PL(W1,0,0) - PL(W1,-1,0), dxi, (PL(U1,0,0) - PL(U0,0,0))*dzhi1);
                         // u at the cell centre i-1.
                         {
                             const TF uw = PL(U0,-1,0) + PL(U0,0,0);
-                            const TF A = uw*upwind5<true>(uw, PL(U0,-3,0), PL(U0,-2,0), PL(U0,-1,0), PL(U0,0,0), PL(U0,1,0), PL(U0,2,0));
-                            gx[(gxi)*4 + 0] = fma(fma(PL(E0,-1,0), TF(2)*dxi, TF(2)*dxi*visc), PL(U0,0,0) - PL(U0,-1,0), -A);
+                            const TF A = (!ADV ? TF(0) : uw*upwind5<true>(uw, PL(U0,-3,0), PL(U0,-2,0), PL(U0,-1,0), PL(U0,0,0), PL(U0,1,0), PL(U0,2,0)));
+                            gx[(gxi)*4 + 0] = DIF ? fma(fma(PL(E0,-1,0), TF(2)*dxi, TF(2)*dxi*visc), PL(U0,0,0) - PL(U0,-1,0), -A) : -A;
                         }
                         // v at (i-1/2, j-1/2).
                         {
                             const TF uw = PL(U0,0,-1) + PL(U0,0,0);
-                            gx[(gxi)*4 + 1] = fma(-uw, upwind5<true>(uw, PL(V0,-3,0), PL(V0,-2,0), PL(V0,-1,0), PL(V0,0,0), PL(V0,1,0), PL(V0,2,0)), txy);
+                            gx[(gxi)*4 + 1] = ADV ? fma(-uw, upwind5<true>(uw, PL(V0,-3,0), PL(V0,-2,0), PL(V0,-1,0), PL(V0,0,0), PL(V0,1,0), PL(V0,2,0)), txy) : txy;
                         }
                         // w at (i-1/2, m+1/2).
                         {
                             const TF uw = PL(U0,0,0) + PL(U1,0,0);
-                            gx[(gxi)*4 + 2] = fma(-uw, upwind5<true>(uw, PL(W1,-3,0), PL(W1,-2,0), PL(W1,-1,0), PL(W1,0,0), PL(W1,1,0), PL(W1,2,0)), txz);
+                            gx[(gxi)*4 + 2] = ADV ? fma(-uw, upwind5<true>(uw, PL(W1,-3,0), PL(W1,-2,0), PL(W1,-1,0), PL(W1,0,0), PL(W1,1,0), PL(W1,2,0)), txz) : txz;
                         }
                         if (SCAL)
                         {
                             const TF uw = PL(U0,0,0);
-                            const TF A = LIM ? lim_flux(uw, PL(S0,-2,0), PL(S0,-1,0), PL(S0,0,0), PL(S0,1,0), 0)
-                                             : uw*upwind5<false>(uw, PL(S0,-3,0), PL(S0,-2,0), PL(S0,-1,0), PL(S0,0,0), PL(S0,1,0), PL(S0,2,0));
-                            gx[(gxi)*4 + 3] = fma(fma(ex0, TF(0.5)*tpri*dxi, svisc*dxi), PL(S0,0,0) - PL(S0,-1,0), -A);
+                            const TF A = LIM && ADV ? lim_flux(uw, PL(S0,-2,0), PL(S0,-1,0), PL(S0,0,0), PL(S0,1,0), 0)
+                                             : (!ADV ? TF(0) : uw*upwind5<false>(uw, PL(S0,-3,0), PL(S0,-2,0), PL(S0,-1,0), PL(S0,0,0), PL(S0,1,0), PL(S0,2,0)));
+                            gx[(gxi)*4 + 3] = DIF ? fma(fma(ex0, TF(0.5)*tpri*dxi, svisc*dxi), PL(S0,0,0) - PL(S0,-1,0), -A) : -A;
                         }
                     }
                     if (face_y)
                     {
-                        tyz = fma(ey0 + ey1, TF(0.25), visc)
+                        if (DIF) tyz = fma(ey0 + ey1, TF(0.25), visc)
                             * fma(PL(W1,0,0) - PL(W1,0,-1), dyi, (PL(V1,0,0) - PL(V0,0,0))*dzhi1);
                         // u at (i-1/2, j-1/2).
                         {
                             const TF vs = PL(V0,-1,0) + PL(V0,0,0);
-                            gy[(gyi)*4 + 0] = fma(-vs, upwind5<true>(vs, PL(U0,0,-3), PL(U0,0,-2), PL(U0,0,-1), PL(U0,0,0), PL(U0,0,1), PL(U0,0,2)), txy);
+                            gy[(gyi)*4 + 0] = ADV ? fma(-vs, upwind5<true>(vs, PL(U0,0,-3), PL(U0,0,-2), PL(U0,0,-1), PL(U0,0,0), PL(U0,0,1), PL(U0,0,2)), txy) : txy;
                         }
                         // v at the cell centre j-1.
                         {
                             const TF vs = PL(V0,0,-1) + PL(V0,0,0);
-                            const TF A = vs*upwind5<true>(vs, PL(V0,0,-3), PL(V0,0,-2), PL(V0,0,-1), PL(V0,0,0), PL(V0,0,1), PL(V0,0,2));
-                            gy[(gyi)*4 + 1] = fma(fma(PL(E0,0,-1), TF(2)*dyi, TF(2)*dyi*visc), PL(V0,0,0) - PL(V0,0,-1), -A);
+                            const TF A = (!ADV ? TF(0) : vs*upwind5<true>(vs, PL(V0,0,-3), PL(V0,0,-2), PL(V0,0,-1), PL(V0,0,0), PL(V0,0,1), PL(V0,0,2)));
+                            gy[(gyi)*4 + 1] = DIF ? fma(fma(PL(E0,0,-1), TF(2)*dyi, TF(2)*dyi*visc), PL(V0,0,0) - PL(V0,0,-1), -A) : -A;
                         }
                         // w at (j-1/2, m+1/2).
                         {
                             const TF vs = PL(V0,0,0) + PL(V1,0,0);
-                            gy[(gyi)*4 + 2] = fma(-vs, upwind5<true>(vs, PL(W1,0,-3), PL(W1,0,-2), PL(W1,0,-1), PL(W1,0,0), PL(W1,0,1), PL(W1,0,2)), tyz);
+                            gy[(gyi)*4 + 2] = ADV ? fma(-vs, upwind5<true>(vs, PL(W1,0,-3), PL(W1,0,-2), PL(W1,0,-1), PL(W1,0,0), PL(W1,0,1), PL(W1,0,2)), tyz) : tyz;
                         }
                         if (SCAL)
                         {
                             const TF vs = PL(V0,0,0);
-                            const TF A = LIM ? lim_flux(vs, PL(S0,0,-2), PL(S0,0,-1), PL(S0,0,0), PL(S0,0,1), 0)
-                                             : vs*upwind5<false>(vs, PL(S0,0,-3), PL(S0,0,-2), PL(S0,0,-1), PL(S0,0,0), PL(S0,0,1), PL(S0,0,2));
-                            gy[(gyi)*4 + 3] = fma(fma(ey0, TF(0.5)*tpri*dyi, svisc*dyi), PL(S0,0,0) - PL(S0,0,-1), -A);
+                            const TF A = LIM && ADV ? lim_flux(vs, PL(S0,0,-2), PL(S0,0,-1), PL(S0,0,0), PL(S0,0,1), 0)
+                                             : (!ADV ? TF(0) : vs*upwind5<false>(vs, PL(S0,0,-3), PL(S0,0,-2), PL(S0,0,-1), PL(S0,0,0), PL(S0,0,1), PL(S0,0,2)));
+                            gy[(gyi)*4 + 3] = DIF ? fma(fma(ey0, TF(0.5)*tpri*dyi, svisc*dyi), PL(S0,0,0) - PL(S0,0,-1), -A) : -A;
                         }
                     }
                 }
@@ -375,7 +381,7 @@ namespace mhh
             if (cell)
             {
                 const int kf = m + 1;
-                const int ot = face_order_full(d, kf);
+                const int ot = ADV ? face_order_full(d, kf) : 0;      // 0: no advective flux
                 const TF rhoh1 = pl[1*PLEV];
                 // u and v: diffusive flux from the shear stress of the same
                 // face, or the surface model's flux at the walls.
@@ -418,7 +424,7 @@ namespace mhh
                 if (SCAL)
                 {
                     const TF ds = (SURF && kf == d.kstart) ? -sfb : ((SURF && kf == d.kend) ? -sft
-                                : (TF(0.5)*(PL(E0,0,0) + PL(E1,0,0))*tpri + svisc)*(qs[3] - qs[2])*dzhi1);
+                                : (DIF ? (TF(0.5)*(PL(E0,0,0) + PL(E1,0,0))*tpri + svisc)*(qs[3] - qs[2])*dzhi1 : TF(0)));
                     TF as;
                     if (paired) as = aws.y;
                     else if (LIM)
@@ -435,9 +441,10 @@ namespace mhh
                 if (kf < d.kend)
                 {
                     const int ow = face_order_w(d, kf);
-                    const TF dw = TF(2)*(PL(E1,0,0) + visc)*(qw[3] - qw[2])*pl[3*PLEV];
+                    const TF dw = !DIF ? TF(0) : TF(2)*(PL(E1,0,0) + visc)*(qw[3] - qw[2])*pl[3*PLEV];
                     TF aw;
-                    if (paired) aw = aws.x;
+                    if (!ADV) aw = TF(0);
+                    else if (paired) aw = aws.x;
                     else if (sizeof(TF) == 8 && ow == 6)
                     {
                         const TF ww = qw[2] + qw[3];
@@ -464,7 +471,8 @@ namespace mhh
             if (m + 3 < k1)
             {
                 const int so = (m & 3)*FPS;
-                plane(SU, u, lo4, so); plane(SV, v, lo4, so); plane(SW, w, lo4, so); plane(SE, ev, lo4, so);
+                plane(SU, u, lo4, so); plane(SV, v, lo4, so); plane(SW, w, lo4, so);
+                if (DIF) plane(SE, ev, lo4, so);
                 if (SCAL) plane(SS, s, (unsigned)(m + 3)*ij, ((m + 3) & 3)*FPS);
             }
             cp_async_commit();
@@ -528,14 +536,14 @@ namespace mhh
         cp_async_wait_all();
     }
 
-    template<typename TF, bool SURF, bool SCAL, bool BUOY, bool LIM = false>
+    template<typename TF, bool SURF, bool SCAL, bool BUOY, bool LIM = false, bool ADV = true, bool DIF = true>
     static void launch_flux_t(const Dims& d, const Prof<TF>& pr, const TendArgs<TF>& a, int kchunk, cudaStream_t s)
     {
         const size_t smem = flux_smem<TF>();
         kchunk = auto_kchunk(kchunk, (long long)((d.itot + FTX - 1)/FTX)*((d.jtot + FTY - 1)/FTY), d.ktot,
                              sizeof(TF) == 8, FKCHUNK_MAX);
         dim3 grid((d.itot + FTX - 1)/FTX, (d.jtot + FTY - 1)/FTY, (d.ktot + kchunk - 1)/kchunk);
-        launch_body<TendFluxP<TF>, tend_flux_body<TF, SURF, SCAL, BUOY, LIM>, NTHR, FluxOcc<TF>::v>(
+        launch_body<TendFluxP<TF>, tend_flux_body<TF, SURF, SCAL, BUOY, LIM, ADV, DIF>, NTHR, FluxOcc<TF>::v>(
             grid, dim3(NTHR), smem, s, TendFluxP<TF>{d, pr, a, kchunk});
         count_launch();
     }
@@ -567,6 +575,30 @@ namespace mhh
         }
     }
 
+    template<typename TF>
+    void launch_tendency_flux_term(const Dims& d, const Prof<TF>& pr, const TendArgs<TF>& a, bool adv, bool surf,
+                                   bool scal, bool lim, int kchunk, cudaStream_t s)
+    {
+        if (adv)
+        {
+            if (lim && scal) launch_flux_t<TF, false, true, false, true, true, false>(d, pr, a, kchunk, s);
+            else if (scal) launch_flux_t<TF, false, true, false, false, true, false>(d, pr, a, kchunk, s);
+            else launch_flux_t<TF, false, false, false, false, true, false>(d, pr, a, kchunk, s);
+        }
+        else if (surf)
+        {
+            if (scal) launch_flux_t<TF, true, true, false, false, false, true>(d, pr, a, kchunk, s);
+            else launch_flux_t<TF, true, false, false, false, false, true>(d, pr, a, kchunk, s);
+        }
+        else
+        {
+            if (scal) launch_flux_t<TF, false, true, false, false, false, true>(d, pr, a, kchunk, s);
+            else launch_flux_t<TF, false, false, false, false, false, true>(d, pr, a, kchunk, s);
+        }
+    }
+
+    template void launch_tendency_flux_term<double>(const Dims&, const Prof<double>&, const TendArgs<double>&, bool, bool, bool, bool, int, cudaStream_t);
+    template void launch_tendency_flux_term<float>(const Dims&, const Prof<float>&, const TendArgs<float>&, bool, bool, bool, bool, int, cudaStream_t);
     template void launch_tendency_flux<double>(const Dims&, const Prof<double>&, const TendArgs<double>&, bool, bool, bool, bool, int, cudaStream_t);
     template void launch_tendency_flux<float>(const Dims&, const Prof<float>&, const TendArgs<float>&, bool, bool, bool, bool, int, cudaStream_t);
 }
