@@ -122,6 +122,11 @@ long long mhh_launch_count(void);
 /* Adds n to that count: a driver that replays a captured CUDA graph adds the
    graph's kernel nodes per replay (no counterpart in the reference). */
 int mhh_launch_count_add(long long n);
+/* A number that changes with every setting that a launch of this context reads
+   (options, flux limiter, surface tables, buffer layer); 0 while timing is on,
+   when launches must not be replayed.  A driver that keeps captured launches
+   drops them when it changes (no counterpart in the reference). */
+unsigned long long mhh_ctx_settings(const mhh_ctx* ctx);
 /* Device memory the context allocated (measured at creation), and an upper
    estimate of it from the grid alone, for admission by memory budget (no
    counterpart in the reference). */

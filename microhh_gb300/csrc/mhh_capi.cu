@@ -21,6 +21,7 @@ namespace
     struct TimerEntry { std::string name; long long count = 0; double ms = 0.; };
     struct PendingPair { int idx; cudaEvent_t a, b; };
     bool g_timing = false;
+    std::atomic<unsigned long long> g_settings{1};   // changes of process-wide options
     std::vector<TimerEntry> g_timers;
     std::vector<PendingPair> g_pending;
     std::vector<cudaEvent_t> g_event_pool;
@@ -143,6 +144,7 @@ constexpr int STAT_SPLIT = 16;
 
 struct mhh_ctx
 {
+    unsigned long long settings = 0;    // changes of this context's settings
     mhh_grid g;
     Dims d;
     int prec;
@@ -626,9 +628,15 @@ extern "C" {
 
 const char* mhh_last_error(void) { return g_last_error.c_str(); }
 
+unsigned long long mhh_ctx_settings(const mhh_ctx* c)
+{
+    return !c || g_timing ? 0 : g_settings + c->settings;
+}
+
 int mhh_set_option(const char* name, int value)
 {
     if (!name) return fail(MHH_ERR_ARG, "NULL option");
+    ++g_settings;
     if (!std::strcmp(name, "tendency_kernel"))
     {
         if (value < -1 || value > 2) return fail(MHH_ERR_ARG, "tendency_kernel is -1, 0, 1 or 2");
@@ -677,6 +685,7 @@ int mhh_set_option(const char* name, int value)
 int mhh_ctx_set_option(mhh_ctx* c, const char* name, int value)
 {
     if (!c || !name) return fail(MHH_ERR_ARG, "NULL argument");
+    ++c->settings;
     const bool reset = value == -2;
     if (!std::strcmp(name, "tendency_kernel"))
     {
@@ -1000,6 +1009,7 @@ int mhh_boundary_ghost_cells(mhh_ctx* c, void* a, int bt, const void* abot, cons
 int mhh_boundary_surface_init(mhh_ctx* c, int thermo_bc)
 {
     if (!c) return fail(MHH_ERR_ARG, "NULL argument");
+    ++c->settings;
     if (thermo_bc != MHH_BC_FLUX && thermo_bc != MHH_BC_DIRICHLET)
         return fail(MHH_ERR_ARG, "surface model needs a flux or Dirichlet scalar BC");
     std::vector<float> zL, f;
@@ -1086,6 +1096,7 @@ int mhh_advec_2i5_exec(mhh_ctx* c, const mhh_fields* f, cudaStream_t s)
 int mhh_advec_2i5_set_fluxlimit(mhh_ctx* c, int limit_scalar)
 {
     if (!c) return fail(MHH_ERR_ARG, "NULL argument");
+    ++c->settings;
     // The limiter's wall treatment needs four levels (src/advec_2i5.cxx
     // applies separate stencils at kstart, kstart+1, kend-2 and kend-1).
     if (limit_scalar && c->d.ktot < 4) return fail(MHH_ERR_ARG, "the flux limiter needs ktot >= 4");
@@ -1260,6 +1271,7 @@ static int upload_buffer(mhh_ctx* c)
 int mhh_buffer_setup(mhh_ctx* c, double zstart, double sigma, double beta)
 {
     if (!c) return fail(MHH_ERR_ARG, "NULL argument");
+    ++c->settings;
     const Dims& d = c->d;
     const int kc = d.kcells;
     if (c->hbuf.empty()) c->hbuf.assign(5*(size_t)kc, 0.);
@@ -1286,6 +1298,7 @@ int mhh_buffer_setup(mhh_ctx* c, double zstart, double sigma, double beta)
 int mhh_buffer_set_profile(mhh_ctx* c, const char* name, const double* prof)
 {
     if (!c || !name || !prof) return fail(MHH_ERR_ARG, "NULL argument");
+    ++c->settings;
     if (!c->buf_on) return fail(MHH_ERR_ARG, "buffer layer not set up");
     int q = -1;
     if (!std::strcmp(name, "u")) q = 2;

@@ -306,6 +306,7 @@ namespace mhh_host
             bool in_substep() const { return substep > 0; }
             // src/timeloop.cxx:179-188: status every outputiter iterations at
             // the start of a step (every substep with outputiter = 0).
+            bool checks_substeps() const { return outputiter == 0; }
             bool do_check() const { return outputiter == 0 || (iteration % outputiter == 0 && !in_substep()); }
             void step_time();
             double get_dt() const { return dt; }
@@ -380,7 +381,28 @@ namespace mhh_host
             void check_status();
         private:
             void set_time_step();
-            void substep_modules();
+            // A substep's launches, without the step's time.
+            void work_fused();
+            void work_modules();
+            // The rest of a fixed-dt step as one graph launch, from its first
+            // substep (fused) or its second (modules, whose first asks for the
+            // time-step limits); false: not replayed.
+            bool replay(bool fused);
+            bool capture(bool fused);
+            void drop_graph();
+            struct StepKey
+            {
+                mhh_fields f;
+                mhh_bcfields b;
+                double dt;
+                unsigned long long settings;
+                unsigned long long fused;
+            };
+            StepKey key_{};
+            int seen_ = 0;              // steps begun with this key
+            cudaGraphExec_t graph_ = nullptr;
+            long long graph_kernels_ = 0;
+            cudaStream_t cap_ = nullptr;
             std::string ini_text;
             std::vector<double> z_full;
             bool adaptive_ = true;
