@@ -8,6 +8,9 @@
 
 namespace mhh
 {
+    // Blocks that a launch may have along y and along z.
+    constexpr int MAX_GRID_YZ = 65535;
+
     // Grid dimensions as kernel parameters (by value).
     struct Dims
     {

@@ -232,6 +232,13 @@ namespace mhh
         const int nitem = 2*d.igc*d.jcells + 2*d.jgc*d.itot;
         const int bx = min((nitem + NT - 1)/NT, 64);
         const int wall = gl.n ? ((d.ijcells + NT - 1)/NT + bx - 1)/bx : 0;
+        if (d.kcells + wall > MAX_GRID_YZ)
+        {
+            // The tallest grids and the widest planes: one launch after the other.
+            launch_cyclic(fl, d, MHH_EDGE_BOTH, s);
+            if (gl.n) launch_ghost(gl, d, dzh, s);
+            return;
+        }
         launch_body<GhostsP<TF>, ghosts_body<TF>, NT>(dim3(bx, d.kcells + wall), dim3(NT), 0, s, GhostsP<TF>{fl, gl, d, dzh});
         count_launch();
     }
@@ -578,18 +585,21 @@ namespace mhh
     {
         const int i = blockIdx.x*blockDim.x + threadIdx.x;
         const int j = blockIdx.y*blockDim.y + threadIdx.y;
-        const int k = blockIdx.z;
         if (i >= d.icells || j >= d.jcells) return;
-        const long long n = ijk(d, i, j, k);
-        const bool interior = i >= d.istart && i < d.iend && j >= d.jstart && j < d.jend && k >= d.kstart && k < d.kend;
-        if (interior)
+        // One level per block of the grid's z, which ends at MAX_GRID_YZ.
+        for (int k = blockIdx.z; k < d.kcells; k += gridDim.z)
         {
-            const TF t = at[n];
-            a[n] = a[n] + mulx(cbdt, t);
-            at[n] = last ? TF(0) : t*ca;
+            const long long n = ijk(d, i, j, k);
+            const bool interior = i >= d.istart && i < d.iend && j >= d.jstart && j < d.jend && k >= d.kstart && k < d.kend;
+            if (interior)
+            {
+                const TF t = at[n];
+                a[n] = a[n] + mulx(cbdt, t);
+                at[n] = last ? TF(0) : t*ca;
+            }
+            else if (last)
+                at[n] = TF(0);
         }
-        else if (last)
-            at[n] = TF(0);
     }
 
     // ---------------------------------------------------------------------
@@ -645,7 +655,7 @@ namespace mhh
         const double cA[3] = {0., -5./9., -153./128.};
         const double cB[3] = {1./3., 15./16., 8./15.};
         const int sn = (substep + 1) % 3;
-        dim3 block(32, 8), grid((d.icells + 31)/32, (d.jcells + 7)/8, d.kcells);
+        dim3 block(32, 8), grid((d.icells + 31)/32, (d.jcells + 7)/8, min(d.kcells, MAX_GRID_YZ));
         k_rk3<TF><<<grid, block, 0, s>>>(a, at, d, TF(cB[substep]*dt), TF(cA[sn]), sn == 0);
         count_launch();
     }
