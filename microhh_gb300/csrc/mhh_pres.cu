@@ -717,9 +717,13 @@ namespace mhh
         if (!INV) return src[e*S + q];
         const int kk = 2*e <= n ? e : n - e;
         const bool real_only = kk == 0 || 2*kk == n;
-        const T2 a = src[kk*S + q], b = src[(real_only ? kk : n - kk)*S + q];
         using TF = std::remove_cv_t<decltype(T2::x)>;
-        const TF sg = real_only ? TF(0) : (2*e <= n ? TF(1) : TF(-1));
+        const T2 a = src[kk*S + q];
+        // The imaginary part of a real coefficient is left out, not multiplied
+        // by zero: an infinite mean of one row stays out of its partner.
+        T2 b; b.x = TF(0); b.y = TF(0);
+        if (!real_only) b = src[(n - kk)*S + q];
+        const TF sg = 2*e <= n ? TF(1) : TF(-1);
         T2 u;
         u.x = a.x - sg*b.y;
         u.y = -(sg*b.x + a.y);
