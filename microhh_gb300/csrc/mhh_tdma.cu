@@ -789,6 +789,18 @@ namespace mhh
                 xc[0] = y;
                 xc += NC; r += G; den += G;
             }
+            // div_by turns an infinite quotient into a NaN.  A column with a
+            // value that is not finite ends in one (a_k is not zero), and
+            // sweeps again from its input with the quotients themselves.
+            if (!isfinite(y))
+            {
+                for (k=0; k<ktot; ++k)
+                {
+                    const double p = mulx(lev[ktot + k], A.pk[col + k*kk]);
+                    y = (k ? p - mulx(lev[k], y) : p)/tab[(ktot + k)*G + gl];
+                    x[k*NC + c] = y;
+                }
+            }
             // Back: x_k = y_k - (c_k/den_k) x_{k+1}.
             const double* w3 = tab + (3*ktot - 2)*G + gl;
             xc = x + (ktot - 2)*NC + c;

@@ -57,3 +57,40 @@ def test_inverse_mean(mhh, n, precision, axis):
     else:
         assert torch.equal(t[0], plain[0]) and torch.equal(t[3], plain[3])
         assert bool(torch.isinf(t[1]).all()) and bool(torch.isinf(t[2]).all())
+
+
+@pytest.mark.parametrize("ktot", [3, 8, 301, 3300])
+@pytest.mark.parametrize("level", ["bottom", "top"])
+def test_column_quotients(mhh, ktot, level):
+    """FP64, the reference's order of operations on one column: an infinite
+    right-hand side at its bottom or top level gives the quotients x/d, signed
+    infinities, as in the recurrence written out here."""
+    from microhh_gb300 import cases
+    kern, _ = mhh.load()
+    case = cases.channel(1, 1, ktot, seed=95, dt=1.e-4, adaptivestep=False)
+    m = mhh.Model(case, precision=64)
+    w = m.get("w")
+    # w at the lower face of the lowest cell, or at the upper of the highest.
+    w[1 if level == "bottom" else ktot + 1] = np.inf
+    m.set("w", w)
+    f, _ = m.device_fields()
+    mhh.check(kern.mhh_pres_2_exec(m.ctx(), ctypes.byref(f), 1.e-4, None), "pres_2")
+    m.synchronize()
+    got = case.interior(m.get("p")).ravel()
+    dz, dzhi = m.profile("dz")[1:-1], m.profile("dzhi")[1:]
+    m.close()
+    a, c = dz * dzhi[:-1], dz * dzhi[1:]
+    rhs = np.zeros(ktot)
+    rhs[0 if level == "bottom" else -1] = -np.inf if level == "bottom" else np.inf
+    b = -(a + c)
+    b[0] += a[0]
+    b[-1] -= c[-1]
+    y, den = np.zeros(ktot), np.zeros(ktot)
+    den[0] = b[0]
+    y[0] = rhs[0] / den[0]
+    for k in range(1, ktot):
+        den[k] = b[k] - a[k] * (c[k - 1] / den[k - 1])
+        y[k] = (rhs[k] - a[k] * y[k - 1]) / den[k]
+    for k in range(ktot - 2, -1, -1):
+        y[k] -= c[k] / den[k] * y[k + 1]
+    assert np.array_equal(np.sign(got), np.sign(y)) and np.isinf(got).all()
