@@ -633,10 +633,9 @@ unsigned long long mhh_ctx_settings(const mhh_ctx* c)
     return !c || g_timing ? 0 : g_settings + c->settings;
 }
 
-int mhh_set_option(const char* name, int value)
+static int store_option(const char* name, int value)
 {
     if (!name) return fail(MHH_ERR_ARG, "NULL option");
-    ++g_settings;
     if (!std::strcmp(name, "tendency_kernel"))
     {
         if (value < -1 || value > 2) return fail(MHH_ERR_ARG, "tendency_kernel is -1, 0, 1 or 2");
@@ -682,10 +681,18 @@ int mhh_set_option(const char* name, int value)
     return fail(MHH_ERR_ARG, "unknown option");
 }
 
+int mhh_set_option(const char* name, int value)
+{
+    // The number of the settings changes after the setting: whoever reads the
+    // new number finds the new value.
+    const int rc = store_option(name, value);
+    if (rc == MHH_OK) ++g_settings;
+    return rc;
+}
+
 int mhh_ctx_set_option(mhh_ctx* c, const char* name, int value)
 {
     if (!c || !name) return fail(MHH_ERR_ARG, "NULL argument");
-    ++c->settings;
     const bool reset = value == -2;
     if (!std::strcmp(name, "tendency_kernel"))
     {
@@ -710,6 +717,7 @@ int mhh_ctx_set_option(mhh_ctx* c, const char* name, int value)
     }
     else
         return fail(MHH_ERR_ARG, "unknown option");
+    ++c->settings;
     return MHH_OK;
 }
 
@@ -1009,7 +1017,6 @@ int mhh_boundary_ghost_cells(mhh_ctx* c, void* a, int bt, const void* abot, cons
 int mhh_boundary_surface_init(mhh_ctx* c, int thermo_bc)
 {
     if (!c) return fail(MHH_ERR_ARG, "NULL argument");
-    ++c->settings;
     if (thermo_bc != MHH_BC_FLUX && thermo_bc != MHH_BC_DIRICHLET)
         return fail(MHH_ERR_ARG, "surface model needs a flux or Dirichlet scalar BC");
     std::vector<float> zL, f;
@@ -1027,6 +1034,7 @@ int mhh_boundary_surface_init(mhh_ctx* c, int thermo_bc)
     cudaMemsetAsync(c->sw.dbdz, 0, sizeof(double)*n, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return fail(MHH_ERR_CUDA, "surface_init");
     c->surf_ready = 1;
+    ++c->settings;
     return check_cuda("surface_init");
 }
 
@@ -1096,11 +1104,11 @@ int mhh_advec_2i5_exec(mhh_ctx* c, const mhh_fields* f, cudaStream_t s)
 int mhh_advec_2i5_set_fluxlimit(mhh_ctx* c, int limit_scalar)
 {
     if (!c) return fail(MHH_ERR_ARG, "NULL argument");
-    ++c->settings;
     // The limiter's wall treatment needs four levels (src/advec_2i5.cxx
     // applies separate stencils at kstart, kstart+1, kend-2 and kend-1).
     if (limit_scalar && c->d.ktot < 4) return fail(MHH_ERR_ARG, "the flux limiter needs ktot >= 4");
     c->fluxlimit_s = limit_scalar ? 1 : 0;
+    ++c->settings;
     return MHH_OK;
 }
 
@@ -1271,7 +1279,6 @@ static int upload_buffer(mhh_ctx* c)
 int mhh_buffer_setup(mhh_ctx* c, double zstart, double sigma, double beta)
 {
     if (!c) return fail(MHH_ERR_ARG, "NULL argument");
-    ++c->settings;
     const Dims& d = c->d;
     const int kc = d.kcells;
     if (c->hbuf.empty()) c->hbuf.assign(5*(size_t)kc, 0.);
@@ -1292,13 +1299,13 @@ int mhh_buffer_setup(mhh_ctx* c, double zstart, double sigma, double beta)
     }
     c->buf_kb = std::min(kb, kbh);
     c->buf_on = 1;
+    ++c->settings;
     return upload_buffer(c);
 }
 
 int mhh_buffer_set_profile(mhh_ctx* c, const char* name, const double* prof)
 {
     if (!c || !name || !prof) return fail(MHH_ERR_ARG, "NULL argument");
-    ++c->settings;
     if (!c->buf_on) return fail(MHH_ERR_ARG, "buffer layer not set up");
     int q = -1;
     if (!std::strcmp(name, "u")) q = 2;
@@ -1310,6 +1317,7 @@ int mhh_buffer_set_profile(mhh_ctx* c, const char* name, const double* prof)
     const double off = q == 4 ? c->th0 : 0.;
     for (int k=0; k<kc; ++k) c->hbuf[(size_t)q*kc + k] = prof[k] - off;
     c->buf_set |= 1 << (q - 2);
+    ++c->settings;
     return upload_buffer(c);
 }
 
