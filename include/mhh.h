@@ -122,6 +122,9 @@ long long mhh_launch_count(void);
 /* Adds n to that count: a driver that replays a captured CUDA graph adds the
    graph's kernel nodes per replay (no counterpart in the reference). */
 int mhh_launch_count_add(long long n);
+/* The part of that count that the calling thread made: the difference over a
+   capture is the kernels captured, whatever other threads launch meanwhile. */
+long long mhh_launch_count_thread(void);
 /* A number that changes with every setting that a launch of this context reads
    (options, flux limiter, surface tables, buffer layer); 0 while timing is on,
    when launches must not be replayed.  A driver that keeps captured launches

@@ -15,6 +15,7 @@ namespace
 {
     thread_local std::string g_last_error;
     std::atomic<long long> g_launches{0};
+    thread_local long long t_launches = 0;           // those of this thread
 
     // Live per-kernel timing: CUDA events recorded on the launching stream
     // around each kernel group, collected after a synchronisation.
@@ -66,7 +67,7 @@ void mhh_set_last_error(const char* msg) { g_last_error = msg ? msg : ""; }
 
 namespace mhh
 {
-    void count_launch(int n) { g_launches += n; }
+    void count_launch(int n) { g_launches += n; t_launches += n; }
     static int g_tend_variant = -1;
     int tendency_variant() { return g_tend_variant; }
     void set_tendency_variant(int v) { g_tend_variant = v; }
@@ -723,9 +724,12 @@ int mhh_ctx_set_option(mhh_ctx* c, const char* name, int value)
 
 int mhh_launch_count_add(long long n)
 {
-    mhh::count_launch((int)n);
+    g_launches += n;
+    t_launches += n;
     return MHH_OK;
 }
+
+long long mhh_launch_count_thread(void) { return t_launches; }
 
 int mhh_timing_enable(int on)
 {

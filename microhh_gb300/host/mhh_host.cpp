@@ -965,6 +965,7 @@ namespace mhh_host
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         cudaThreadExchangeStreamCaptureMode(&mode);
         const int first = timeloop->get_substep();
+        const long long n0 = mhh_launch_count_thread();
         const cudaStream_t own = stream;
         cudaGraph_t g = nullptr;
         bool ok = cap_ || cudaStreamCreateWithFlags(&cap_, cudaStreamNonBlocking) == cudaSuccess;
@@ -982,24 +983,13 @@ namespace mhh_host
         }
         ok = ok && cudaGraphInstantiate(&graph_, g, 0) == cudaSuccess;
         if (!ok) graph_ = nullptr;
-        // The kernels of this capture (other threads may be launching).
-        graph_kernels_ = 0;
-        size_t nn = 0;
-        if (g && cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0)
-        {
-            std::vector<cudaGraphNode_t> nodes(nn);
-            cudaGraphGetNodes(g, nodes.data(), &nn);
-            for (auto node : nodes)
-            {
-                cudaGraphNodeType t = cudaGraphNodeTypeEmpty;
-                if (cudaGraphNodeGetType(node, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) ++graph_kernels_;
-            }
-        }
         if (g) cudaGraphDestroy(g);
         cudaThreadExchangeStreamCaptureMode(&mode);
         while (timeloop->get_substep() != first) timeloop->advance_substep();
         if (!fused) { advec->set_stream(stream); diff->set_stream(stream); pres->set_stream(stream); }
-        mhh_launch_count_add(-graph_kernels_);      // captured, not yet run
+        // Captured, not run (nor ever, where the capture failed).
+        graph_kernels_ = mhh_launch_count_thread() - n0;
+        mhh_launch_count_add(-graph_kernels_);
         if (!ok) cudaGetLastError();
         return ok;
     }
