@@ -49,6 +49,10 @@ int mhh_model_get_div(mhh_model* m, double* out);
 int mhh_model_get_dt(mhh_model* m, double* out);
 int mhh_model_get_time(mhh_model* m, double* out);
 int mhh_model_get_substep(mhh_model* m, int* out);
+/* Steps that were launched as one captured graph: with a fixed time step from
+   the fourth step on, again from the fourth after a change of a setting or of
+   the time step (no counterpart in the reference). */
+int mhh_model_get_replayed(mhh_model* m, long long* out);
 int mhh_model_get_grid(mhh_model* m, mhh_grid* out);
 int mhh_model_get_profile(mhh_model* m, const char* name, double* out);
 int mhh_model_get_surface(mhh_model* m, const char* name, double* out);

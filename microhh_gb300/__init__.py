@@ -163,6 +163,7 @@ def load():
     for n in ("mhh_model_get_cfl", "mhh_model_get_dn", "mhh_model_get_div", "mhh_model_get_dt", "mhh_model_get_time"):
         _declare(host, n, I, [P, dp])
     _declare(host, "mhh_model_get_substep", I, [P, ctypes.POINTER(ctypes.c_int)])
+    _declare(host, "mhh_model_get_replayed", I, [P, ctypes.POINTER(ctypes.c_longlong)])
     _declare(host, "mhh_model_get_grid", I, [P, ctypes.POINTER(Grid)])
     _declare(host, "mhh_model_get_profile", I, [P, ctypes.c_char_p, dp])
     _declare(host, "mhh_model_get_surface", I, [P, ctypes.c_char_p, dp])
@@ -344,6 +345,12 @@ class Model:
 
     def time(self):
         return self._scalar(self.host.mhh_model_get_time)
+
+    def replayed_steps(self):
+        """Steps launched as one captured graph (include/mhh_model.h)."""
+        v = ctypes.c_longlong()
+        check(self.host.mhh_model_get_replayed(self.h, ctypes.byref(v)))
+        return v.value
 
     def profile(self, name):
         a = np.empty(self.grid.kcells, dtype=np.float64)

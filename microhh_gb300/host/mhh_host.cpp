@@ -1019,6 +1019,7 @@ namespace mhh_host
         }
         cuda_check(cudaGraphLaunch(graph_, stream), "graph launch");
         mhh_launch_count_add(graph_kernels_);
+        ++replayed_;
         do timeloop->advance_substep(); while (timeloop->in_substep());
         timeloop->step_time();
         return true;
@@ -1414,6 +1415,7 @@ int mhh_model_get_dn(mhh_model* mm, double* out) { WITH_MODEL(mm, *out = m.get_d
 int mhh_model_get_div(mhh_model* mm, double* out) { WITH_MODEL(mm, *out = m.get_div()); }
 int mhh_model_get_dt(mhh_model* mm, double* out) { WITH_MODEL(mm, *out = m.get_timeloop().get_dt()); }
 int mhh_model_get_time(mhh_model* mm, double* out) { WITH_MODEL(mm, *out = m.get_timeloop().get_time()); }
+int mhh_model_get_replayed(mhh_model* mm, long long* out) { WITH_MODEL(mm, *out = m.replayed_steps()); }
 int mhh_model_get_substep(mhh_model* mm, int* out) { WITH_MODEL(mm, *out = m.get_timeloop().get_substep()); }
 int mhh_model_get_grid(mhh_model* mm, mhh_grid* out) { WITH_MODEL(mm, *out = m.get_grid().get_grid_data()); }
 int mhh_model_get_profile(mhh_model* mm, const char* name, double* out)

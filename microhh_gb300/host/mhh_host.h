@@ -379,6 +379,9 @@ namespace mhh_host
             // or a value outside [0, 10) throws Nonfinite_error ("Simulation
             // has non-finite numbers").  Synchronises the stream.
             void check_status();
+            // Steps whose launches (for the module calls those of the second
+            // and third substep) went out as one graph.
+            long long replayed_steps() const { return replayed_; }
         private:
             void set_time_step();
             // A substep's launches, without the step's time.
@@ -402,6 +405,7 @@ namespace mhh_host
             int seen_ = 0;              // steps begun with this key
             cudaGraphExec_t graph_ = nullptr;
             long long graph_kernels_ = 0;
+            long long replayed_ = 0;
             cudaStream_t cap_ = nullptr;
             std::string ini_text;
             std::vector<double> z_full;
