@@ -169,8 +169,25 @@ namespace mhh_host
                 if (mode != MHH_ENS_GRAPHS && mode != MHH_ENS_BATCHED) throw std::runtime_error("unknown ensemble mode");
                 for (auto* h : members)
                     if (!has_fixed_step(*h)) throw std::runtime_error("graph mode needs adaptivestep=false in every member");
-                if ((mode == MHH_ENS_BATCHED) != batched) drop_graphs();
+                // Captured launches hold the settings and time steps of their
+                // members.  While timing is on (settings 0) nothing is replayed.
+                std::vector<MemberKey> now;
+                bool timing = false;
+                for (auto* h : members)
+                {
+                    MemberKey k{mhh_ctx_settings(ctx_of(*h)), 0.};
+                    h->visit([&](auto& m) { k.dt = m.get_timeloop().get_dt(); });
+                    timing = timing || k.settings == 0;
+                    now.push_back(k);
+                }
+                if (timing)
+                {
+                    for (int step=0; step<n; ++step) eager_step();
+                    return;
+                }
+                if ((mode == MHH_ENS_BATCHED) != batched || !(now == keys)) drop_graphs();
                 batched = mode == MHH_ENS_BATCHED;
+                keys = std::move(now);
                 int done = 0;
                 if (!captured && done < n)
                 {
@@ -212,6 +229,14 @@ namespace mhh_host
             std::string autotune();
 
         private:
+            struct MemberKey
+            {
+                unsigned long long settings;
+                double dt;
+                bool operator==(const MemberKey& o) const { return settings == o.settings && dt == o.dt; }
+            };
+            std::vector<MemberKey> keys;      // of the captured launches
+
             void eager_step()
             {
                 // Fork from the main stream so that earlier sequential work
