@@ -909,12 +909,10 @@ int mhh_ctx_estimate_bytes(const mhh_grid_desc* g, int precision, size_t* bytes)
     const double icells = g->itot + 2*g->igc, jcells = g->jtot + 2*g->jgc, kcells = g->ktot + 2*g->kgc;
     const double ij = icells*jcells;
     const double n = double(g->itot)*g->jtot*g->ktot;
-    const double groups = double(g->itot/2 + 1)*(g->jtot/2 + 1)*g->ktot;
     double b = 0.;
     b += 14.*kcells*tf;                         // profiles
     b += n*tf + n*8. + g->ktot*8.;              // packed pressure + work + level means
-    b += groups*(8. + 8. + 8. + 8. + 4. + 8.); // elimination tables
-    b += 1.1*groups*(precision == MHH_FP64 ? 24. : 12. + 20.);   // the same in block order
+    b += tdma_bytes(g->itot, g->jtot, g->ktot, precision);   // elimination tables
     b += 2.*(g->itot + g->jtot)*(16. + 8.);    // twiddles
     b += 11.*ij*8. + ij*4. + 2.*10000*4.;      // surface layer
     b += 2.*kcells*8.;                          // mixing length

@@ -154,7 +154,10 @@ namespace mhh
         double* dz2;          // ktot: dz^2
         double* dz2rho;       // ktot: dz^2 * rhoref
         double* work;         // itot*jtot*ktot doubles: forward-swept right-hand side
-        double* rtab;         // (itot/2+1)*(jtot/2+1)*ktot: den per column group and level
+        // Tables of (itot/2+1)*(jtot/2+1)*ktot values.  rtab and wtab: NULL in
+        // FP64 contexts with the column-resident solve; stab only in FP32
+        // contexts, stabd only in FP64 contexts.
+        double* rtab;         // den per column group and level
         double* wtab;         // same shape: c_k/den_k, the back-substitution factor
         double* gtab;         // same shape: forward coefficient of the rescaled recurrence
         double* htab;         // same shape: backward coefficient of the rescaled recurrence
@@ -192,6 +195,9 @@ namespace mhh
     void set_fft_column_pairs(int p);
 
     int tdma_table(PresWork& pw, int itot, int jtot, int ktot, int precision, cudaStream_t s);
+    // At most the bytes of the tables that tdma_table leaves (FP32 contexts
+    // hold up to 20 bytes a group and level less, by their levels).
+    double tdma_bytes(int itot, int jtot, int ktot, int precision);
 
     template<typename TF> void launch_pres_in(const Dims& d, const Prof<TF>& pr, const TF* u, const TF* v, const TF* w,
                                               const TF* ut, const TF* vt, const TF* wt, TF* pk, double dti, cudaStream_t s);

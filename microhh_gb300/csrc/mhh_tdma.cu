@@ -72,8 +72,8 @@ namespace mhh
         for (int k=0; k<ktot; ++k)
         {
             const double sk = dz2[k]/rtab[base + k*stride];
-            stabd[base + k*stride] = sk;
-            stab[base + k*stride] = float(sk);
+            if (stabd) stabd[base + k*stride] = sk;
+            else stab[base + k*stride] = float(sk);
             gtab[base + k*stride] = k ? a[k]*(dz2[k-1]/rtab[base + (k-1)*stride])/dz2[k] : 0.;
             htab[base + k*stride] = k < ktot-1 ? c[k]*(dz2[k+1]/rtab[base + (k+1)*stride])/dz2[k] : 0.;
         }
@@ -319,7 +319,7 @@ namespace mhh
         // Backward: xi_k = z_k - h_k xi_{k+1}; x_k = s_k xi_k.
         {
             const long long k = ktot - 1;
-            const float s = __ldg(&stab[base + k*stride]);
+            const float s = sizeof(TF) == 4 ? __ldg(&stab[base + k*stride]) : 0.f;
             const double sd = sizeof(TF) == 8 ? __ldg(&stabd[base + k*stride]) : 0.;
             TF* row = pk + k*kk;
             #pragma unroll
@@ -339,7 +339,7 @@ namespace mhh
                 {
                     const long long k = k0 - b;
                     h[b] = __ldg(&htab[base + k*stride]);
-                    s[b] = __ldg(&stab[base + k*stride]);
+                    s[b] = sizeof(TF) == 4 ? __ldg(&stab[base + k*stride]) : 0.f;
                     sd[b] = sizeof(TF) == 8 ? __ldg(&stabd[base + k*stride]) : 0.;
                     const double* wrow = work + k*kk;
                     #pragma unroll
@@ -435,7 +435,7 @@ namespace mhh
         // Backward: xi_k = z_k - h_k xi_{k+1}; x_k = s_k xi_k.
         {
             const long long k = ktot - 1;
-            const float s = __ldg(stab + base + k*stride);
+            const float s = sizeof(TF) == 4 ? __ldg(stab + base + k*stride) : 0.f;
             const double sd = sizeof(TF) == 8 ? __ldg(stabd + base + k*stride) : 0.;
             pk[col + k*kk] = dc_out<TF>(scale_out<TF>(z, s, sd), col, (int)k, itot, jtot, dcm);
         }
@@ -450,7 +450,7 @@ namespace mhh
                 {
                     const long long k = k0 - b;
                     h[b] = __ldg(htab + base + k*stride);
-                    s[b] = __ldg(stab + base + k*stride);
+                    s[b] = sizeof(TF) == 4 ? __ldg(stab + base + k*stride) : 0.f;
                     sd[b] = sizeof(TF) == 8 ? __ldg(stabd + base + k*stride) : 0.;
                     zv[b] = work[col + k*kk];
                 }
@@ -863,8 +863,9 @@ namespace mhh
         if (cudaMallocAsync((void**)&pw.wtab, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
         if (cudaMallocAsync((void**)&pw.gtab, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
         if (cudaMallocAsync((void**)&pw.htab, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.stab, sizeof(float)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
-        if (cudaMallocAsync((void**)&pw.stabd, sizeof(double)*n, s) != cudaSuccess) return MHH_ERR_CUDA;
+        // The output scale in the fields' precision.
+        if ((dbl ? cudaMallocAsync((void**)&pw.stabd, sizeof(double)*n, s)
+                 : cudaMallocAsync((void**)&pw.stab, sizeof(float)*n, s)) != cudaSuccess) return MHH_ERR_CUDA;
         if (cudaMallocAsync((void**)&pw.fmode, ng, s) != cudaSuccess) return MHH_ERR_CUDA;
         dim3 grid((pw.niu + 127)/128, pw.nju);
         k_tdma_table<<<grid, 128, 0, s>>>(pw.niu, pw.nju, ktot, pw.bmati, pw.bmatj, pw.a, pw.c, pw.dz2rho, pw.dz2,
@@ -886,7 +887,15 @@ namespace mhh
         if ((dbl ? cudaMallocAsync((void**)&pw.dtab, 3*sizeof(double)*nr, s)
                  : cudaMallocAsync((void**)&pw.ctab, 3*sizeof(float)*nr, s)) != cudaSuccess) return MHH_ERR_CUDA;
         chunks(pw.lg, ng, nullptr, 0);
-        if (!dbl)
+        if (dbl)
+        {
+            // The resident solve has den and c/den in its blocks' order; no
+            // other solve of double fields reads them.
+            cudaFreeAsync(pw.rtab, s);
+            cudaFreeAsync(pw.wtab, s);
+            pw.rtab = pw.wtab = nullptr;
+        }
+        else
         {
             // The groups with FP64 sweeps, listed on the host.
             std::vector<unsigned char> fm(ng);
@@ -905,6 +914,18 @@ namespace mhh
             if (cudaStreamSynchronize(s) != cudaSuccess) return MHH_ERR_CUDA;   // list is a host buffer
         }
         return cudaStreamSynchronize(s) == cudaSuccess ? MHH_OK : MHH_ERR_CUDA;
+    }
+
+    double tdma_bytes(int itot, int jtot, int ktot, int precision)
+    {
+        const bool dbl = precision == MHH_FP64;
+        const long long ng = (long long)(itot/2 + 1)*(jtot/2 + 1);
+        const int lg = ktot > 65535 ? -1 : tdr_groups(ng, ktot, dbl);
+        // g, h and the output scale; den and c/den; blocks of the resident
+        // solve, in FP32 contexts with every group listed.
+        const double each = double(ng)*ktot, blocks = double(((ng + (1LL << std::max(lg, 0)) - 1) >> std::max(lg, 0)) << std::max(lg, 0))*ktot;
+        if (dbl) return lg < 0 ? 40.*each : 24.*each + 24.*blocks;
+        return 36.*each + double(ng) + (lg < 0 ? 0. : 12.*blocks + 20.*blocks + 4.*ng);
     }
 
     template<typename TF>
