@@ -103,9 +103,9 @@ namespace mhh
         // SM count.
         int best = 0;
         double cost = 0.;
-        for (int n = (ktot + most - 1)/most; n <= ktot; ++n)
+        // From the tallest chunk down; of equal costs the first.
+        for (int kc = std::min(most, ktot); kc > 0; --kc)
         {
-            const int kc = (ktot + n - 1)/n;
             const double blocks = double(tiles)*((ktot + kc - 1)/kc);
             const double t = dbl ? std::ceil(blocks/nsm)*(kc + 3)
                                  : (double(tiles)*ktot + 3.*blocks)/nsm + 1.25*(kc + 3);
