@@ -76,7 +76,7 @@ def build(verbose=False, force=False, extra_nvcc=()):
     os.makedirs(OBJDIR, exist_ok=True)
 
     cu = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
-    hdr = sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + sorted(glob.glob(os.path.join(INCLUDE, "*.h")))
+    hdr = sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + sorted(glob.glob(os.path.join(CSRC, "*.h"))) + sorted(glob.glob(os.path.join(INCLUDE, "*.h")))
     if force or not os.path.exists(LIB_KERNELS) or _newest(cu + hdr) > os.path.getmtime(LIB_KERNELS):
         objs, cmds = [], []
         for src in cu:

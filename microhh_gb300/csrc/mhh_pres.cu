@@ -17,6 +17,7 @@
 
 #include "mhh_kernels.cuh"
 #include "mhh_batchable.cuh"
+#include "mhh_fft_plan.h"
 
 namespace mhh
 {
@@ -1174,63 +1175,6 @@ namespace mhh
     }
 
 #if MHH_PREC == 64
-    // The radices (2 to 10) of the run-time plan: the fewest factors, and of
-    // those the smallest sum (the least arithmetic), larger ones first.
-    static void plan_radices(FftPlan* pl)
-    {
-        const int n = pl->n;
-        std::vector<int> divs, best, pick;      // divisors of n, best radix of each
-        for (int d=1; d<=n; ++d) if (n % d == 0) divs.push_back(d);
-        best.assign(divs.size(), 1 << 20);
-        pick.assign(divs.size(), 0);
-        best[0] = 0;
-        for (size_t a=1; a<divs.size(); ++a)
-            for (int r=2; r<=10; ++r)
-                if (divs[a] % r == 0)
-                {
-                    const size_t b = std::lower_bound(divs.begin(), divs.end(), divs[a]/r) - divs.begin();
-                    const int cost = best[b] + 64 + r;
-                    if (cost < best[a]) { best[a] = cost; pick[a] = r; }
-                }
-        pl->ngfac = 0;
-        for (int d = n; d > 1; )
-        {
-            const size_t a = std::lower_bound(divs.begin(), divs.end(), d) - divs.begin();
-            pl->gfac[pl->ngfac++] = pick[a];
-            d /= pick[a];
-        }
-        std::sort(pl->gfac, pl->gfac + pl->ngfac, [](int x, int y) { return x > y; });
-    }
-
-    // The float plan: elementary radices 8, 4, 2, 3 for 2^a 3 (a >= 4), 8 after
-    // 2, 4 or 8 in frequency for 128, 256 and 512, and 4, 2, 3, 5, 7 for other
-    // lengths; neighbours grouped where a stage of the product is at hand.
-    static void plan_floats(FftPlan* pl)
-    {
-        const int n = pl->n;
-        pl->nffac = 0;
-        if (n == 128 || n == 256 || n == 512)
-        {
-            pl->ffac[0] = n/64; pl->ffac[1] = pl->ffac[2] = 8;
-            pl->nffac = 3;
-            return;
-        }
-        bool eights = false;
-        for (int m : {16, 32, 48, 64, 96, 192, 384, 768, 1024}) eights = eights || n == m;
-        std::vector<int> rad;
-        int r = n;
-        for (int f : {8, 4, 2, 3, 5, 7})
-            while ((f < 8 || eights) && r % f == 0) { rad.push_back(f); r /= f; }
-        for (size_t q=0; q<rad.size(); ++q)
-        {
-            int code = rad[q] + 16;
-            if (q + 1 < rad.size())
-                for (int pair : {0x32, 0x52, 0x24, 0x33, 0x34})
-                    if (rad[q] == (pair & 15) && rad[q+1] == pair >> 4) { code = pair; ++q; break; }
-            pl->ffac[pl->nffac++] = code;
-        }
-    }
-
     int fft_plan_init(FftPlan* pl, int n, cudaStream_t s)
     {
         std::memset(pl, 0, sizeof(*pl));
@@ -1238,8 +1182,8 @@ namespace mhh
         int r = n;
         for (int f : {2, 3, 5, 7}) while (r % f == 0) r /= f;
         if (r != 1) return MHH_ERR_UNSUPPORTED;
-        plan_radices(pl);
-        plan_floats(pl);
+        pl->ngfac = plan_radices(n, pl->gfac);
+        pl->nffac = plan_floats(n, pl->ffac);
         std::vector<double> td(2*(size_t)n);
         std::vector<float> tf(2*(size_t)n);
         const long double twopi = 6.283185307179586476925286766559005768L;
