@@ -149,7 +149,8 @@ int mhh_ctx_estimate_bytes(const mhh_grid_desc* desc, int precision, size_t* byt
    thread, 2 = the same with the four columns of one eigenvalue per thread,
    3 = the rescaled recurrence in float for the column groups whose forward
    sweep damps (max |g| <= 0.999) and in FP64 for the others (FP32 contexts;
-   1 in FP64 contexts and for columns above about 8000 levels), -1 =
+   1 in FP64 contexts and for columns above 4411 levels, which a block cannot
+   keep in shared memory), -1 =
    automatic (0 for FP64 contexts, 3 for FP32 contexts; the default). */
 int mhh_set_option(const char* name, int value);
 /* "fft_pipeline": 0 or 1, without effect (the transforms have one schedule;

@@ -500,7 +500,9 @@ namespace mhh
     }
 
     // log2 of the groups per block, or -1 where not even one group's columns
-    // fit (the kernels that sweep through global memory take those).  16
+    // fit: above 4411 levels in the mixed solve (52 bytes a level, those of its
+    // FP64 blocks) and 3185 in double (72).  The kernels that sweep through
+    // global memory take those.  16
     // groups in float (64-byte runs; the FP64 blocks of the mixed solve then
     // fill a warp) and 8 in double, fewer while that leaves no room for a
     // second block on the SM, and 8 where 16 would leave SMs idle.  Measured
