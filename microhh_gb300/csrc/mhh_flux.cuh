@@ -1,6 +1,6 @@
-// mhh_flux.cuh -- device helpers shared by the flux-form tendency kernels
-// (mhh_tend_flux.cu): asynchronous plane copies and the
-// advective face fluxes of src/advec_2i5.cxx:150-728 (6th-order
+// mhh_flux.cuh -- device helpers shared by the marching kernels
+// (mhh_tend_flux.cu, mhh_tend_2.cu, mhh_visc_planes.cu): asynchronous plane
+// copies and the advective face fluxes of src/advec_2i5.cxx:150-728 (6th-order
 // interpolation with 5th-order upwind dissipation, lower orders next to the
 // walls) and of the flux limiter (include/advec_monotonic.h:28-219).
 #pragma once
@@ -10,18 +10,7 @@
 
 namespace mhh
 {
-    // Asynchronous global -> shared copy of one element; a copy with
-    // valid == false writes zero and reads nothing.
-    template<typename TF>
-    __device__ __forceinline__ void cp_async_el(TF* dst, const TF* src, bool valid)
-    {
-        const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-        const int n = valid ? (int)sizeof(TF) : 0;
-        if constexpr (sizeof(TF) == 4)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" :: "r"(s), "l"(src), "r"(n) : "memory");
-        else
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(s), "l"(src), "r"(n) : "memory");
-    }
+    // Asynchronous global -> shared copy of one element.
     template<typename TF>
     __device__ __forceinline__ void cp_async_one(TF* dst, const TF* src)
     {

@@ -73,7 +73,6 @@ namespace mhh
     };
 
     template<typename TF> void launch_cyclic(const FieldList<TF>& fl, const Dims& d, int edges, cudaStream_t s);
-    template<typename TF> void launch_cyclic2d(TF* a, const Dims& d, cudaStream_t s);
     template<typename TF> void launch_set_bc(TF* val, TF* grad, TF* flux, int type, double aval, double visc,
                                              int sfg, const Dims& d, cudaStream_t s);
     template<typename TF> void launch_ghost(const GhostList<TF>& gl, const Dims& d, const TF* dzh, cudaStream_t s);

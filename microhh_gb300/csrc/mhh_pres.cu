@@ -65,21 +65,12 @@ namespace mhh
     }
 
     // ---- fixed-length transforms -----------------------------------------
-    // The radices are compile-time constants (8 first, then 4, 2, 3, 5), so all
-    // index arithmetic folds into shifts and multiplications and each stage is
+    // The radices are compile-time constants (8 first, then 4), so all index
+    // arithmetic folds into shifts and multiplications and each stage is
     // unrolled.
     __host__ __device__ constexpr int fixed_radix(int n, int s)
     {
-        int r = n;
-        for (int q=0; q<=s; ++q)
-        {
-            int f = 0;
-            const int cand[5] = {8, 4, 2, 3, 5};
-            for (int t=0; t<5 && !f; ++t) if (r % cand[t] == 0) f = cand[t];
-            if (q == s) return f;
-            r /= f;
-        }
-        return 0;
+        return s == 0 && n % 8 == 0 ? 8 : 4;
     }
 
     template<typename T2>
@@ -111,46 +102,18 @@ namespace mhh
         u[3] = cadd(c2, c3); u[7] = csub(c2, c3);
     }
 
-    // Radix-R butterfly of u[0..R-1] in place (forward), for the stage with
-    // sub-length T = N/R (general radices take their twiddles from tws).
-    template<typename TF, int N, int R, int T>
-    __device__ __forceinline__ void radix_bfly(typename C2<TF>::T* u, const typename C2<TF>::T* __restrict__ tws)
+    // Radix-R butterfly of u[0..R-1] in place (forward).
+    template<typename TF, int R>
+    __device__ __forceinline__ void radix_bfly(typename C2<TF>::T* u)
     {
         using T2 = typename C2<TF>::T;
+        static_assert(R == 8 || R == 4, "radices 8 and 4");
         if (R == 8) dft8<TF, T2>(u);
-        else if (R == 4)
+        else
         {
             const T2 a = cadd(u[0], u[2]), b = csub(u[0], u[2]);
             const T2 c = cadd(u[1], u[3]), e = mul_mi<T2>(csub(u[1], u[3]));
             u[0] = cadd(a, c); u[2] = csub(a, c); u[1] = cadd(b, e); u[3] = csub(b, e);
-        }
-        else if (R == 2)
-        {
-            const T2 a = u[0];
-            u[0] = cadd(a, u[1]); u[1] = csub(a, u[1]);
-        }
-        else if (R == 3)
-        {
-            const TF s3 = TF(0.86602540378443864676);
-            const T2 t1 = cadd(u[1], u[2]), t4 = csub(u[1], u[2]);
-            T2 t2; t2.x = u[0].x - TF(0.5)*t1.x; t2.y = u[0].y - TF(0.5)*t1.y;
-            u[0] = cadd(u[0], t1);
-            u[1].x = t2.x + s3*t4.y; u[1].y = t2.y - s3*t4.x;
-            u[2].x = t2.x - s3*t4.y; u[2].y = t2.y + s3*t4.x;
-        }
-        else
-        {
-            T2 v[R];
-            #pragma unroll
-            for (int r=0; r<R; ++r)
-            {
-                T2 acc = u[0];
-                #pragma unroll
-                for (int q=1; q<R; ++q) acc = cadd(acc, cmul(u[q], tws[(q*r*T) % N]));
-                v[r] = acc;
-            }
-            #pragma unroll
-            for (int r=0; r<R; ++r) u[r] = v[r];
         }
     }
 
@@ -177,7 +140,7 @@ namespace mhh
                 #pragma unroll
                 for (int q=1; q<R; ++q)
                     u[q] = (PACC == 1) ? src[xb + q*T] : cmul(src[xb + q*T], tws[(q*k*step) % N]);
-                radix_bfly<TF, N, R, T>(u, tws);
+                radix_bfly<TF, R>(u);
                 #pragma unroll
                 for (int r=0; r<R; ++r) dst[j + r*PACC] = u[r];
             }
@@ -285,8 +248,7 @@ namespace mhh
 
     // One block transforms 2P real sequences: load them into shared memory,
     // pack pairs as complex, FFT, separate into halfcomplex (forward) or take
-    // real and imaginary parts (inverse), store.  NFIX > 0 selects the
-    // fixed-length path (NFIX = n, PFIX = P); NFIX = 0 the run-time plan.
+    // real and imaginary parts (inverse), store (n = NFIX, P = PFIX).
     // The float transform with the fused right-hand side keeps five blocks
     // per SM (at most 51 registers): its batched loads need the residency to
     // cover the latency of HBM.
@@ -392,9 +354,9 @@ namespace mhh
                 fft_cp_async(r1 + ls*ns + j, ok ? data + ti.sb[ls] + j : data, ok);
             }
         }
-        else if ((256 % (2*PFIX)) == 0)
+        else
         {
-            // Columns: with 2P dividing the block size every thread keeps
+            // Columns: 2P divides the block size, so every thread keeps
             // one sequence (ls) and walks its elements.
             const int ls = threadIdx.x % (2*P);
             const bool ok = ls < nloc;
@@ -403,15 +365,6 @@ namespace mhh
             const TF* sp = src + (long long)(threadIdx.x/(2*P))*L.itot;
             for (int j = threadIdx.x/(2*P); j < n; j += blockDim.x/(2*P), sp += st)
                 fft_cp_async(r1 + ls*ns + j, ok ? sp : data, ok);
-        }
-        else
-        {
-            for (int e = threadIdx.x; e < tot; e += blockDim.x)
-            {
-                const int j = e / (2*P), ls = e - j*(2*P);
-                const bool ok = ls < nloc;
-                fft_cp_async(r1 + ls*ns + j, ok ? data + ti.sb[ls] + (long long)j*L.itot : data, ok);
-            }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -500,7 +453,7 @@ namespace mhh
                 if (ls < nloc) data[ti.sb[ls] + j] = rout[ls*ns + j];
             }
         }
-        else if ((256 % (2*PFIX)) == 0)
+        else
         {
             const int ls = threadIdx.x % (2*P);
             if (ls < nloc)
@@ -509,14 +462,6 @@ namespace mhh
                 TF* dp = data + ti.sb[ls] + (long long)(threadIdx.x/(2*P))*L.itot;
                 for (int j = threadIdx.x/(2*P); j < n; j += blockDim.x/(2*P), dp += st)
                     *dp = rout[ls*ns + j];
-            }
-        }
-        else
-        {
-            for (int e = threadIdx.x; e < tot; e += blockDim.x)
-            {
-                const int j = e / (2*P), ls = e - j*(2*P);
-                if (ls < nloc) data[ti.sb[ls] + (long long)j*L.itot] = rout[ls*ns + j];
             }
         }
     }

@@ -93,31 +93,6 @@ namespace mhh
         count_launch();
     }
 
-    // Periodic fill of a 2-D array (icells*jcells).
-    template<typename TF> struct Cyclic2P { TF* a; Dims d; };
-
-    template<typename TF>
-    __device__ __forceinline__ void cyclic2d_body(const Cyclic2P<TF>& P, const VBlock& vb)
-    {
-        TF* a = P.a;
-        const Dims& d = P.d;
-        const int n = vb.x*blockDim.x + threadIdx.x;
-        if (n >= d.ijcells) return;
-        const int i = n % d.icells, j = n / d.icells;
-        if (i >= d.istart && i < d.iend && j >= d.jstart && j < d.jend) return;
-        int si = i, sj = j;
-        if (i < d.istart) si += d.itot; else if (i >= d.iend) si -= d.itot;
-        if (j < d.jstart) sj += d.jtot; else if (j >= d.jend) sj -= d.jtot;
-        a[n] = a[si + sj*d.icells];
-    }
-
-    template<typename TF>
-    void launch_cyclic2d(TF* a, const Dims& d, cudaStream_t s)
-    {
-        launch_body<Cyclic2P<TF>, cyclic2d_body<TF>, 256>(dim3((d.ijcells + 255)/256), dim3(256), 0, s, Cyclic2P<TF>{a, d});
-        count_launch();
-    }
-
     // ---------------------------------------------------------------------
     // Homogeneous boundary values, src/boundary.cxx:50-100.
     // ---------------------------------------------------------------------
@@ -907,7 +882,6 @@ namespace mhh
 
 #define MHH_INSTANTIATE(TF) \
     template void launch_cyclic<TF>(const FieldList<TF>&, const Dims&, int, cudaStream_t); \
-    template void launch_cyclic2d<TF>(TF*, const Dims&, cudaStream_t); \
     template void launch_set_bc<TF>(TF*, TF*, TF*, int, double, double, int, const Dims&, cudaStream_t); \
     template void launch_ghost<TF>(const GhostList<TF>&, const Dims&, const TF*, cudaStream_t); \
     template void launch_cyclic_tend<TF>(TF*, TF*, const Dims&, cudaStream_t); \
