@@ -38,11 +38,15 @@ int mhh_ensemble_create(mhh_ensemble** out);
 int mhh_ensemble_add(mhh_ensemble* e, mhh_model* m);
 /* Picks, per distinct grid size, the tendency and viscosity kernel variant and
    level chunk that run fastest, by timing a scratch model of that size, and
-   sets them on the members' contexts (mhh_ctx_set_option).  The members'
+   sets them on the members' contexts (mhh_ctx_set_option; -2 where no choice
+   is faster than what the context does by itself).  The members'
    state is not touched.  A one-line summary of the choices goes to report. */
 int mhh_ensemble_autotune(mhh_ensemble* e, char* report, int report_len);
 /* n RK3 steps of every member in the given mode; does not synchronise.  In
-   graph mode the first call runs one step eagerly and captures the next. */
+   graph and batched mode the first call runs one step eagerly and captures the
+   next, and so does the next call after a change of a member's settings
+   (mhh_ctx_settings) or time step.  While timing is on every step is launched
+   kernel by kernel. */
 int mhh_ensemble_run_steps(mhh_ensemble* e, int n, int mode);
 int mhh_ensemble_synchronize(mhh_ensemble* e);
 int mhh_ensemble_destroy(mhh_ensemble* e);
