@@ -54,7 +54,8 @@ namespace mhh
     // issue at two lanes per cycle and SM here, while the selects run on the
     // idle integer pipe.  With the shared viscosity sums and folded factors of
     // the double branch of tend_flux_body it took the tendencies at 256 x 256 x
-    // 128 from 15.6 to 9.3 ms per step (64^3: 0.627 to 0.38).  HALF: vel is twice the face velocity.
+    // 128 from 15.6 to 9.3 ms per step (64^3: 0.627 to 0.38).  HALF: vel is twice
+    // the face velocity.
     template<bool HALF>
     __device__ __forceinline__ double upwind5(double vel, double a, double b, double c, double d, double e, double f)
     {

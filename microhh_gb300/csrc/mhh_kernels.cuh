@@ -37,8 +37,8 @@ namespace mhh
     const Prof<float>& ctx_prof_float(const mhh_ctx* c);
     // Kernel variant of the LES tendencies: 0 = one thread per cell with
     // cached global loads, 1 = tiled shared-memory planes marching in k,
-    // 2 = flux form (every face flux once) marching in k; -1 = automatic
-    // (2 for float fields, 0 for double fields; the default).
+    // 2 = flux form (every face flux once) marching in k; -1 = automatic (2;
+    // the default).
     int tendency_variant();
     void set_tendency_variant(int v);
 
@@ -200,8 +200,8 @@ namespace mhh
 
     template<typename TF> void launch_pres_in(const Dims& d, const Prof<TF>& pr, const TF* u, const TF* v, const TF* w,
                                               const TF* ut, const TF* vt, const TF* wt, TF* pk, double dti, cudaStream_t s);
-    // Work fused into the row (x) FFT: mode 1 computes the pressure
-    // right-hand side in place of loading the forward transform's input; mode 2 stores the
+    // Work fused into the row (x) FFT: mode 1 computes the pressure right-hand
+    // side in place of loading the forward transform's input; mode 2 stores the
     // inverse transform's output into the ghost layout of p.
     // With mode 2, dcm (if set) holds each level's mean, which the tridiagonal
     // solve took out of the mean mode; it is added to every stored point.

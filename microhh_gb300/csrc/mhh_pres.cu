@@ -7,8 +7,8 @@
 // FFT: two real sequences x, y of length n are transformed together as
 // z = x + i y with a mixed-radix Stockham autosort FFT in shared memory
 // (ping-pong buffers, one barrier per stage; run-time plans of radices 2 to 12,
-// compile-time stages for n = 32 in float), then separated by Hermitian
-// symmetry into FFTW's halfcomplex order r_0 .. r_{n/2}, i_{(n+1)/2-1} .. i_1
+// mhh_fft_plan.h, compile-time stages for n = 32 in float), then separated by
+// Hermitian symmetry into FFTW's halfcomplex order r_0 .. r_{n/2}, i_{(n+1)/2-1} .. i_1
 // (the convention of src/fft.cxx:145-206).
 #include <algorithm>
 #include <cmath>

@@ -150,10 +150,11 @@ namespace mhh
     // The surface layer runs as two kernels over all cells of the 2-D arrays,
     // ghost cells included: the Obukhov state of every cell, then everything
     // that needs its neighbours'; a ghost cell computes its image's values from
-    // the same operands, which equals the periodic copy of the reference.  One kernel per module of the reference and
-    // per periodic copy made nine launches, bound by launch and latency: per RK3
-    // step with the scalar's ghost levels 0.125 ms at 32^3 and 0.19 at 512 x
-    // 512, now 0.049 and 0.11; in double 0.36 at 64^3, now 0.15.
+    // the same operands, which equals the periodic copy of the reference.  One
+    // kernel per module of the reference and per periodic copy made nine
+    // launches, bound by launch and latency: per RK3 step with the scalar's ghost
+    // levels 0.125 ms at 32^3 and 0.19 at 512 x 512, now 0.049 and 0.11; in double
+    // 0.36 at 64^3, now 0.15.
     constexpr int SURF_NT = 64;
 
     // Wind speed, Obukhov length and friction velocity,

@@ -14,8 +14,8 @@
 // and divides by the density (1 in the Boussinesq base state, the only one):
 // some 190 FP64 operations per cell against 70 here, which is what bounds the
 // double form (two FP64 lanes per cycle and SM); the float form is bound by
-// instruction issue.  256 x 192 x 128 per step: FP64 5.83 -> 3.44 ms, FP32 0.513
-// -> 0.318.
+// instruction issue.  256 x 192 x 128 per step: FP64 5.83 -> 3.01 ms, FP32 0.513
+// -> 0.28 (3.44 and 0.318 before the level chunks were chosen by the busiest SM).
 #include "mhh_kernels.cuh"
 #include "mhh_flux.cuh"
 #include "mhh_batchable.cuh"

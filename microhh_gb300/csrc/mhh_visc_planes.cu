@@ -52,8 +52,9 @@ namespace mhh
         // mlen^2 sqrt(S^2) sqrt(1 - min(N^2/(S^2 Pr), 1 - 1e-9)), as mlen^2
         // sqrt(max(S^2 - N^2/Pr, (1 - (1 - 1e-9)) S^2)): one square root and
         // no division (in double they are a dozen operations each on the
-        // narrow FP64 pipe: 3.94 to 2.84 ms per step at 256 x 256 x 128).  As there, a NaN of the ratio takes the clip.  In
-        // float, where 1 - 1e-9 rounds to 1, the clip is 0.
+        // narrow FP64 pipe: 3.94 to 2.84 ms per step at 256 x 256 x 128).  As
+        // there, a NaN of the ratio takes the clip.  In float, where 1 - 1e-9
+        // rounds to 1, the clip is 0.
         template<typename TF>
         __device__ __forceinline__ TF evisc_of(TF ml2, TF s2, TF n2, TF tpri)
         {
